@@ -14,16 +14,17 @@
 // Other rows take one fused hash pass, binned by their product count P_i:
 //   * P_i <= 64:    a team of 8 lanes, hash table in shared memory (128 slots),
 //                   persistent teams that reset only the slots a row used;
-//   * P_i <= 256:   one warp, hash table in shared memory (512 slots);
-//   * P_i <= 4096:  one CTA, hash table in shared memory (8192 slots);
+//   * P_i <= 6144:  one warp, hash table in shared memory (512 to 8192 slots;
+//                   see gustavson_warp);
 //   * larger:       one CTA, hash table in a global workspace (2*P_i slots).
-// The row's products are visited B-row by B-row in the reference's order; the
-// columns of one B row are distinct, so the lanes of one step never collide
-// and every table slot accumulates its products in (j, k) order --
-// deterministic, and the same summation order as the reference.  A column's
-// slot records the product index p of its first touch; since these indices
-// are distinct, posmap[p] = slot followed by an ordered compaction of posmap
-// yields the columns in first-touch order without a comparison sort.  Each row
+// The first and the last of these visit the row's products B-row by B-row in
+// the reference's order; the columns of one B row are distinct, so the lanes
+// of one step never collide and every table slot accumulates its products in
+// (j, k) order -- deterministic, and the same summation order as the
+// reference.  A column's slot records the product index p of its first touch;
+// since these indices are distinct, posmap[p] = slot followed by an ordered
+// compaction of posmap yields the columns in first-touch order without a
+// comparison sort.  Each row
 // writes its columns/values at its product offset (an upper bound, as the
 // reference's padded buffer), then a scan of the counts gives C's row_ptr and
 // a compaction pass packs C_col / C_val.
@@ -40,12 +41,16 @@ namespace {
 constexpr int kSmallP = 64, kSmallTS = 128;    // small-row path: products, table slots
 constexpr int kSmallTeam = 8;                  // lanes per row of the small-row path
 constexpr int kSmallWarps = 4;                 // warps per CTA: 16 teams, 1.8 KB of tables each
-constexpr int kWarpP = 256, kWarpTS = 512;     // warp path
-constexpr int kCtaP = 4096, kCtaTS = 8192;     // CTA path
-constexpr int kCtaThreads = 512;
-constexpr int kWarpsPerCta = 4;
+// warp path: a row of at most warp_products(b) products takes a table of
+// warp_slots(b) slots, so a table is at most three quarters full; the smaller
+// the table, the more warps an SM holds (32 of 512 slots, two of 8192)
+constexpr int kWarpBins = 5;
+__host__ __device__ constexpr int warp_slots(int b) { return 512 << b; }
+__host__ __device__ constexpr int warp_products(int b) { return b == 0 ? 256 : warp_slots(b) * 3 / 4; }
+constexpr int kCtaThreads = 512;               // CTA of the global-table path
 constexpr int kMergeLists = 8;                 // merge path: at most this many entries in the row of A
-constexpr int kBins = 5;                       // small (hash), warp, CTA, global, merge
+constexpr int kBinGlobal = 1 + kWarpBins, kBinMerge = kBinGlobal + 1;
+constexpr int kBins = kBinMerge + 1;           // small (hash), the warp bins, global, merge
 constexpr int kMergeWriteThreads = 128;        // direct write pass: 4 warps, each staging its rows in shared memory
 
 __device__ __forceinline__ unsigned hash_col(int c) { return (unsigned)c * 0x9E3779B1u; }
@@ -85,9 +90,9 @@ __global__ void b_sorted_kernel(const int *__restrict__ brp, const int *__restri
             }
 }
 
-// rows into five lists: the merge path (B's rows sorted, at most kMergeLists
+// rows into kBins lists: the merge path (B's rows sorted, at most kMergeLists
 // entries in the row of A and kSmallP products), then by product count the
-// small-row, warp, CTA and global hash paths; the order inside a list is
+// small-row, warp and global hash paths; the order inside a list is
 // irrelevant (rows are independent)
 __global__ void bin_rows(const long long *__restrict__ P, const int *__restrict__ arp, int64_t n,
                          const int *__restrict__ b_sorted, int *__restrict__ lists, int *counts) {
@@ -95,7 +100,16 @@ __global__ void bin_rows(const long long *__restrict__ P, const int *__restrict_
     const bool valid = i < n;
     const long long p = valid ? P[i] : 0;
     const bool merge = valid && *b_sorted && p <= kSmallP && arp[i + 1] - arp[i] <= kMergeLists;
-    const int bin = merge ? 4 : (p <= kSmallP ? 0 : (p <= kWarpP ? 1 : (p <= kCtaP ? 2 : 3)));
+    int bin = kBinMerge;
+    if (!merge) {
+        bin = 0;
+        if (p > kSmallP) {
+            bin = kBinGlobal;
+#pragma unroll
+            for (int b = kWarpBins - 1; b >= 0; --b)
+                if (p <= warp_products(b)) bin = 1 + b;
+        }
+    }
     const unsigned active = __ballot_sync(0xffffffffu, valid);
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -110,22 +124,21 @@ __global__ void bin_rows(const long long *__restrict__ P, const int *__restrict_
     }
 }
 
-// The body shared by all three paths: a team of `tsize` threads (`t` its
-// rank) fills a table of `TS` slots for row i.  sync() orders the steps.
-template <typename VT, typename Sync>
-__device__ __forceinline__ void gustavson_row(int i, int t, int tsize, const int *__restrict__ arp,
+// A CTA fills a table of `TS` slots for row i (t: the thread).
+template <typename VT>
+__device__ __forceinline__ void gustavson_row(int i, int t, const int *__restrict__ arp,
                                               const int *__restrict__ acol, const VT *__restrict__ aval,
                                               const int *__restrict__ brp, const int *__restrict__ bcol,
                                               const VT *__restrict__ bval, int *keys, int *first, VT *vals,
                                               int *posmap, unsigned TS, long long P, long long out_off,
-                                              int *__restrict__ pcol, VT *__restrict__ pval, int *__restrict__ count,
-                                              Sync sync) {
+                                              int *__restrict__ pcol, VT *__restrict__ pval, int *__restrict__ count) {
+    constexpr int tsize = kCtaThreads;
     for (unsigned h = t; h < TS; h += tsize) {
         keys[h] = -1;
         vals[h] = VT(0);
     }
     for (long long q = t; q < P; q += tsize) posmap[q] = -1;
-    sync();
+    __syncthreads();
     long long base = 0;  // product index of the first product of the current B row
     for (int j = arp[i]; j < arp[i + 1]; ++j) {
         const int c = acol[j];
@@ -147,11 +160,11 @@ __device__ __forceinline__ void gustavson_row(int i, int t, int tsize, const int
             vals[h] += prod;  // one product per slot per step: the (j, k) order
         }
         base += be - bs;
-        sync();
+        __syncthreads();
     }
     for (unsigned h = t; h < TS; h += tsize)
         if (keys[h] != -1) posmap[first[h]] = (int)h;
-    sync();
+    __syncthreads();
     // ordered compaction of posmap: entries in first-touch order
     __shared__ int team_total[kCtaThreads / 32];
     int written = 0;
@@ -159,25 +172,17 @@ __device__ __forceinline__ void gustavson_row(int i, int t, int tsize, const int
         const long long q = q0 + t;
         const int h = q < P ? posmap[q] : -1;
         const int take = h >= 0;
-        // team-wide exclusive scan of `take` (warp ballots, then warps in
-        // order); a team smaller than a warp uses only its own lanes' bits
-        const int lane = (int)(threadIdx.x & 31), warp = t >> 5;
-        const unsigned tmask =
-            tsize >= 32 ? 0xffffffffu : (((1u << tsize) - 1u) << ((unsigned)lane & ~(unsigned)(tsize - 1)));
-        const unsigned bal = __ballot_sync(tmask, take) & tmask;
-        const int before_in_warp = __popc(bal & ((1u << lane) - 1u));
-        int before = before_in_warp, total = __popc(bal);
-        if (tsize > 32) {
-            if (lane == 0) team_total[warp] = total;
-            sync();
-            before = before_in_warp;
-            total = 0;
-            for (int w = 0; w < tsize / 32; ++w) {
-                if (w < warp) before += team_total[w];
-                total += team_total[w];
-            }
-            sync();
+        // CTA-wide exclusive scan of `take` (warp ballots, then warps in order)
+        const int lane = t & 31, warp = t >> 5;
+        const unsigned bal = __ballot_sync(0xffffffffu, take);
+        if (lane == 0) team_total[warp] = __popc(bal);
+        __syncthreads();
+        int before = __popc(bal & ((1u << lane) - 1u)), total = 0;
+        for (int w = 0; w < tsize / 32; ++w) {
+            if (w < warp) before += team_total[w];
+            total += team_total[w];
         }
+        __syncthreads();
         if (take) {
             pcol[out_off + written + before] = keys[h];
             pval[out_off + written + before] = vals[h];
@@ -187,37 +192,128 @@ __device__ __forceinline__ void gustavson_row(int i, int t, int tsize, const int
     if (t == 0) count[i] = written;
 }
 
-// the lanes of one team inside a warp (the whole warp for a team of 32)
-struct GroupSync {
-    unsigned mask;
-    __device__ void operator()() const { __syncwarp(mask); }
-};
-struct CtaSync {
-    __device__ void operator()() const { __syncthreads(); }
-};
-
-// A team of G lanes (G <= 32, a power of two) per row of at most WP products,
-// with a WTS-slot table (load at most 1/2); WARPS warps per CTA, 32 / G rows
-// per warp.  Small teams suit rows whose B rows are short: a team covers one
-// B row per step of the product loop.
-template <typename VT, int WP, int WTS, int WARPS, int G>
-__global__ void __launch_bounds__(WARPS * 32) gustavson_warp(
-    const int *__restrict__ rows, int n_rows_bin, const long long *__restrict__ P, const long long *__restrict__ Poff,
+// One warp per row (a CTA of one warp; rows r, r + gridDim.x, ...), its hash
+// table of TS slots in shared memory.  The row's products are numbered in the
+// reference's (j, k) order and taken 32 at a time, one per lane, however short
+// the B rows are; the next 32 are loaded while the current ones are inserted.
+// Lanes of a step with equal columns (__match_any_sync) elect the lowest, which
+// finds the slot: columns new in this step are appended to `used` in lane
+// order, so the list is in first-touch order and needs no sort or second
+// pass.  A slot's products are added one lane after the other, in product
+// order.  The row's slots are reset from the list.
+// Bound by the latency of a step (its loads, the probe and the sum in shared
+// memory), so rows are spread over as many warps as the tables leave room
+// for.  C = A A of the 27-point stencil on 48^3, FP64 (80 M products): 1.2 ms,
+// where a CTA of 512 threads per row, stepping one 27-entry B row at a time
+// through an 8192-slot table, took 14.2 ms.  36000 lognormal rows (9.2 M
+// products): 0.94 ms against 1.95 ms.
+template <typename VT>
+__global__ void __launch_bounds__(32) gustavson_warp(
+    const int *__restrict__ rows, int n_rows_bin, unsigned TS, const long long *__restrict__ Poff,
     const int *__restrict__ arp, const int *__restrict__ acol, const VT *__restrict__ aval,
     const int *__restrict__ brp, const int *__restrict__ bcol, const VT *__restrict__ bval, int *__restrict__ pcol,
     VT *__restrict__ pval, int *__restrict__ count) {
-    constexpr int TEAMS = WARPS * 32 / G;
-    __shared__ int keys[TEAMS][WTS];
-    __shared__ int first[TEAMS][WTS];
-    __shared__ VT vals[TEAMS][WTS];
-    __shared__ int posmap[TEAMS][WP];
-    const int g = threadIdx.x / G;
-    const int64_t r = (int64_t)blockIdx.x * TEAMS + g;
-    if (r >= n_rows_bin) return;  // uniform per team; teams never touch CTA barriers
-    const int i = rows[r];
-    const unsigned mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(unsigned)(G - 1)));
-    gustavson_row<VT>(i, (int)(threadIdx.x % G), G, arp, acol, aval, brp, bcol, bval, keys[g], first[g], vals[g],
-                      posmap[g], WTS, P[i], Poff[i], pcol, pval, count, GroupSync{mask});
+    extern __shared__ __align__(16) unsigned char smem[];
+    VT *vals = reinterpret_cast<VT *>(smem);
+    int *keys = reinterpret_cast<int *>(vals + TS);
+    unsigned short *used = reinterpret_cast<unsigned short *>(keys + TS);
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x;
+    const unsigned below = (1u << lane) - 1u;
+    for (unsigned h = lane; h < TS; h += 32) {
+        keys[h] = -1;
+        vals[h] = VT(0);
+    }
+    __syncwarp();
+    for (int r = blockIdx.x; r < n_rows_bin; r += gridDim.x) {
+        const int i = rows[r];
+        const int a0 = arp[i], a1 = arp[i + 1];
+        int n_used = 0;
+        for (int g0 = a0; g0 < a1; g0 += 32) {
+            // up to 32 entries of the row of A, one per lane
+            const int j = g0 + lane;
+            int bs = 0, len = 0;
+            VT av = VT(0);
+            if (j < a1) {
+                const int c = acol[j];
+                av = aval[j];
+                bs = brp[c];
+                len = brp[c + 1] - bs;
+            }
+            int incl = len;  // products up to and including this entry's
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int total = __shfl_sync(FULL, incl, 31);
+            const int first = bs - (incl - len);  // product p of this entry is B's entry first + p
+            // product p of the group: its column (-1 past the end) and value
+            auto fetch = [&](int p, int &col, VT &prod) {
+                int e = 0;  // entries whose products all lie before p
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    if (__shfl_sync(FULL, incl, e + o - 1) <= p) e += o;
+                const int k = __shfl_sync(FULL, first, e & 31) + p;
+                const VT a = __shfl_sync(FULL, av, e & 31);
+                col = -1;
+                if (p < total) {
+                    col = bcol[k];
+                    prod = a * bval[k];
+                }
+            };
+            int col, ncol;
+            VT prod = VT(0), nprod = VT(0);
+            fetch(lane, col, prod);
+            for (int p0 = 0; p0 < total; p0 += 32) {
+                fetch(p0 + 32 + lane, ncol, nprod);
+                const unsigned active = __ballot_sync(FULL, col >= 0);
+                if (col >= 0) {
+                    const unsigned same = __match_any_sync(active, col);
+                    const int leader = __ffs(same) - 1;
+                    unsigned h = 0;
+                    bool fresh = false;
+                    if (lane == leader) {
+                        h = hash_col(col) & (TS - 1);
+                        while (true) {
+                            const int old = atomicCAS(keys + h, -1, col);
+                            fresh = old == -1;
+                            if (fresh || old == col) break;
+                            h = (h + 1) & (TS - 1);
+                        }
+                    }
+                    h = __shfl_sync(active, h, leader);
+                    const unsigned made = __ballot_sync(active, fresh);
+                    if (fresh) used[n_used + __popc(made & below)] = (unsigned short)h;
+                    n_used += __popc(made);
+                    const int rank = __popc(same & below);
+                    const unsigned repeats = __ballot_sync(active, rank > 0);
+                    if (rank == 0) vals[h] += prod;
+                    if (repeats) {
+                        const int most = (int)__reduce_max_sync(active, (unsigned)rank);
+                        for (int q = 1; q <= most; ++q) {
+                            __syncwarp(active);
+                            if (rank == q) vals[h] += prod;
+                        }
+                    }
+                }
+                n_used = __shfl_sync(FULL, n_used, 0);  // lanes past the row's end did not count; lane 0 is never past it
+                __syncwarp();
+                col = ncol;
+                prod = nprod;
+            }
+        }
+        const long long out = Poff[i];
+        for (int u = lane; u < n_used; u += 32) {
+            const unsigned h = used[u];
+            pcol[out + u] = keys[h];
+            pval[out + u] = vals[h];
+            keys[h] = -1;
+            vals[h] = VT(0);
+        }
+        if (lane == 0) count[i] = n_used;
+        __syncwarp();
+    }
 }
 
 // The small-row path as persistent teams of G lanes: a team keeps its WTS-slot
@@ -491,23 +587,7 @@ __global__ void __launch_bounds__(kMergeWriteThreads) gustavson_merge_write(
     }
 }
 
-template <typename VT>
-__global__ void __launch_bounds__(kCtaThreads) gustavson_cta(
-    const int *__restrict__ rows, int n_rows_bin, const long long *__restrict__ P, const long long *__restrict__ Poff,
-    const int *__restrict__ arp, const int *__restrict__ acol, const VT *__restrict__ aval,
-    const int *__restrict__ brp, const int *__restrict__ bcol, const VT *__restrict__ bval, int *__restrict__ pcol,
-    VT *__restrict__ pval, int *__restrict__ count) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    VT *vals = reinterpret_cast<VT *>(smem);
-    int *keys = reinterpret_cast<int *>(vals + kCtaTS);
-    int *first = keys + kCtaTS;
-    int *posmap = first + kCtaTS;
-    const int i = rows[blockIdx.x];
-    gustavson_row<VT>(i, threadIdx.x, kCtaThreads, arp, acol, aval, brp, bcol, bval, keys, first, vals, posmap,
-                      kCtaTS, P[i], Poff[i], pcol, pval, count, CtaSync());
-}
-
-// rows with more than kCtaP products: tables in a global workspace
+// rows with more products than the largest warp table takes: tables in a global workspace
 template <typename VT>
 __global__ void __launch_bounds__(kCtaThreads) gustavson_global(
     const int *__restrict__ rows, const long long *__restrict__ ws_off, const unsigned *__restrict__ ws_ts,
@@ -518,8 +598,8 @@ __global__ void __launch_bounds__(kCtaThreads) gustavson_global(
     const int b = blockIdx.x;
     const int i = rows[b];
     const long long o = ws_off[b];
-    gustavson_row<VT>(i, threadIdx.x, kCtaThreads, arp, acol, aval, brp, bcol, bval, ws_keys + o, ws_first + o,
-                      ws_vals + o, ws_pos + Poff[i], ws_ts[b], P[i], Poff[i], pcol, pval, count, CtaSync());
+    gustavson_row<VT>(i, threadIdx.x, arp, acol, aval, brp, bcol, bval, ws_keys + o, ws_first + o,
+                      ws_vals + o, ws_pos + Poff[i], ws_ts[b], P[i], Poff[i], pcol, pval, count);
 }
 
 __global__ void ws_sizes(const int *__restrict__ rows, int m, const long long *__restrict__ P,
@@ -678,8 +758,8 @@ void spgemm(const DevCRS &A, const DevCRS &B, DevCRS &C, SpgemmWork &w, SpgemmTi
     SMAX_CUDA(cudaMemcpyAsync(h.counts, w.counts.p, sizeof(int) * kBins, cudaMemcpyDeviceToHost, st));
     SMAX_CUDA(cudaStreamSynchronize(st));
     const long long total_p = h.total_p;
-    const int ns = h.counts[0], nw = h.counts[1], nc = h.counts[2], ng = h.counts[3], nm = h.counts[4];
-    const int *rs = w.lists.as<int>(), *rw = rs + n, *rc = rs + 2 * n, *rg = rs + 3 * n, *rm = rs + 4 * n;
+    const int ns = h.counts[0], ng = h.counts[kBinGlobal], nm = h.counts[kBinMerge];
+    const int *rs = w.lists.as<int>(), *rg = rs + kBinGlobal * n, *rm = rs + kBinMerge * n;
     pe.mark(1, st);
     // --- fused Gustavson pass into product-offset (padded) buffers
     if (nm != n || n == 0) {  // the direct merge path writes C itself
@@ -716,14 +796,18 @@ void spgemm(const DevCRS &A, const DevCRS &B, DevCRS &C, SpgemmWork &w, SpgemmTi
             rm, nm, Poff, A.rp(), A.ci(), A.val.as<VT>(), B.rp(), B.ci(), B.val.as<VT>(), pcol, pval, count, nullptr,
             nullptr, nullptr);
     }
-    if (nw > 0)
-        gustavson_warp<VT, kWarpP, kWarpTS, kWarpsPerCta, 32><<<ceil_div_u(nw, kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(
-            rw, nw, P, Poff, A.rp(), A.ci(), A.val.as<VT>(), B.rp(), B.ci(), B.val.as<VT>(), pcol, pval, count);
-    if (nc > 0) {
-        const size_t sm = (size_t)kCtaTS * (sizeof(VT) + 2 * sizeof(int)) + sizeof(int) * kCtaP;
-        SMAX_CUDA(cudaFuncSetAttribute(gustavson_cta<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        gustavson_cta<VT><<<nc, kCtaThreads, sm, st>>>(rc, nc, P, Poff, A.rp(), A.ci(), A.val.as<VT>(), B.rp(),
-                                                       B.ci(), B.val.as<VT>(), pcol, pval, count);
+    for (int b = kWarpBins - 1; b >= 0; --b) {  // the longest rows first
+        const int nw = h.counts[1 + b];
+        if (nw == 0) continue;
+        const size_t sm = (size_t)warp_slots(b) * (sizeof(VT) + sizeof(int)) + sizeof(unsigned short) * warp_products(b);
+        // set on every call: the attribute belongs to the current device
+        SMAX_CUDA(cudaFuncSetAttribute(gustavson_warp<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        // as many one-warp CTAs as an SM's shared memory holds (1 KB of it is reserved per CTA), at most 32
+        const int per_sm = (int)std::min<size_t>(32, (size_t)227 * 1024 / (sm + 1024));
+        const unsigned grid = (unsigned)std::min<int64_t>(nw, (int64_t)per_sm * sm_count());
+        gustavson_warp<VT><<<grid, 32, sm, st>>>(rs + (1 + b) * n, nw, (unsigned)warp_slots(b), Poff, A.rp(), A.ci(),
+                                                 A.val.as<VT>(), B.rp(), B.ci(), B.val.as<VT>(), pcol, pval, count);
+        SMAX_CUDA(cudaGetLastError());
     }
     if (ng > 0) {
         w.wts.ensure(sizeof(unsigned) * ng);
