@@ -276,22 +276,24 @@ void spgemm_finalize(smax_kernel_s *k) {
     // (symbolic_phase_impl.hpp:132-151); so does this platform
     require(k->spgemm_done, SMAX_ERR_STATE, "apply before finalize");
     const DevCRS &c = k->dCm;
-    int *rp = new int[c.n_rows + 1];
-    int *col = new int[c.nnz > 0 ? c.nnz : 1];
-    void *val = k->vbytes == 8 ? static_cast<void *>(new double[c.nnz > 0 ? c.nnz : 1])
-                               : static_cast<void *>(new float[c.nnz > 0 ? c.nnz : 1]);
-    SMAX_CUDA(cudaMemcpyAsync(rp, c.row_ptr.p, sizeof(int) * (c.n_rows + 1), cudaMemcpyDeviceToHost, k->stream));
-    if (c.nnz) {
-        SMAX_CUDA(cudaMemcpyAsync(col, c.col.p, sizeof(int) * c.nnz, cudaMemcpyDeviceToHost, k->stream));
-        SMAX_CUDA(cudaMemcpyAsync(val, c.val.p, (size_t)k->vbytes * c.nnz, cudaMemcpyDeviceToHost, k->stream));
-    }
-    SMAX_CUDA(cudaStreamSynchronize(k->stream));
+    const int64_t m = c.nnz > 0 ? c.nnz : 1;
+    std::unique_ptr<int[]> rp(new int[c.n_rows + 1]), col(new int[m]);
+    std::unique_ptr<double[]> v64(k->vbytes == 8 ? new double[m] : nullptr);
+    std::unique_ptr<float[]> v32(k->vbytes == 8 ? nullptr : new float[m]);
+    void *val = k->vbytes == 8 ? static_cast<void *>(v64.get()) : static_cast<void *>(v32.get());
+    download(k->download,
+             {{rp.get(), c.row_ptr.p, sizeof(int) * (size_t)(c.n_rows + 1)},
+              {col.get(), c.col.p, sizeof(int) * (size_t)c.nnz},
+              {val, c.val.p, (size_t)k->vbytes * (size_t)c.nnz}},
+             k->stream);
     *k->Cref.n_rows = (uint64_t)c.n_rows;
     *k->Cref.n_cols = (uint64_t)c.n_cols;
     *k->Cref.nnz = (uint64_t)c.nnz;
-    *k->Cref.row_ptr = rp;
-    *k->Cref.col = col;
+    *k->Cref.row_ptr = rp.release();
+    *k->Cref.col = col.release();
     *k->Cref.val = val;
+    v64.release();
+    v32.release();
 }
 
 

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "download.cuh"
 #include "spmv_crs.cuh"
 #include "spmv_formats.cuh"
 #include "spgemm.cuh"
@@ -150,6 +151,7 @@ struct smax_kernel_s {
     smax::SpgemmTimes spgemm_times;
     smax::SpgemmWork spgemm_work;
     bool spgemm_done = false;
+    smax::DownloadStage download;  // of C
 
     // triangular solves (SpTRSV / SpTRSM)
     smax::DevBuf D;                 // peeled diagonal

@@ -414,15 +414,25 @@ def _ftype(dtype) -> int:
     raise TypeError("values must be float32 or float64")
 
 
+class _HostArray:
+    """Owner of a library-allocated host array: numpy views it without a copy and keeps the owner alive."""
+
+    def __init__(self, p, n, dtype):
+        self._p = p
+        self.__array_interface__ = dict(version=3, shape=(int(n),), typestr=np.dtype(dtype).str, data=(p, False))
+
+    def __del__(self, free=lib.smax_free_host):
+        free(self._p)
+
+
 def _take(p, n, dtype):
-    """Copies n elements of a library-allocated host array into numpy and frees it."""
+    """n elements of a library-allocated host array as a numpy array that owns it."""
     if not p:
         return np.zeros(0, dtype)
-    out = np.empty(n, dtype=dtype)
-    if n:
-        C.memmove(out.ctypes.data, p, n * out.itemsize)
-    lib.smax_free_host(p)
-    return out
+    if not n:
+        lib.smax_free_host(p)
+        return np.zeros(0, dtype)
+    return np.asarray(_HostArray(p, n, dtype))
 
 
 class Utils:

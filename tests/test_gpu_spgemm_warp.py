@@ -1,5 +1,5 @@
 """SpGEMM rows on the warp hash path (tables of 512 to 8192 slots) around the
-product counts where the path changes."""
+product counts where the path changes, and the download of large products."""
 import numpy as np
 import pytest
 
@@ -47,3 +47,26 @@ def test_spgemm_rows_at_the_bin_edges(vt, long_len, sort, n_cols):
     np.testing.assert_array_equal(rp, orp)
     np.testing.assert_array_equal(col, ocol)
     assert normwise(val, oval) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("nnz", [(4 << 20) // 12 - 4096, 1_000_003])
+def test_large_product_is_downloaded_whole(vt, nnz):
+    """I * B = B, with C's arrays below and above the size from which the
+    download is cut into pieces, and no multiple of a piece; the arrays stay
+    valid after the kernel object is gone and can be written."""
+    rng = np.random.default_rng(nnz)
+    n = 5000
+    lens = np.full(n, nnz // n)
+    lens[: nnz - lens.sum()] += 1
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    col = (np.arange(nnz) - np.repeat(rp[:-1].astype(np.int64), lens)).astype(np.int32)
+    val = rng.uniform(-1, 1, nnz).astype(vt)
+    eye = (np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), np.ones(n, vt))
+    _, _, got, crp, ccol, cval = gpu_spgemm(eye, (rp, col, val), n, n)
+    assert got == nnz
+    np.testing.assert_array_equal(crp, rp)
+    np.testing.assert_array_equal(ccol, col)
+    np.testing.assert_array_equal(cval, val)
+    cval[-1] = 2
+    assert cval[-1] == 2
