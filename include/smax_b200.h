@@ -90,7 +90,7 @@ typedef int smax_status;
 #define SMAX_FLAG_DEVICE_POINTERS 8    /* B and C registered as device pointers */
 #define SMAX_FLAG_A_DIRTY 9            /* re-upload A at the next initialize */
 #define SMAX_FLAG_SPMV_VARIANT 10      /* CRS SpMV kernel: 0 auto, 1 warp-stream, 2 row-tile; row-major SpMM:
-                                          0 auto (= 1), 1 a grid of all rows, 2 one CTA per SM walking a row range */
+                                          0 auto, 1 a grid of all rows, 2 one CTA per SM walking a row range */
 #define SMAX_FLAG_SOLVE_MODE 11        /* SpTRSV/SpTRSM launch scheme, one of SMAX_SOLVE_* */
 #define SMAX_FLAG_LEVEL_MERGE 12       /* levels with <= this many rows*rhs run merged in one CTA (0: never) */
 #define SMAX_FLAG_SPIN_LIMIT 13        /* polls (x 1000) before a wait of the persistent or sync-free solve times out */

@@ -181,18 +181,22 @@ void spmm_upload(smax_kernel_s *k) {
     validate_crs(k->dA, dstatus(k), k->stream);
     read_status(k);
     k->crs_stream = CrsStreamPlan();
-    k->spmm_plan = SpmmPlan();  // its row ranges and staged tiles describe the previous matrix
+    k->spmm_plan.build(k->dA, k->stream);
     if (!k->f_row_major) k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, k->stream);
 }
 
 template <typename VT> void spmm_apply_t(smax_kernel_s *k, const VT *X, VT *Y) {
     const int64_t kk = (int64_t)(k->B.n_cols ? k->B.n_cols : 1);
     if (k->f_row_major) {
-        crs_spmm_row_major<VT>(k->dA, kk, X, Y, k->stream, &k->spmm_plan, k->spmv_variant);
+        crs_spmm_row_major<VT>(k->dA, kk, X, Y, k->stream, k->spmm_plan, k->spmv_variant);
     } else {
         // column-major: the reference uses A's n_rows as the leading dimension
         // of both X and Y (src/kernels/spmm/spmm_cpu/spmm_cpu_crs_impl.hpp:29,44)
         const int64_t ld = k->dA.n_rows;
+        if (kk > 1 && (int64_t)k->spmm_plan.work.bytes >= spmm_col_major_work(k->dA.n_cols, kk, k->vbytes)) {
+            crs_spmm_col_major<VT>(k->dA, kk, X, Y, ld, k->spmm_plan.work.as<VT>(), k->stream, k->spmm_plan);
+            return;
+        }
         for (int64_t v = 0; v < kk; ++v)
             crs_spmv_stream<VT>(k->crs_stream, k->dA.ci(), k->dA.val.as<VT>(), X + v * ld, Y + v * ld, k->stream);
     }
@@ -465,6 +469,16 @@ void do_initialize(smax_kernel_s *k, bool wait = true) {
         k->a_dirty = false;
         ++k->a_version;
         ++k->vals_version;
+    }
+    // column-major SpMM: the workspace of X's row-major copy, allocated here so
+    // that applies allocate nothing; without room for it they run one product
+    // per column
+    if (k->ktype == SMAX_KERNEL_SPMM && !k->f_row_major && k->B.n_cols > 1) {
+        try {
+            k->spmm_plan.work.ensure((size_t)spmm_col_major_work(k->dA.n_cols, (int64_t)k->B.n_cols, k->vbytes));
+        } catch (const Error &e) {
+            if (e.code != SMAX_ERR_OOM) throw;
+        }
     }
     if (!k->f_device) {
         size_t bb = (size_t)k->B.elems() * k->vbytes, cb = (size_t)k->C.elems() * k->vbytes;

@@ -142,7 +142,7 @@ struct smax_kernel_s {
     smax::DevBuf dB, dC;
     smax::CrsTilePlan crs_plan;
     smax::CrsStreamPlan crs_stream;
-    smax::SpmmPlan spmm_plan;  // row ranges of the row-major SpMM walk
+    smax::SpmmPlan spmm_plan;
     int spmv_variant = 0;  // 0 auto, 1 warp-stream, 2 row-tile
     smax::DevBuf status;   // smax::DevStatus
 

@@ -1,17 +1,37 @@
 // spmm.cu -- CRS SpMM Y = A X against a block of k dense vectors, sm_100a.
 //
 // Reference semantics: SPMM::CPU::naive_crs_spmm_row_maj / _col_maj
-// (src/kernels/spmm/spmm_cpu/spmm_cpu_crs_impl.hpp:9-89).  Row-major blocks
-// (X[col*k+v], Y[row*k+v]) are the layout the platform is built for: a row of
-// X is k contiguous values, so one group of G lanes owns one row of A and
-// reads/writes whole rows of X/Y with 128-bit loads and stores.  The group
-// loads G (col, val) pairs of its row at once (coalesced) and broadcasts them
-// with shuffles; each lane accumulates NV vectors of VEC = 16/sizeof(VT)
-// values.  X rows are gathered through L2 (neighbouring rows of a stencil
-// matrix reuse them); A is streamed once with evict-first loads.
-// Column-major blocks are k independent SpMVs on the columns and reuse the
-// CRS SpMV kernel (abi.cu).
+// (src/kernels/spmm/spmm_cpu/spmm_cpu_crs_impl.hpp:9-89).
+//
+// A row of a row-major block (X[col*k+v], Y[row*k+v]) is k contiguous values,
+// read as 16-, 8- or 4-byte vectors, the widest that k and the addresses
+// allow.  Two kernels, each summing a row's products in stored order:
+//
+// * spmm_group_kernel, the default.  G lanes share a row of A, NV vectors
+//   each, for any G up to 32, so block widths that are no power of two keep
+//   nearly all lanes busy.  One CTA per SM goes through a contiguous range of
+//   rows (the rows of X that neighbouring rows share are still in its L1), and
+//   a row's (col, val) pairs are in shared memory (cp.async) before they are
+//   needed.  Bound by L1 wavefronts and the latency of the X rows.
+// * spmm_row_major_kernel, a grid of all rows, for regular matrices where it
+//   is the faster one (grid_suits).  Bound by L2 bandwidth when a row of X is
+//   wide: it holds twice the warps.
+//
+// Column-major blocks are transposed into a row-major workspace (one pass over
+// X) and run the group kernel, which writes Y column-major: A is read once
+// and not once per vector.
+//
+// Measured before and after (before: the grid kernel, a warp per row for
+// widths that are no power of two, k SpMVs for column-major blocks):
+//   27-point 128^3, k = 16, FP64              635 -> 489 us
+//   27-point 96^3, k = 5, FP64                560 -> 136 us
+//   27-point 96^3, k = 8, column-major, FP64  664 -> 191 us
+//   lognormal 600000 rows, k = 20, FP32       366 -> 208 us
+//   lognormal 500000 rows, k = 16, FP64       569 -> 256 us
 #include "spmv_formats.cuh"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace smax {
 
@@ -114,22 +134,281 @@ __global__ void __launch_bounds__(256) spmm_row_major_kernel(const int *__restri
     spmm_row<VT, G, NV, VEC>(row, lane % G, group_mask<G>(lane), row_ptr, col, val, k, X, Y);
 }
 
-// CTA b walks rows ranges[b] .. ranges[b+1] in order, kWalkThreads / G rows
-// at a time
-constexpr int kWalkThreads = 1024;
-template <typename VT, int G, int NV, int VEC>
-__global__ void __launch_bounds__(kWalkThreads, 1)
-    spmm_walk_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col, const VT *__restrict__ val,
-                     const int64_t *__restrict__ ranges, int64_t k, const VT *__restrict__ X, VT *__restrict__ Y) {
-    const int lane = threadIdx.x & 31;
-    const int64_t r0 = ranges[blockIdx.x], r1 = ranges[blockIdx.x + 1];
-    for (int64_t row = r0 + threadIdx.x / G; row < r1; row += kWalkThreads / G)
-        spmm_row<VT, G, NV, VEC>(row, lane % G, group_mask<G>(lane), row_ptr, col, val, k, X, Y);
+// -------------------------------------------------------------- groups ----
+// Warps of a CTA (one CTA per SM) and entries whose rows of X are loaded at a
+// time, by the vectors a lane holds.  One vector: 24 warps of four entries (27-
+// point 128^3, k = 16 FP64: 16 warps of eight took 713 us, 24 of four 569, both
+// with rows taken from the counter).  More: 16 warps, which have the registers
+// for it (lognormal, k = 48 FP64: 807 us against 957 with 24).
+__host__ __device__ constexpr int group_warps(int nv) { return nv == 1 ? 24 : 16; }
+__host__ __device__ constexpr int group_unroll(int nv) { return nv == 4 ? 2 : 4; }
+constexpr int kStagePad = 4;  // entries between the staged rows: their 16-byte reads spread over the banks
+
+// bytes of one stage of a warp: RW rows of CH + kStagePad values, then columns
+template <typename VT> __host__ __device__ constexpr int stage_bytes(int rw, int ch) {
+    return rw * (ch + kStagePad) * (int)(sizeof(VT) + sizeof(int));
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp_async4(unsigned dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(unsigned dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// VB bytes of X as VB / sizeof(VT) values
+template <typename VT, int VB> struct XVec {
+    static constexpr int N = VB / (int)sizeof(VT);
+    VT v[N];
+    __device__ __forceinline__ void load(const VT *p) {
+        if constexpr (VB == 16 && sizeof(VT) == 8) {
+            const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
+            v[0] = a.x; v[1] = a.y;
+        } else if constexpr (VB == 16) {
+            const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        } else if constexpr (VB == 8 && sizeof(VT) == 4) {
+            const float2 a = __ldg(reinterpret_cast<const float2 *>(p));
+            v[0] = a.x; v[1] = a.y;
+        } else {
+            v[0] = __ldg(p);
+        }
+    }
+};
+
+template <typename VT> __device__ __forceinline__ void read4(const VT *p, VT (&v)[4]) {
+    if constexpr (sizeof(VT) == 8) {
+        const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    } else {
+        const float4 a = *reinterpret_cast<const float4 *>(p);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    }
+}
+
+// U staged entries: their rows of X are all loaded before the first is used.
+template <typename VT, int VB, int NV, int U>
+__device__ __forceinline__ void take(const int *sc, const VT *sv, const VT *const (&xl)[NV], int ldx,
+                                     VT (&acc)[NV][XVec<VT, VB>::N]) {
+    XVec<VT, VB> x[U][NV];
+    int c[U];
+    if constexpr (U % 4 == 0) {
+#pragma unroll
+        for (int u = 0; u < U; u += 4) {
+            const int4 c4 = *reinterpret_cast<const int4 *>(sc + u);
+            c[u] = c4.x; c[u + 1] = c4.y; c[u + 2] = c4.z; c[u + 3] = c4.w;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) c[u] = sc[u];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int m = 0; m < NV; ++m) x[u][m].load(xl[m] + (int64_t)c[u] * ldx);
+    VT v[U];
+    if constexpr (U % 4 == 0) {
+#pragma unroll
+        for (int u = 0; u < U; u += 4) {
+            VT v4[4];
+            read4<VT>(sv + u, v4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[u + i] = v4[i];
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = sv[u];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int m = 0; m < NV; ++m)
+#pragma unroll
+            for (int i = 0; i < XVec<VT, VB>::N; ++i) acc[m][i] += v[u] * x[u][m].v[i];
+}
+
+// Columns [0, kcols) of one panel: nvec vectors of a row of X (row stride ldx
+// values).  COL: Y is column-major, element (row, v) at row + v * ldy, else
+// row-major with row stride ldy.
+// REG: no row has more than CH entries; rows are then dealt out in turn and a
+// row is one chunk.  Otherwise the groups take rows from a shared counter.
+template <typename VT, int VB, int NV, bool COL, bool REG>
+__global__ void __launch_bounds__(group_warps(NV) * 32, 1)
+    spmm_group_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col, const VT *__restrict__ val,
+                      const int64_t *__restrict__ ranges, int G, int ch_shift, int nvec, int kcols, int ldx,
+                      const VT *__restrict__ X, VT *__restrict__ Y, int64_t ldy) {
+    using XV = XVec<VT, VB>;
+    constexpr int VEC = XV::N;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int next_row;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int RW = 32 / G, CH = 1 << ch_shift;
+    const int g = min(lane / G, RW - 1), gl = lane - g * G;  // lanes past the last group have gl >= G
+    const int stage = stage_bytes<VT>(RW, CH);
+    VT *sv0 = reinterpret_cast<VT *>(smem + (size_t)warp * 2 * stage) + g * (CH + kStagePad);
+    int *sc0 = reinterpret_cast<int *>(smem + (size_t)warp * 2 * stage + RW * (CH + kStagePad) * sizeof(VT)) +
+               g * (CH + kStagePad);
+    const int r0 = (int)ranges[blockIdx.x], r1 = (int)ranges[blockIdx.x + 1];
+    if constexpr (!REG) {
+        if (threadIdx.x == 0) next_row = r0;
+        __syncthreads();
+    }
+    const bool worker = gl < G;
+
+    // the lane's vectors of a row; a lane without an m-th vector reads vector 0 and stores nothing
+    const VT *xl[NV];
+#pragma unroll
+    for (int m = 0; m < NV; ++m) xl[m] = X + (worker && m * G + gl < nvec ? (m * G + gl) * VEC : 0);
+
+    // the group's next row and its bounds (row >= r1: none left)
+    auto grab = [&](bool need, int &row, int &s, int &e) {
+        // one atomic per warp for the groups that need a row
+        const unsigned want = __ballot_sync(0xffffffffu, need && gl == 0);
+        if (!want) return;
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&next_row, __popc(want));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (need) {
+            row = base + __popc(want & ((1u << (g * G)) - 1u));
+            s = e = 0;
+            if (row < r1) {
+                s = row_ptr[row];
+                e = row_ptr[row + 1];
+            }
+        }
+    };
+    // entries [at, at + CH) of a row that ends at e into stage b
+    auto issue = [&](int b, int at, int e) {
+        VT *sv = reinterpret_cast<VT *>(reinterpret_cast<unsigned char *>(sv0) + b * stage);
+        int *sc = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(sc0) + b * stage);
+        if (worker)
+            for (int j = gl; j < CH && at + j < e; j += G) {
+                cp_async4(smem_u32(sc + j), col + at + j);
+                if constexpr (sizeof(VT) == 8) cp_async8(smem_u32(sv + j), val + at + j);
+                else cp_async4(smem_u32(sv + j), val + at + j);
+            }
+        cp_async_commit();
+    };
+
+    VT acc[NV][VEC];
+#pragma unroll
+    for (int m = 0; m < NV; ++m)
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) acc[m][i] = VT(0);
+
+    // the entries of a staged chunk, n of them, into acc
+    auto chunk = [&](int b, int n) {
+        const VT *sv = reinterpret_cast<const VT *>(reinterpret_cast<unsigned char *>(sv0) + b * stage);
+        const int *sc = reinterpret_cast<const int *>(reinterpret_cast<unsigned char *>(sc0) + b * stage);
+        // U entries' vectors of X are loaded before any is used; with several vectors a
+        // lane, fewer entries at a time, for the same bytes in flight
+        constexpr int U = group_unroll(NV);
+        int j = 0;
+        for (; j + U <= n; j += U) take<VT, VB, NV, U>(sc + j, sv + j, xl, ldx, acc);
+        if constexpr (U > 2)
+            if (j + 2 <= n) {
+                take<VT, VB, NV, 2>(sc + j, sv + j, xl, ldx, acc);
+                j += 2;
+            }
+        if (j < n) take<VT, VB, NV, 1>(sc + j, sv + j, xl, ldx, acc);
+    };
+    // the finished row to Y, and acc back to zero
+    auto finish = [&](int row) {
+#pragma unroll
+        for (int m = 0; m < NV; ++m) {
+            const int off = (m * G + gl) * VEC;
+            if (worker && row < r1 && m * G + gl < nvec) {
+                if constexpr (COL) {
+#pragma unroll
+                    for (int i = 0; i < VEC; ++i)
+                        if (off + i < kcols) __stcs(Y + (int64_t)(off + i) * ldy + row, acc[m][i]);
+                } else {
+                    VT *y = Y + (int64_t)row * ldy + off;
+                    if constexpr (VB == 16 && sizeof(VT) == 8)
+                        __stcs(reinterpret_cast<double2 *>(y), make_double2(acc[m][0], acc[m][1]));
+                    else if constexpr (VB == 16)
+                        __stcs(reinterpret_cast<float4 *>(y),
+                               make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]));
+                    else if constexpr (VB == 8 && sizeof(VT) == 4)
+                        __stcs(reinterpret_cast<float2 *>(y), make_float2(acc[m][0], acc[m][1]));
+                    else
+                        __stcs(y, acc[m][0]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) acc[m][i] = VT(0);
+        }
+    };
+
+    int row, s, e, row1, s1, e1, b = 0;
+    if constexpr (REG) {
+        const int stride = (int)(blockDim.x >> 5) * RW;
+        auto bounds = [&](int r, int &s, int &e) {
+            s = e = 0;
+            if (r < r1) {
+                s = row_ptr[r];
+                e = row_ptr[r + 1];
+            }
+        };
+        int wr = r0 + warp * RW;  // the warp's first row
+        row = wr + g;
+        bounds(row, s, e);
+        issue(0, s, e);
+        bounds(row + stride, s1, e1);
+        for (; wr < r1; wr += stride, row += stride, b ^= 1) {
+            issue(b ^ 1, s1, e1);
+            int s2, e2;
+            bounds(row + 2 * stride, s2, e2);
+            cp_async_wait<1>();
+            __syncwarp();
+            chunk(b, e - s);
+            __syncwarp();
+            finish(row);
+            s = s1;
+            e = e1;
+            s1 = s2;
+            e1 = e2;
+        }
+    } else {
+        // row: computed; row1: staged next; row2: its bounds are loaded
+        int row2, s2, e2;
+        grab(true, row, s, e);
+        grab(true, row1, s1, e1);
+        grab(true, row2, s2, e2);
+        issue(0, s, e);
+        while (__any_sync(0xffffffffu, row < r1)) {
+            const bool more = e - s > CH;
+            issue(b ^ 1, more ? s + CH : s1, more ? e : e1);
+            cp_async_wait<1>();
+            __syncwarp();
+            chunk(b, min(e - s, CH));
+            __syncwarp();
+            if (more) {
+                s += CH;
+            } else {
+                finish(row);
+                row = row1;
+                s = s1;
+                e = e1;
+                row1 = row2;
+                s1 = s2;
+                e1 = e2;
+            }
+            grab(!more, row2, s2, e2);
+            b ^= 1;
+        }
+    }
+    cp_async_wait<0>();
 }
 
 // ranges[b] = first row r with row_ptr[r] + r >= b * (nnz + n) / grid
 // (nonzeros and rows balanced: a row costs its entries plus its Y write)
-__global__ void walk_ranges_kernel(const int *__restrict__ row_ptr, int64_t n, int grid, int64_t *__restrict__ ranges) {
+__global__ void row_ranges_kernel(const int *__restrict__ row_ptr, int64_t n, int grid, int64_t *__restrict__ ranges) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b > grid) return;
     const int64_t total = (int64_t)row_ptr[n] + n;
@@ -143,41 +422,93 @@ __global__ void walk_ranges_kernel(const int *__restrict__ row_ptr, int64_t n, i
     ranges[b] = b == grid ? n : lo;
 }
 
-template <typename VT, int G, int NV, int VEC>
-void launch_rm(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStream_t st, const SpmmPlan *walk) {
-    if (walk) {
-        static bool carve[64] = {};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev >= 0 && dev < 64 && !carve[dev]) {
-            // no shared memory: the whole unified L1 holds X rows
-            SMAX_CUDA(cudaFuncSetAttribute(spmm_walk_kernel<VT, G, NV, VEC>,
-                                           cudaFuncAttributePreferredSharedMemoryCarveout, 0));
-            carve[dev] = true;
-        }
-        spmm_walk_kernel<VT, G, NV, VEC><<<walk->grid, kWalkThreads, 0, st>>>(
-            a.rp(), a.ci(), a.val.template as<VT>(), walk->ranges.as<int64_t>(), k, X, Y);
-        return;
+// T (n x kp, row-major, kp >= k, zeros beyond column k) = X (column-major, leading dimension ld)
+constexpr int kTrRows = 32;
+template <typename VT>
+__global__ void __launch_bounds__(256) to_row_major_kernel(const VT *__restrict__ X, int64_t n, int k, int kp,
+                                                           int64_t ld, VT *__restrict__ T) {
+    // 32 rows by up to 64 columns through shared memory: both sides coalesced
+    __shared__ VT tile[64][kTrRows + 1];
+    const int64_t r0 = (int64_t)blockIdx.x * kTrRows;
+    const int v0 = blockIdx.y * 64, nv = min(64, kp - v0);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int v = w; v < nv; v += 8)
+        tile[v][lane] = (v0 + v < k && r0 + lane < n) ? ld_stream(X + (int64_t)(v0 + v) * ld + r0 + lane) : VT(0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kTrRows * nv; i += 256) {
+        const int r = i / nv, v = i - r * nv;
+        if (r0 + r < n) T[(r0 + r) * kp + v0 + v] = tile[v][r];
     }
+}
+
+template <typename VT, int G, int NV, int VEC>
+void launch_rm(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStream_t st) {
     const uint64_t threads = (uint64_t)a.n_rows * G;
     spmm_row_major_kernel<VT, G, NV, VEC><<<ceil_div_u(threads, 256), 256, 0, st>>>(a.rp(), a.ci(),
                                                                                     a.val.template as<VT>(),
                                                                                     a.n_rows, k, X, Y);
 }
 
-const SpmmPlan *walk_plan(const DevCRS &a, SpmmPlan *plan, cudaStream_t st) {
-    if (!plan) return nullptr;
-    if (plan->key != a.row_ptr.p || plan->n != a.n_rows || plan->nnz != a.nnz) {
-        plan->grid = sm_count();
-        plan->ranges.ensure(sizeof(int64_t) * (plan->grid + 1));
-        walk_ranges_kernel<<<ceil_div_u((uint64_t)plan->grid + 1, 256), 256, 0, st>>>(a.rp(), a.n_rows, plan->grid,
-                                                                                      plan->ranges.as<int64_t>());
-        SMAX_CUDA(cudaGetLastError());
-        plan->key = a.row_ptr.p;
-        plan->n = a.n_rows;
-        plan->nnz = a.nnz;
+// Lanes per row and vectors per lane for a panel of nvec vectors: the pair
+// that keeps most lanes busy, with at least four rows a warp where it can.
+void group_shape(int nvec, int &G, int &NV) {
+    double best = 0;
+    for (int nv : {1, 2, 4}) {
+        const int gg = (nvec + nv - 1) / nv;
+        if (gg > 32) continue;
+        double score = (double)nvec * (32 / gg) / (32.0 * nv);
+        if (gg > 8) score *= 0.8;
+        score *= nv == 1 ? 1.0 : (nv == 2 ? 0.99 : 0.97);
+        if (score > best) {
+            best = score;
+            G = gg;
+            NV = nv;
+        }
     }
-    return plan;
+}
+
+template <typename VT, int VB, bool COL>
+void launch_groups(const DevCRS &a, const SpmmPlan &p, int64_t k, int64_t ldx, const VT *X, VT *Y, int64_t ldy,
+                   cudaStream_t st) {
+    constexpr int VEC = VB / (int)sizeof(VT);
+    const int64_t nvec_all = (k + VEC - 1) / VEC;
+    const int64_t panels = (nvec_all + 127) / 128;
+    for (int64_t pn = 0; pn < panels; ++pn) {
+        const int64_t v0 = nvec_all * pn / panels, v1 = nvec_all * (pn + 1) / panels;
+        const int nvec = (int)(v1 - v0);
+        const int kcols = (int)std::min<int64_t>(k - v0 * VEC, (int64_t)nvec * VEC);
+        int G = 1, NV = 1;
+        group_shape(nvec, G, NV);
+        const int rw = 32 / G;
+        // a chunk holds a row of mean length, a warp's stage at most 256 entries
+        int shift = 2;
+        while (shift < 5 && (rw << (shift + 1)) <= 256 && (int64_t)a.n_rows << shift < a.nnz) ++shift;
+        // rows of nearly equal length: a chunk that holds the longest
+        bool reg = false;
+        if (p.regular) {
+            int sh = shift;
+            while (sh < 5 && (1 << sh) < p.longest && (rw << (sh + 1)) <= 256) ++sh;
+            reg = (1 << sh) >= p.longest;
+            if (reg) shift = sh;
+        }
+        auto go = [&](auto kern, int warps) {
+            const size_t sm = (size_t)warps * 2 * stage_bytes<VT>(rw, 1 << shift);
+            // set on every call: the attribute belongs to the current device
+            SMAX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            kern<<<p.grid, warps * 32, sm, st>>>(a.rp(), a.ci(), a.val.template as<VT>(), p.ranges.as<int64_t>(), G,
+                                                 shift, nvec, kcols, (int)ldx, X + v0 * VEC,
+                                                 COL ? Y + v0 * VEC * ldy : Y + v0 * VEC, ldy);
+            SMAX_CUDA(cudaGetLastError());
+        };
+        auto pick = [&](auto NVc) {
+            constexpr int N = NVc.value;
+            if (reg) go(spmm_group_kernel<VT, VB, N, COL, true>, group_warps(N));
+            else go(spmm_group_kernel<VT, VB, N, COL, false>, group_warps(N));
+        };
+        if (NV == 1) pick(std::integral_constant<int, 1>());
+        else if (NV == 2) pick(std::integral_constant<int, 2>());
+        else pick(std::integral_constant<int, 4>());
+    }
 }
 
 // scalar fallback for any k: one warp per row, lanes over the k columns
@@ -198,41 +529,70 @@ __global__ void spmm_row_major_generic(const int *__restrict__ row_ptr, const in
 
 }  // namespace
 
+static __global__ void longest_row_kernel(const int *__restrict__ row_ptr, int64_t n, int *__restrict__ longest) {
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int len = r < n ? row_ptr[r + 1] - row_ptr[r] : 0;
+    len = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
+    if ((threadIdx.x & 31) == 0 && len > 0) atomicMax(longest, len);
+}
+
+void SpmmPlan::build(const DevCRS &a, cudaStream_t st) {
+    DevBuf d(sizeof(int));
+    SMAX_CUDA(cudaMemsetAsync(d.p, 0, sizeof(int), st));
+    if (a.n_rows > 0)
+        longest_row_kernel<<<ceil_div_u(a.n_rows, 256), 256, 0, st>>>(a.rp(), a.n_rows, d.as<int>());
+    SMAX_CUDA(cudaMemcpyAsync(&longest, d.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SMAX_CUDA(cudaStreamSynchronize(st));
+    regular = (int64_t)longest * a.n_rows <= 2 * a.nnz + 8 * a.n_rows;
+    grid = sm_count();
+    ranges.ensure(sizeof(int64_t) * (grid + 1));
+    row_ranges_kernel<<<ceil_div_u((uint64_t)grid + 1, 256), 256, 0, st>>>(a.rp(), a.n_rows, grid,
+                                                                           ranges.as<int64_t>());
+    SMAX_CUDA(cudaGetLastError());
+}
+
+// Whether a row-major product runs on the grid of all rows: rows of nearly
+// equal length, a power of two of 16-byte vectors, and either a wide block,
+// whose rows of X are more than an SM keeps (27-point 96^3, grid against
+// groups: k = 64 FP64 655 / 801 us, k = 64 FP32 359 / 396, k = 128 FP64 1199 /
+// 1997; k = 16 FP64 276 / 257), or rows too short to pay for the groups' work
+// per row (7-point 100^3: k = 16 FP64 134 / 154 us, k = 16 FP32 79 / 83; k = 4
+// FP64 73 / 48), or rows of X of one 16-byte FP64 vector (27-point 96^3, k = 2:
+// 239 / 495 us).  Rows of uneven length always take the groups (lognormal
+// 500000, k = 64 FP64: 946 against 1543 us).
+static bool grid_suits(const DevCRS &a, const SpmmPlan &p, int64_t nvec, int vbytes) {
+    if (!p.regular || nvec <= 0 || nvec > 128 || (nvec & (nvec - 1))) return false;
+    return nvec >= 16 || (nvec >= 4 && a.nnz <= 12 * a.n_rows) || (nvec == 1 && vbytes == 8);
+}
+
 template <typename VT>
-void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStream_t st, SpmmPlan *plan,
+void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStream_t st, const SpmmPlan &plan,
                         int variant) {
     if (a.n_rows == 0 || k == 0) return;
-    const SpmmPlan *w = variant == 2 ? walk_plan(a, plan, st) : nullptr;
     constexpr int VEC = V16<VT>::N;
-    // vector path when k is a multiple of VEC: k/VEC vectors spread over G lanes
-    // (and X, Y 16-byte aligned: offsets given to apply() may shift them)
-    const bool aligned = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15) == 0;
-    const int64_t nvec = (aligned && k % VEC == 0) ? k / VEC : 0;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y) | (k * sizeof(VT));
+    const bool grid = variant == 1 || (variant == 0 && grid_suits(a, plan, (bits & 15) == 0 ? k / VEC : 0, sizeof(VT)));
+    if (!grid && k > 1 && k < (1 << 30)) {
+        if ((bits & 15) == 0) launch_groups<VT, 16, false>(a, plan, k, k, X, Y, k, st);
+        else if ((bits & 7) == 0 || sizeof(VT) == 8) launch_groups<VT, 8, false>(a, plan, k, k, X, Y, k, st);
+        else launch_groups<VT, sizeof(VT), false>(a, plan, k, k, X, Y, k, st);
+        return;
+    }
+    const int64_t nvec = (bits & 15) == 0 ? k / VEC : 0;
     bool done = true;
     switch (nvec) {
-    case 1: launch_rm<VT, 1, 1, VEC>(a, k, X, Y, st, w); break;
-    case 2: launch_rm<VT, 2, 1, VEC>(a, k, X, Y, st, w); break;
-    case 4: launch_rm<VT, 4, 1, VEC>(a, k, X, Y, st, w); break;
-    case 8: launch_rm<VT, 8, 1, VEC>(a, k, X, Y, st, w); break;
-    // 16 and 32 vectors: 8 lanes per row with 2 / 4 vectors each (k = 64 on
-    // the 27-point stencil: FP32 0.99 -> 0.84 ms, FP64 2.05 -> 1.58 ms against
-    // one vector per lane); 64 vectors: 16 lanes with 4 each (k = 128 FP64
-    // 2.91 -> 2.85 ms, k = 256 FP32 2.84 -> 2.73 ms); more vectors per lane
-    // cost occupancy
-    case 16: launch_rm<VT, 8, 2, VEC>(a, k, X, Y, st, w); break;
-    case 32: launch_rm<VT, 8, 4, VEC>(a, k, X, Y, st, w); break;
-    case 64: launch_rm<VT, 16, 4, VEC>(a, k, X, Y, st, w); break;
-    case 128: launch_rm<VT, 32, 4, VEC>(a, k, X, Y, st, w); break;
+    case 1: launch_rm<VT, 1, 1, VEC>(a, k, X, Y, st); break;
+    case 2: launch_rm<VT, 2, 1, VEC>(a, k, X, Y, st); break;
+    case 4: launch_rm<VT, 4, 1, VEC>(a, k, X, Y, st); break;
+    case 8: launch_rm<VT, 8, 1, VEC>(a, k, X, Y, st); break;
+    case 16: launch_rm<VT, 8, 2, VEC>(a, k, X, Y, st); break;
+    case 32: launch_rm<VT, 8, 4, VEC>(a, k, X, Y, st); break;
+    case 64: launch_rm<VT, 16, 4, VEC>(a, k, X, Y, st); break;
+    case 128: launch_rm<VT, 32, 4, VEC>(a, k, X, Y, st); break;
     default: done = false;
     }
     if (!done) {
-        // k not a power-of-two number of vectors: small k -> scalar lanes per
-        // element, otherwise one warp per row
-        if (k == 1) launch_rm<VT, 1, 1, 1>(a, k, X, Y, st, w);
-        else if (k == 2) launch_rm<VT, 2, 1, 1>(a, k, X, Y, st, w);
-        else if (k == 4) launch_rm<VT, 4, 1, 1>(a, k, X, Y, st, w);
-        else if (k == 8) launch_rm<VT, 8, 1, 1>(a, k, X, Y, st, w);
-        else if (k == 16) launch_rm<VT, 16, 1, 1>(a, k, X, Y, st, w);
+        if (k == 1) launch_rm<VT, 1, 1, 1>(a, k, X, Y, st);
         else
             spmm_row_major_generic<VT><<<ceil_div_u((uint64_t)a.n_rows * 32, 256), 256, 0, st>>>(
                 a.rp(), a.ci(), a.val.template as<VT>(), a.n_rows, k, X, Y);
@@ -240,9 +600,30 @@ void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStre
     SMAX_CUDA(cudaGetLastError());
 }
 
-template void crs_spmm_row_major<double>(const DevCRS &, int64_t, const double *, double *, cudaStream_t, SpmmPlan *,
-                                         int);
-template void crs_spmm_row_major<float>(const DevCRS &, int64_t, const float *, float *, cudaStream_t, SpmmPlan *,
-                                        int);
+int64_t spmm_col_major_work(int64_t n_cols, int64_t k, int vbytes) {
+    const int64_t per = 16 / vbytes, kp = (k + per - 1) / per * per;
+    return n_cols * kp * vbytes;
+}
+
+template <typename VT>
+void crs_spmm_col_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, int64_t ld, VT *work, cudaStream_t st,
+                        const SpmmPlan &plan) {
+    if (a.n_rows == 0 || k == 0) return;
+    constexpr int VEC = V16<VT>::N;
+    const int64_t kp = (k + VEC - 1) / VEC * VEC;
+    to_row_major_kernel<VT><<<dim3(ceil_div_u(a.n_cols, kTrRows), ceil_div_u(kp, 64)), 256, 0, st>>>(
+        X, a.n_cols, (int)k, (int)kp, ld, work);
+    SMAX_CUDA(cudaGetLastError());
+    launch_groups<VT, 16, true>(a, plan, k, kp, work, Y, ld, st);
+}
+
+template void crs_spmm_col_major<double>(const DevCRS &, int64_t, const double *, double *, int64_t, double *,
+                                         cudaStream_t, const SpmmPlan &);
+template void crs_spmm_col_major<float>(const DevCRS &, int64_t, const float *, float *, int64_t, float *,
+                                        cudaStream_t, const SpmmPlan &);
+template void crs_spmm_row_major<double>(const DevCRS &, int64_t, const double *, double *, cudaStream_t,
+                                         const SpmmPlan &, int);
+template void crs_spmm_row_major<float>(const DevCRS &, int64_t, const float *, float *, cudaStream_t,
+                                        const SpmmPlan &, int);
 
 }  // namespace smax

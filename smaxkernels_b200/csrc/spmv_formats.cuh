@@ -61,20 +61,24 @@ void crs_to_bcrs(const DevCRS &a, int vbytes, int64_t bh, int64_t bw, int64_t hp
 // Y = A X with k right-hand sides.  Row-major: X[col*k+v], Y[row*k+v].
 // Column-major: X[ldx*v+col], Y[row+ldy*v] (the reference uses A's n_rows as
 // the leading dimension of X and Y, src/kernels/spmm/spmm_cpu/spmm_cpu_crs_impl.hpp:29,44).
-// Row-major SpMM launch plan.  variant 1: one thread group per row over a
-// grid of all rows.  variant 2 ("walk"): one CTA per SM, each walking a
-// contiguous, nonzero-balanced range of rows in order, so the X rows that
-// neighbouring rows share can stay in that SM's L1 (an autotuner candidate:
-// on the 27-point stencil it loses to the grid's occupancy).  variant 0: the
-// grid.
+// Row ranges of the SpMM kernel's CTAs: contiguous, each with its share of the nonzeros and rows.
 struct SpmmPlan {
-    DevBuf ranges;  // int64 row bounds of the walk CTAs, grid + 1 entries
+    DevBuf ranges;  // int64 row bounds, grid + 1 entries
     int grid = 0;
-    const void *key = nullptr;
-    int64_t n = -1, nnz = -1;
+    int longest = 0;       // entries of the longest row
+    bool regular = false;  // ... at most twice the mean plus 8
+    DevBuf work;    // column-major blocks: X as a row-major block
+    void build(const DevCRS &a, cudaStream_t st);
 };
+// variant 0: chosen by the matrix and the block's width; 1: a grid of all
+// rows; 2: lane groups going through a range of rows per SM
 template <typename VT>
-void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStream_t st, SpmmPlan *plan = nullptr,
+void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStream_t st, const SpmmPlan &plan,
                         int variant = 0);
+// bytes of workspace crs_spmm_col_major needs for k vectors
+int64_t spmm_col_major_work(int64_t n_cols, int64_t k, int vbytes);
+template <typename VT>
+void crs_spmm_col_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, int64_t ld, VT *work, cudaStream_t st,
+                        const SpmmPlan &plan);
 
 }  // namespace smax
