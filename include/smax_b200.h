@@ -97,7 +97,8 @@ typedef int smax_status;
 #define SMAX_FLAG_TEST_FORCE_TIMEOUT 14 /* test only: the persistent solve's barrier waits for a missing arrival */
 #define SMAX_FLAG_REFINE 15            /* float64 SpTRSV: solve in FP32, then this many FP64-residual corrections (0: off) */
 #define SMAX_FLAG_REFINE_TOL 16        /* stop refining once max|dx| <= 10^-value * max|x| (host check per step; 0: run all) */
-#define SMAX_FLAG_SWEEP_CLUSTER 17     /* SpTRSV: runs with levels wider than 1024 rows on a thread-block cluster (0: one CTA) */
+#define SMAX_FLAG_SWEEP_CLUSTER 17     /* SpTRSV: accepted and kept; every run of levels is swept by one CTA, which
+                                          measured faster than a thread-block cluster at every width */
 #define SMAX_FLAG_SPMV_PIPELINE 18     /* CRS SpMV with host pointers: B row blocks, block b with 2^b/(2^B-1) of the entries, whose y is downloaded while later blocks compute (default 6, at most 16 used; 0/1: off) */
 #define SMAX_FLAG_TIMERS 19            /* 1 (default): time every apply with a pair of CUDA events (timer "apply", SpGEMM's phases); 0: no events, those timers stay 0.  A timing event between launches costs about 2.5 us of device time */
 
@@ -253,8 +254,7 @@ smax_status smax_kernel_get_refine_stats(smax_kernel k, int *steps, double *last
 /* --------------------------------------------------------------- autotuning */
 /* Times the launch variants of an initialized kernel on its registered
  * operands and keeps the fastest: the CRS SpMV kernel for SpMV; the solve
- * mode, the level-merge threshold and (SpTRSV) cluster runs for SpTRSV /
- * SpTRSM.  Choices are cached
+ * mode and the level-merge threshold for SpTRSV / SpTRSM.  Choices are cached
  * for the life of the process per matrix (kernel type, value type, sizes and
  * a hash of the pattern); a later kernel with the same matrix takes them from
  * the cache.  Overwrites the output operand (C for SpMV, B for solves). */
@@ -262,7 +262,7 @@ typedef struct smax_tuning {
     int spmv_variant; /* SMAX_FLAG_SPMV_VARIANT chosen (SpMV, row-major SpMM) */
     int solve_mode;   /* SMAX_SOLVE_* chosen (SpTRSV / SpTRSM) */
     int level_merge;  /* SMAX_FLAG_LEVEL_MERGE chosen (SpTRSV / SpTRSM) */
-    int sweep_cluster; /* SMAX_FLAG_SWEEP_CLUSTER chosen (SpTRSV) */
+    int sweep_cluster; /* SMAX_FLAG_SWEEP_CLUSTER as set (SpTRSV) */
     int from_cache;   /* 1: taken from the process-wide cache */
     int n_candidates; /* configurations timed (0 from the cache) */
     double seconds;   /* one apply with the choice */

@@ -63,6 +63,7 @@ DevStatus *dstatus(smax_kernel_s *k) { return k->status.as<DevStatus>(); }
 bool is_tri(const smax_kernel_s *k) { return k->ktype == SMAX_KERNEL_SPTRSV || k->ktype == SMAX_KERNEL_SPTRSM; }
 
 void tri_plan(smax_kernel_s *k) {
+    k->tri.status = dstatus(k);
     if (k->f_perm) {
         require(k->ctx != nullptr && k->ctx->n_levels > 0, SMAX_ERR_STATE,
                 "level-scheduled solve needs the levels of generate_perm in the context");
@@ -228,7 +229,6 @@ void tri_upload(smax_kernel_s *k) {
 
 template <typename VT> void tri_apply_t(smax_kernel_s *k, const VT *Bv, VT *Xv) {
     tri_plan(k);
-    k->tri.set_allow_cluster(k->sweep_cluster);
     if constexpr (sizeof(VT) == 8) {
         if (k->refine_steps > 0) {
             require(k->ktype == SMAX_KERNEL_SPTRSV, SMAX_ERR_UNSUPPORTED,

@@ -108,23 +108,18 @@ void tune_kernel(smax_kernel_s *k, smax_tuning &r) {
         }
         k->spmv_variant = r.spmv_variant;
     } else if (is_tri(k)) {
-        struct Cand { int mode, merge; bool cluster; };
+        struct Cand { int mode, merge; };
         std::vector<Cand> cands;
-        for (int m : {0, 1024, 4096, 16384, 65536}) cands.push_back({SMAX_SOLVE_GRAPH, m, false});
+        for (int m : {0, 1024, 2048, 4096, 8192, 16384, 65536}) cands.push_back({SMAX_SOLVE_GRAPH, m});
         const bool one_rhs = k->ktype == SMAX_KERNEL_SPTRSV || (k->B.n_cols <= 1);
-        if (k->ktype == SMAX_KERNEL_SPTRSV) {
-            cands.push_back({SMAX_SOLVE_GRAPH, 4096, true});
-            cands.push_back({SMAX_SOLVE_GRAPH, 16384, true});
-        }
         if (k->ktype == SMAX_KERNEL_SPTRSV && one_rhs && k->refine_steps == 0) {
-            cands.push_back({SMAX_SOLVE_PERSISTENT, 0, false});
-            cands.push_back({SMAX_SOLVE_SYNCFREE, 0, false});
+            cands.push_back({SMAX_SOLVE_PERSISTENT, 0});
+            cands.push_back({SMAX_SOLVE_SYNCFREE, 0});
         }
-        if (k->ktype == SMAX_KERNEL_SPTRSM) cands.push_back({SMAX_SOLVE_SYNCFREE, 0, false});
+        if (k->ktype == SMAX_KERNEL_SPTRSM) cands.push_back({SMAX_SOLVE_SYNCFREE, 0});
         for (const Cand &c : cands) {
             k->solve_mode = c.mode;
             k->level_merge = c.merge;
-            k->sweep_cluster = c.cluster;
             double t;
             try {
                 t = time_apply(k);
@@ -134,11 +129,10 @@ void tune_kernel(smax_kernel_s *k, smax_tuning &r) {
                 continue;
             }
             ++r.n_candidates;
-            if (t < best) { best = t; r.solve_mode = c.mode; r.level_merge = c.merge; r.sweep_cluster = c.cluster; }
+            if (t < best) { best = t; r.solve_mode = c.mode; r.level_merge = c.merge; }
         }
         k->solve_mode = r.solve_mode;
         k->level_merge = r.level_merge;
-        k->sweep_cluster = r.sweep_cluster != 0;
     } else {
         best = time_apply(k);
         r.n_candidates = 1;

@@ -204,65 +204,75 @@ void TriPlan::finish(cudaStream_t) {
     graph_valid = false;
     pack_ok = false;
     pack_unfit = false;
-    pack = LevelPack();
+    pack = SweepPack();
     sf_ok = false;
     sf_unfit = false;
     sf_pack = LevelPack();
 }
 
 bool TriPlan::ensure_pack(const int *rp, const int *ci, const void *val, const void *D, int vbytes, int merge_rows,
-                          uint64_t tag, cudaStream_t st) {
-    if (scheduled_k != 1 || scheduled_merge != merge_rows) schedule(1, merge_rows);
-    if (pack_ok && pack_key[0] == val && pack_key[1] == D && pack_tag == tag && pack_merge == merge_rows &&
-        pack_vbytes == vbytes)
-        return true;
+                          uint64_t tag, cudaStream_t st, int64_t k) {
     if (pack_unfit) return false;  // a property of the pattern and the level sets
-    const int L = n_levels();
-    std::vector<int> src_begin(L), count(L), seg_begin(L);
-    pack_steps.clear();
-    for (const Step &s : steps) {
-        for (int i = 0; i < s.sweep_count; ++i) {
-            const int sw = s.sweep_first + i;
-            const int lv = descending ? L - 1 - sw : sw;
-            src_begin[sw] = lvl_ptr[lv];
-            count[sw] = lvl_ptr[lv + 1] - lvl_ptr[lv];
-            seg_begin[sw] = s.kind == 1 ? s.sweep_first : sw;
+    if (!pack_is(val, D, vbytes, merge_rows, pack_tag, k)) {
+        if (scheduled_k != 1 || scheduled_merge != merge_rows) schedule(1, merge_rows);
+        const int L = n_levels();
+        std::vector<int> src_begin(L), count(L);
+        std::vector<SweepStep> sweep;
+        for (const Step &s : steps) {
+            for (int i = 0; i < s.sweep_count; ++i) {
+                const int sw = s.sweep_first + i;
+                const int lv = descending ? L - 1 - sw : sw;
+                src_begin[sw] = lvl_ptr[lv];
+                count[sw] = lvl_ptr[lv + 1] - lvl_ptr[lv];
+            }
+            sweep.push_back(SweepStep{s.sweep_first, s.sweep_count, s.kind});
         }
-        pack_steps.push_back(PackStep{s.sweep_first, s.sweep_count, s.kind});
+        release_graph();
+        pack_ok = false;
+        const bool ok = build_sweep_pack(pack, rp, ci, val, D, vbytes, n_rows, has_order ? order.as<int>() : nullptr,
+                                         src_begin, count, sweep, k > 1, false, st);
+        if (!ok) {
+            pack_unfit = true;
+            return false;
+        }
+        pack_ok = true;
+        pack_key[0] = val;
+        pack_key[1] = D;
+        pack_tag = tag;
+        pack_merge = merge_rows;
+        pack_vbytes = vbytes;
+    } else if (pack_tag != tag) {
+        // new values on the same pattern: in place, so a captured graph stays valid
+        refill_sweep_pack(pack, rp, val, D, st);
+        pack_tag = tag;
     }
-    release_graph();
-    pack_ok = false;
-    const bool ok = build_level_pack(pack, rp, ci, val, D, vbytes, n_rows, has_order ? order.as<int>() : nullptr,
-                                     src_begin, count, seg_begin, allow_cluster, st);
-    if (!ok) {
-        pack_unfit = true;
-        return false;
-    }
-    pack_ok = true;
-    pack_key[0] = val;
-    pack_key[1] = D;
-    pack_tag = tag;
-    pack_merge = merge_rows;
-    pack_vbytes = vbytes;
+    const void *before = pack.bp.p;
+    sweep_reserve(pack, k);
+    if (pack.bp.p != before) release_graph();
     return true;
 }
 
 bool TriPlan::ensure_syncfree(const int *rp, const int *ci, const void *val, const void *D, int vbytes, uint64_t tag,
-                              cudaStream_t st) {
-    if (sf_ok && sf_key[0] == val && sf_key[1] == D && sf_tag == tag && sf_vbytes == vbytes) return true;
+                              bool values, cudaStream_t st) {
+    if (sf_ok && sf_key[0] == val && sf_key[1] == D && sf_vbytes == vbytes) {
+        if (values && sf_tag != tag) {
+            refill_level_pack(sf_pack, rp, val, D, st);
+            sf_tag = tag;
+        }
+        return true;
+    }
     if (sf_unfit) return false;  // a property of the pattern and the level sets
     const int L = n_levels();
-    std::vector<int> src_begin(L), count(L), seg_begin(L);
+    std::vector<int> src_begin(L), count(L);
     for (int sw = 0; sw < L; ++sw) {
         const int lv = descending ? L - 1 - sw : sw;
         src_begin[sw] = lvl_ptr[lv];
         count[sw] = lvl_ptr[lv + 1] - lvl_ptr[lv];
-        seg_begin[sw] = sw;
     }
     sf_ok = false;
     const bool ok = build_level_pack(sf_pack, rp, ci, val, D, vbytes, n_rows, has_order ? order.as<int>() : nullptr,
-                                     src_begin, count, seg_begin, false, st, true);
-    if (!ok || sf_pack.needs_x_init) {
+                                     src_begin, count, st);
+    if (!ok || sf_pack.reads_unsolved) {
         sf_pack = LevelPack();
         sf_unfit = true;
         return false;
@@ -285,6 +295,15 @@ void TriPlan::prepare(int64_t k, int merge_rows, cudaStream_t st) {
     }
 }
 
+// Up to kLeadLevels levels of more than kRunStart rows at the start of a run
+// are launches of their own: their sources are wide levels and rows long
+// solved, which the sweep would read from global memory, and a launch is the
+// faster way through such a level then (a longer row of wide levels is a band,
+// with its sources in the ring).  Rows ordered by level sets, FP64, 200^2:
+// 40.5 us; with 1024 rows 42.9, 2048 48.5, no limit 59.0.
+constexpr int kLeadLevels = 16;
+constexpr int64_t kRunStart = 512;
+
 // Sequence of steps: wide levels alone, runs of narrow levels merged.
 void TriPlan::schedule(int64_t k, int merge_rows) {
     steps.clear();
@@ -292,70 +311,35 @@ void TriPlan::schedule(int64_t k, int merge_rows) {
     const int L = (int)lvl_ptr.size() - 1;
     int l = 0;
     auto level_at = [&](int idx) { return descending ? L - 1 - idx : idx; };
+    auto level_rows = [&](int idx) {
+        const int lv = level_at(idx);
+        return (int64_t)(lvl_ptr[lv + 1] - lvl_ptr[lv]);
+    };
     while (l < L) {
         const int lv = level_at(l);
-        const int64_t m = lvl_ptr[lv + 1] - lvl_ptr[lv];
-        if (merge_rows > 0 && m * k <= merge_rows) {
-            const int l0 = l;
-            while (l < L) {
+        const int64_t m = level_rows(l);
+        int end = l;
+        while (end < L && merge_rows > 0 && level_rows(end) * k <= merge_rows) ++end;
+        if (k == 1) {
+            int lead = l;
+            while (lead < end && lead - l <= kLeadLevels && level_rows(lead) > kRunStart) ++lead;
+            if (lead > l && lead - l <= kLeadLevels) end = l;
+        }
+        if (end > l) {
+            // one run: splitting it by width, with fewer threads for the
+            // narrower stretches, measured slower (FP64 5-point D+L, 512^2 in
+            // natural order: 271 us in three runs, 260 us in one)
+            Step s;
+            s.kind = 1;
+            s.seg_first = (int)seg_ranges.size();
+            s.sweep_first = l;
+            for (; l < end; ++l) {
                 const int lv2 = level_at(l);
-                const int64_t m2 = lvl_ptr[lv2 + 1] - lvl_ptr[lv2];
-                if (m2 * k > merge_rows) break;
-                ++l;
+                seg_ranges.push_back({lvl_ptr[lv2], lvl_ptr[lv2 + 1]});
             }
-            // One right-hand side: the run's single-CTA sweep is sized by its
-            // widest level (256 / 512 / 1024 threads for up to 512 / 1024 /
-            // more rows), and every warp of it passes every level.  Long
-            // stretches of narrower levels become runs of their own, on fewer
-            // threads; stretches shorter than kMinStretch levels stay with a
-            // neighbour (a run boundary costs a launch, and the first level of
-            // a run reads its sources from global memory instead of the ring).
-            std::vector<std::pair<int, int>> parts;  // (first sweep step, width class)
-            auto width_class = [&](int idx) {
-                const int lv2 = level_at(idx);
-                const int64_t m2 = lvl_ptr[lv2 + 1] - lvl_ptr[lv2];
-                return k == 1 ? (m2 <= 512 ? 0 : (m2 <= 1024 ? 1 : 2)) : 0;
-            };
-            for (int i = l0; i < l; ++i) {
-                const int c = width_class(i);
-                if (parts.empty() || parts.back().second != c) parts.push_back({i, c});
-            }
-            constexpr int kMinStretch = 64;
-            for (bool changed = true; changed && parts.size() > 1;) {
-                changed = false;
-                for (size_t i = 0; i < parts.size(); ++i) {
-                    const int end = i + 1 < parts.size() ? parts[i + 1].first : l;
-                    if (end - parts[i].first >= kMinStretch) continue;
-                    // merge the short stretch into its wider neighbour
-                    size_t j;
-                    if (i == 0) j = 1;
-                    else if (i + 1 == parts.size()) j = i - 1;
-                    else j = parts[i - 1].second >= parts[i + 1].second ? i - 1 : i + 1;
-                    const size_t lo = std::min(i, j);
-                    parts[lo].second = std::max(parts[i].second, parts[j].second);
-                    parts.erase(parts.begin() + (long)(lo + 1));
-                    // neighbours of equal class join
-                    if (lo + 1 < parts.size() && parts[lo + 1].second == parts[lo].second)
-                        parts.erase(parts.begin() + (long)(lo + 1));
-                    if (lo > 0 && parts[lo - 1].second == parts[lo].second) parts.erase(parts.begin() + (long)lo);
-                    changed = true;
-                    break;
-                }
-            }
-            for (size_t pi = 0; pi < parts.size(); ++pi) {
-                const int a = parts[pi].first, b = pi + 1 < parts.size() ? parts[pi + 1].first : l;
-                Step s;
-                s.kind = 1;
-                s.seg_first = (int)seg_ranges.size();
-                s.sweep_first = a;
-                for (int i = a; i < b; ++i) {
-                    const int lv2 = level_at(i);
-                    seg_ranges.push_back({lvl_ptr[lv2], lvl_ptr[lv2 + 1]});
-                }
-                s.seg_count = (int)seg_ranges.size() - s.seg_first;
-                s.sweep_count = s.seg_count;
-                steps.push_back(s);
-            }
+            s.seg_count = (int)seg_ranges.size() - s.seg_first;
+            s.sweep_count = s.seg_count;
+            steps.push_back(s);
         } else {
             Step s;
             s.kind = 0;
@@ -385,9 +369,9 @@ template <typename VT>
 void tri_solve_raw(TriPlan &p, const int *rp, const int *ci, const VT *val, const VT *D, const VT *B, VT *X,
                    int64_t k, bool row_major, int64_t ld, int merge_rows, uint64_t tag, cudaStream_t st) {
     if (p.n_rows == 0) return;
-    if (k == 1 && p.pack_ok && p.pack_key[0] == val && p.pack_key[1] == D && p.pack_tag == tag &&
-        p.pack_merge == merge_rows && p.pack_vbytes == (int)sizeof(VT)) {
-        pack_solve<VT>(p.pack, p.pack_steps, B, X, st);
+    const int64_t rs = row_major ? k : 1, vs = row_major ? 1 : ld;
+    if (k == 1 && p.pack_is(val, D, sizeof(VT), merge_rows, tag, 1)) {
+        sweep_solve<VT>(p.pack, B, X, 1, rs, vs, p.status, st);
         return;
     }
     if (p.scheduled_k != k || p.scheduled_merge != merge_rows) p.schedule(k, merge_rows);
@@ -396,7 +380,6 @@ void tri_solve_raw(TriPlan &p, const int *rp, const int *ci, const VT *val, cons
                                   cudaMemcpyHostToDevice, st));
         p.ranges_uploaded = true;
     }
-    const int64_t rs = row_major ? k : 1, vs = row_major ? 1 : ld;
     const int *order = p.has_order ? p.order.as<int>() : nullptr;
     const int2 *ranges = p.d_ranges.as<int2>();
     for (const auto &s : p.steps) {
@@ -417,7 +400,18 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
                      int64_t ld, int merge_rows, uint64_t tag, cudaStream_t caller) {
     if (p.n_rows == 0) return;
     // the pack is built outside the capture (it synchronises); a rebuild drops the graph
-    if (k == 1) p.ensure_pack(a.rp(), a.ci(), a.val.p, D, sizeof(VT), merge_rows, tag, caller);
+    bool packed = false;
+    if (k == 1 || sweep_suits(p)) {
+        try {
+            packed = p.ensure_pack(a.rp(), a.ci(), a.val.p, D, sizeof(VT), merge_rows, tag, caller, k);
+        } catch (const Error &e) {
+            // a block without room for the sweep's workspace runs the level launches
+            if (k == 1 || e.code != SMAX_ERR_OOM) throw;
+            p.pack = SweepPack();
+            p.pack_ok = false;
+            p.release_graph();
+        }
+    }
     // graphs are captured (and replayed) on a capturable stream
     const bool fenced = !is_capturable(caller);
     cudaStream_t st = fenced ? p.aux.enter(caller) : caller;
@@ -432,11 +426,11 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
             }
         }
     } leave{p, fenced, caller};
-    if (p.scheduled_k != k || p.scheduled_merge != merge_rows) p.schedule(k, merge_rows);
+    if (!packed && (p.scheduled_k != k || p.scheduled_merge != merge_rows)) p.schedule(k, merge_rows);
     const void *key[4] = {B, X, D, a.val.p};
     if (!p.graph_valid || p.graph_key[0] != key[0] || p.graph_key[1] != key[1] || p.graph_key[2] != key[2] ||
-        p.graph_key[3] != key[3] || p.graph_row_major != row_major || p.graph_ld != ld) {
-        if (!p.ranges_uploaded && !p.seg_ranges.empty()) {
+        p.graph_key[3] != key[3] || p.graph_row_major != row_major || p.graph_ld != ld || p.graph_k != k || p.graph_packed != packed) {
+        if (!packed && !p.ranges_uploaded && !p.seg_ranges.empty()) {
             SMAX_CUDA(cudaMemcpyAsync(p.d_ranges.p, p.seg_ranges.data(), sizeof(int2) * p.seg_ranges.size(),
                                       cudaMemcpyHostToDevice, st));
             p.ranges_uploaded = true;
@@ -446,7 +440,10 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
         cudaGraph_t g = nullptr;
         SMAX_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         try {
-            tri_solve_raw<VT>(p, a.rp(), a.ci(), a.val.as<VT>(), D, B, X, k, row_major, ld, merge_rows, tag, st);
+            if (packed)
+                sweep_solve<VT>(p.pack, B, X, k, row_major ? k : 1, row_major ? 1 : ld, p.status, st);
+            else
+                tri_solve_raw<VT>(p, a.rp(), a.ci(), a.val.as<VT>(), D, B, X, k, row_major, ld, merge_rows, tag, st);
         } catch (...) {
             cudaStreamEndCapture(st, &g);
             if (g) cudaGraphDestroy(g);
@@ -465,6 +462,8 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
         p.graph_key[3] = key[3];
         p.graph_row_major = row_major;
         p.graph_ld = ld;
+        p.graph_k = k;
+        p.graph_packed = packed;
     }
     SMAX_CUDA(cudaGraphLaunch(p.graph, st));
 }
@@ -477,9 +476,14 @@ void TriPlan::release_graph() {
 
 TriPlan::~TriPlan() { release_graph(); }
 
+bool sweep_suits(const TriPlan &p) {
+    const int64_t L = p.n_levels();
+    return L > 0 && !p.pack_unfit && p.n_rows <= L * 2048;
+}
+
 bool syncfree_suits(const TriPlan &p, int64_t k) {
     const int64_t L = p.n_levels();
-    if (L <= 0) return false;
+    if (L <= 0 || (k > 1 && sweep_suits(p))) return false;
     if (k == 1) return p.n_rows >= (1 << 17) && p.n_rows >= L * 32768;
     return p.n_rows >= (1 << 16) && L >= 64 && p.n_rows <= L * 16384;
 }
@@ -492,7 +496,7 @@ bool tri_solve_syncfree(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, V
     const uintptr_t b0 = reinterpret_cast<uintptr_t>(B), x0 = reinterpret_cast<uintptr_t>(X);
     const uintptr_t len = sizeof(VT) * (uintptr_t)p.n_rows * (uintptr_t)k;
     if (b0 < x0 + len && x0 < b0 + len) return false;  // B is read while X fills
-    if (!p.ensure_syncfree(a.rp(), a.ci(), a.val.p, D, sizeof(VT), tag, s)) return false;
+    if (!p.ensure_syncfree(a.rp(), a.ci(), a.val.p, D, sizeof(VT), tag, k == 1, s)) return false;
     ctl.ensure(64);
     if (k == 1)
         pack_solve_syncfree<VT>(p.sf_pack, B, X, ctl.p, limit, force_timeout, st, s);

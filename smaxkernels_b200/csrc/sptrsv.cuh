@@ -6,6 +6,7 @@
 #include "levelpack.cuh"
 #include "levels.cuh"
 #include "spmv_formats.cuh"
+#include "sweep.cuh"
 
 namespace smax {
 
@@ -44,31 +45,29 @@ struct TriPlan {
     bool graph_valid = false;
     const void *graph_key[4] = {nullptr, nullptr, nullptr, nullptr};
     bool graph_row_major = false;
-    int64_t graph_ld = 0;
+    int64_t graph_ld = 0, graph_k = 0;
+    bool graph_packed = false;
     AuxStream aux;  // capture stream when the caller's stream cannot be captured
 
-    // level-ordered pack for one right-hand side (levelpack.cu), built for the
-    // value arrays, their version tag and the merge threshold below
-    LevelPack pack;
-    std::vector<PackStep> pack_steps;
+    // level-ordered pack (sweep.cu), built for the value arrays, their version
+    // tag, the merge threshold and one or several right-hand sides below
+    SweepPack pack;
     bool pack_ok = false, pack_unfit = false;
-    bool allow_cluster = false;  // runs wider than one CTA covers may use a cluster
-    // sets allow_cluster; a change drops the pack and the graph
-    void set_allow_cluster(bool v) {
-        if (v != allow_cluster) {
-            allow_cluster = v;
-            pack_ok = false;
-            release_graph();
-        }
-    }
     const void *pack_key[2] = {nullptr, nullptr};
     uint64_t pack_tag = ~0ull;
     int pack_merge = -1, pack_vbytes = 0;
-    // (re)builds the pack when its key changed; false when the matrix does
-    // not pack compactly and the plain kernels must be used.  Synchronises:
-    // call outside stream capture.
+    DevStatus *status = nullptr;  // where a sweep reports a wait that gave up
+    // (re)builds the pack when its key changed (new values of the same arrays
+    // are filled in); false when the matrix does not pack compactly and the
+    // plain kernels must be used.  k > 1: rows divide by D, as the plain
+    // kernels do.  Synchronises: call outside stream capture.
     bool ensure_pack(const int *rp, const int *ci, const void *val, const void *D, int vbytes, int merge_rows,
-                     uint64_t tag, cudaStream_t st);
+                     uint64_t tag, cudaStream_t st, int64_t k = 1);
+    // whether the pack is the one a solve with these arguments uses
+    bool pack_is(const void *val, const void *D, int vbytes, int merge_rows, uint64_t tag, int64_t k) const {
+        return pack_ok && pack_key[0] == val && pack_key[1] == D && pack_tag == tag && pack_merge == merge_rows &&
+               pack_vbytes == vbytes && pack.div == (k > 1);
+    }
 
     // sync-free form of the pack (SMAX_SOLVE_SYNCFREE): every level its own
     // step, entries naming source rows; unfit when padding is too large or an
@@ -78,8 +77,9 @@ struct TriPlan {
     const void *sf_key[2] = {nullptr, nullptr};
     uint64_t sf_tag = ~0ull;
     int sf_vbytes = 0;
+    // values = false: only its order of rows is used
     bool ensure_syncfree(const int *rp, const int *ci, const void *val, const void *D, int vbytes, uint64_t tag,
-                         cudaStream_t st);
+                         bool values, cudaStream_t st);
 
     // dependency levels of the matrix itself (plain solve)
     void build_own(const DevCRS &a, bool upper, cudaStream_t st);
@@ -101,8 +101,8 @@ struct TriPlan {
 // column-major: at r + v*ld).  merge_rows: levels with at most this many
 // (row, vector) pairs are merged into single-CTA runs (0 disables merging).
 // `tag` identifies the current values of (val, D): a caller that changes the
-// values in place passes a new tag so the level-ordered pack is rebuilt.
-// With k == 1 the solve runs on the pack (levelpack.cu); tri_solve_raw does
+// values in place passes a new tag so the level-ordered pack takes them over.
+// With k == 1 the solve runs on the pack (sweep.cu); tri_solve_raw does
 // not build it (it may run inside a stream capture): call ensure_pack first.
 template <typename VT>
 void tri_solve(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *X, int64_t k, bool row_major, int64_t ld,
@@ -112,6 +112,9 @@ void tri_solve(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *X, int
 template <typename VT>
 void tri_solve_raw(TriPlan &p, const int *rp, const int *ci, const VT *val, const VT *D, const VT *B, VT *X,
                    int64_t k, bool row_major, int64_t ld, int merge_rows, uint64_t tag, cudaStream_t st);
+// Whether blocks of k > 1 right-hand sides run as sweeps of the pack, one CTA
+// each: levels of at most 2048 rows on average.
+bool sweep_suits(const TriPlan &p);
 // The sync-free solve of one right-hand side (pack_solve_syncfree).  Returns
 // false, launching nothing, when it does not apply: the matrix does not pack,
 // an entry reads a row not solved before it, or B and X overlap.

@@ -6,12 +6,11 @@
 //    next matrix from a device work queue (an atomic counter over the matrices
 //    in longest-first order) and sweeps that matrix's levels, with
 //    __syncthreads() as the level barrier; when done it takes the next one.
-//    The sweep runs on the level-ordered pack of the batch (levelpack.cu:
-//    per-level ELL blocks, a shared-memory ring of recent solutions, the next
-//    level prefetched into registers); matrices that would pack too sparsely
-//    use the plain kernel below.
-//    There is no spin-wait anywhere: the queue is a fetch-add and the level
-//    barrier is the CTA barrier.  The launch (queue reset + kernel) is
+//    The sweep runs on the level-ordered pack of the batch (sweep.cu:
+//    per-level ELL blocks copied ahead into shared memory, a ring of recent
+//    solutions); matrices that would pack too sparsely use the plain kernel
+//    below.  The queue is a fetch-add, the level barrier is the CTA barrier,
+//    and the waits on the copies are bounded.  The launch (queue reset + kernel) is
 //    captured once into a CUDA graph and replayed.
 // 2. Grid-wide persistent (one matrix, wide levels): a cooperative launch of
 //    co-resident CTAs sweeps all levels, with a software grid barrier between
@@ -235,22 +234,24 @@ void TriBatch::build(int vbytes_, const std::vector<RegCRS> &mats, cudaStream_t 
     SMAX_CUDA(cudaStreamSynchronize(st));
     // sweep steps = every matrix's levels in order; each matrix is one run
     const int L = total_levels;
-    std::vector<int> src_begin(L), count(L), seg_begin(L);
-    for (int m = 0; m < n_mats; ++m)
+    std::vector<int> src_begin(L), count(L);
+    std::vector<SweepStep> steps;
+    for (int m = 0; m < n_mats; ++m) {
         for (int l = moff[m]; l < moff[m + 1]; ++l) {
             src_begin[l] = lrows[l];
             count[l] = lrows[l + 1] - lrows[l];
-            seg_begin[l] = moff[m];
         }
-    pack_ok = build_level_pack(pack, A.rp(), A.ci(), A.val.p, D.p, vbytes, n_rows, order.as<int>(), src_begin, count,
-                               seg_begin, false, st);
+        steps.push_back(SweepStep{moff[m], moff[m + 1] - moff[m], 1});
+    }
+    pack_ok = build_sweep_pack(pack, A.rp(), A.ci(), A.val.p, D.p, vbytes, n_rows, order.as<int>(), src_begin, count,
+                               steps, false, true, st);
 }
 
 template <typename VT>
 void TriBatch::solve_persistent(const VT *B, VT *X, cudaStream_t st) {
     if (n_mats == 0) return;
     if (pack_ok) {
-        pack_solve_batch<VT>(pack, mat_lvl_off.as<int>(), queue_order.as<int>(), n_mats, queue.as<int>(), B, X, st);
+        sweep_solve_batch<VT>(pack, queue_order.as<int>(), n_mats, queue.as<int>(), B, X, st);
         return;
     }
     int per_sm = 0;

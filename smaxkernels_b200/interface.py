@@ -253,7 +253,7 @@ class Kernel:
         return self._flag("spin_limit", kilo_polls)
 
     def set_sweep_cluster(self, v: bool):
-        """SpTRSV: let runs with levels wider than 1024 rows use a thread-block cluster."""
+        """SpTRSV: accepted; every run of levels is swept by one CTA (smax_b200.h)."""
         return self._flag("sweep_cluster", int(bool(v)))
 
     def set_level_merge(self, rows: int):

@@ -1,0 +1,195 @@
+"""Level sweeps of triangular solves (SpTRSV, SpTRSM, batches) at the sizes
+where their layout changes: rows of one to many entries, levels at the CTA
+sizes' edges and wider than a CTA, rows too wide for the shared-memory stage,
+sources older than the ring of recent solutions, and new values on the same
+pattern.  Checked against the oracle; blocks of right-hand sides bit for bit
+against the level launches, whose arithmetic they share."""
+import numpy as np
+import pytest
+
+from helpers import normwise, tol
+from oracle.oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+O = Oracle()
+
+
+def level_matrix(sizes, width, seed, vt, reach=None):
+    """Lower triangle whose dependency levels have the given sizes: a row has
+    an entry in the level before its own and up to width - 1 others among the
+    `reach` rows before its level; the diagonal is last."""
+    rng = np.random.default_rng(seed)
+    starts = np.concatenate([[0], np.cumsum(sizes)])
+    rp, cols = [0], []
+    for s, m in enumerate(sizes):
+        a = int(starts[s])
+        lo = 0 if reach is None else max(0, a - reach)
+        for r in range(a, a + m):
+            c = []
+            if s:
+                k = int(rng.integers(1, width + 1))
+                c = {int(rng.integers(starts[s - 1], a))}
+                c |= set(int(v) for v in rng.integers(lo, a, k - 1))
+                c = sorted(c)
+            cols += c + [r]
+            rp.append(len(cols))
+    rp, col = np.array(rp, np.int32), np.array(cols, np.int32)
+    val = rng.uniform(-1, 1, len(col)) / width
+    val[rp[1:] - 1] = rng.uniform(1, 2, len(rp) - 1)
+    return rp, col, val.astype(vt)
+
+
+def _kernel(kind, rp, col, val, b, k=1, row_major=True, mode=0):
+    from smaxkernels_b200 import FloatType, Interface, IntType, KernelType, PlatformType
+    n = len(rp) - 1
+    smax = Interface()
+    smax.register_kernel("t", KernelType[kind], PlatformType.CUDA, IntType.INT32,
+                         FloatType.FLOAT64 if val.dtype == np.float64 else FloatType.FLOAT32)
+    kern = smax.kernel("t")
+    kern.set_solve_mode(mode)
+    kern.set_mat_lower_triang(True)
+    x = np.full(n * k, 7, val.dtype)
+    dims = (n,) if kind == "SPTRSV" else (n, k)
+    if kind == "SPTRSM":
+        kern.set_vec_row_major(row_major)
+    kern.register_A(n, n, len(col), col.copy(), rp, val.copy())
+    kern.register_B(*dims, x)
+    kern.register_C(*dims, b)
+    return smax, kern, x
+
+
+def _solve(*args, **kw):
+    smax, kern, x = _kernel(*args, **kw)
+    kern.run()
+    smax.close()
+    return x
+
+
+EDGES = [1, 2, 3, 4, 5, 31, 33, 127, 128, 129, 1, 255, 256, 257, 479, 480, 481, 607, 608, 609, 1215, 1217, 2000, 7]
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("width", [1, 2, 3, 4, 9, 40])
+@pytest.mark.parametrize("sizes", ["edges", "narrow", "wide"])
+def test_sweep_vs_oracle(vt, width, sizes):
+    sizes = {"edges": EDGES, "narrow": [5, 9, 1, 30] * 60, "wide": [700, 4097, 3, 4096, 50] * 2}[sizes]
+    rp, col, val = level_matrix(sizes, width, width, vt)
+    b = np.random.default_rng(1).uniform(-1, 1, len(rp) - 1).astype(vt)
+    x = _solve("SPTRSV", rp, col, val, b)
+    assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+def test_sweep_reads_solutions_older_than_the_ring(vt):
+    """Recent and old sources mixed: 30000 rows against a ring of 8192."""
+    rp, col, val = level_matrix([600] * 50, 4, 3, vt)
+    b = np.random.default_rng(2).uniform(-1, 1, len(rp) - 1).astype(vt)
+    x = _solve("SPTRSV", rp, col, val, b)
+    assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("side", [96, 700])
+def test_sweep_of_many_records_repeats(vt, side):
+    """5-point lower triangle in natural order: enough records for the copies
+    to go round the stage and their mbarriers many times; every solve is equal."""
+    n = side * side
+    r = np.arange(n)
+    cols = np.stack([np.where(r >= side, r - side, -1), np.where(r % side, r - 1, -1), r], 1)
+    keep = cols >= 0
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    col = cols[keep].astype(np.int32)
+    rng = np.random.default_rng(side)
+    val = (rng.uniform(-1, 1, len(col)) / 4).astype(vt)
+    val[rp[1:] - 1] = rng.uniform(1, 2, n)
+    b = rng.uniform(-1, 1, n).astype(vt)
+    smax, kern, x = _kernel("SPTRSV", rp, col, val, b)
+    kern.run()
+    assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
+    first = x.copy()
+    for _ in range(20):
+        x[:] = 7
+        kern.run()
+        np.testing.assert_array_equal(x, first)
+    smax.close()
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+def test_sweep_rows_too_wide_for_the_stage(vt):
+    """A row of 8000 entries among short ones is read in place."""
+    rng = np.random.default_rng(4)
+    n = 9000
+    rows = [[r - 1, r] if r else [0] for r in range(n)]
+    rows[8500] = list(range(500, 8500)) + [8500]
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    col = np.concatenate(rows).astype(np.int32)
+    val = (rng.uniform(-1, 1, len(col)) / 50).astype(vt)
+    val[rp[1:] - 1] = rng.uniform(1, 2, n)
+    b = rng.uniform(-1, 1, n).astype(vt)
+    x = _solve("SPTRSV", rp, col, val, b)
+    assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
+
+
+MERGED = 2
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("k", [2, 31, 33, 150])
+@pytest.mark.parametrize("row_major", [True, False])
+def test_blocks_equal_the_level_launches(vt, k, row_major):
+    rp, col, val = level_matrix(EDGES, 3, 5, vt)
+    b = np.random.default_rng(k).uniform(-1, 1, (len(rp) - 1) * k).astype(vt)
+    x = _solve("SPTRSM", rp, col, val, b, k=k, row_major=row_major)
+    np.testing.assert_array_equal(x, _solve("SPTRSM", rp, col, val, b, k=k, row_major=row_major, mode=MERGED))
+
+
+@pytest.mark.parametrize("kind,k", [("SPTRSV", 1), ("SPTRSM", 5)])
+def test_new_values_equal_a_new_kernel(kind, k):
+    rp, col, val = level_matrix([40, 300, 5, 700] * 5, 5, 6, np.float64)
+    n = len(rp) - 1
+    rng = np.random.default_rng(7)
+    b = rng.uniform(-1, 1, n * k)
+    smax, kern, x = _kernel(kind, rp, col, val, b, k=k)
+    kern.run()
+    for _ in range(2):
+        val = val * rng.uniform(0.5, 1.5, len(val))
+        kern.update_A_values(val)
+        kern.run()
+        np.testing.assert_array_equal(x, _solve(kind, rp, col, val, b, k=k))
+    smax.close()
+
+
+def test_new_values_sync_free():
+    """The sync-free pack (few wide levels) takes new values over as well."""
+    rp, col, val = level_matrix([70000, 70000], 2, 8, np.float64)
+    rng = np.random.default_rng(9)
+    b = rng.uniform(-1, 1, len(rp) - 1)
+    smax, kern, x = _kernel("SPTRSV", rp, col, val, b, mode=5)
+    kern.run()
+    val = val * rng.uniform(0.5, 1.5, len(val))
+    kern.update_A_values(val)
+    kern.run()
+    np.testing.assert_array_equal(x, _solve("SPTRSV", rp, col, val, b, mode=5))
+    smax.close()
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("count,most", [(3, 900), (170, 60)])
+def test_batches(vt, count, most):
+    """Few matrices with wide levels, and more matrices than SMs."""
+    import torch
+    from smaxkernels_b200.interface import FloatType, TriangularBatch
+    rng = np.random.default_rng(count)
+    mats = [level_matrix(rng.integers(1, most, 12).tolist(), 1 + m % 4, m, vt) for m in range(count)]
+    tb = TriangularBatch(mats, FloatType.FLOAT64 if vt == np.float64 else FloatType.FLOAT32)
+    n = sum(len(m[0]) - 1 for m in mats)
+    b = rng.uniform(-1, 1, n).astype(vt)
+    bd = torch.from_numpy(b).cuda()
+    xd = torch.zeros_like(bd)
+    tb.solve(bd, xd)
+    torch.cuda.synchronize()
+    x = xd.cpu().numpy()
+    for m, (rp, col, val) in enumerate(mats):
+        a, e = tb.row_offset(m), tb.row_offset(m + 1)
+        assert normwise(x[a:e], O.sptrsv(rp, col, val, b[a:e])) <= tol(vt), m
+    tb.close()
