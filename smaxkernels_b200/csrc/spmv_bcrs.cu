@@ -18,13 +18,17 @@
 // rows (three or more warp steps on average) use a four-step loop with more
 // loads in flight; short ones (under two steps: e.g. a stencil in 4x4 blocks)
 // give each block row a group of bs/VEC lanes instead of a warp.  Other block
-// shapes: one thread per block row in the reference's loop order.
+// sizes up to kMaxBs give a lane each in-block position; larger ones, and many
+// short block rows, one thread per block row in the reference's loop order.
 //
 // Conversion: per block row, the sorted distinct block columns of its bh rows
 // (segmented radix sort of col/bw over the block row's entries, then a
 // uniqueness pass and a scan), then every entry is written into its block at
 // the in-block index of the chosen order; blocks are zero-filled first.
 #include "spmv_formats.cuh"
+
+#include <algorithm>
+#include <type_traits>
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -54,22 +58,92 @@ __device__ __forceinline__ void load16(const VT *p, VT *o) {
     }
 }
 
-constexpr int kMaxBs = 128;  // largest block size of the stream path
+constexpr int kMaxBs = 128;  // largest block size of the stream and lane paths
 
-// The stream loop of one block row per warp (the kernels below launch it).
-template <typename VT, bool UNROLL>
-__device__ __forceinline__ void bcrs_stream_rows(const int *__restrict__ row_ptr, const int *__restrict__ col,
-                                                 const VT *__restrict__ val, int64_t n_brows, int bh, int bw,
-                                                 int hpad, int wpad, int col_major, const VT *__restrict__ x,
-                                                 VT *__restrict__ y, const int *__restrict__ order) {
+// How a lane reads the x values of its VEC consecutive in-block positions.
+enum XMode {
+    kEach = 0,  // one load per position that is inside the block (padded blocks, odd shapes)
+    kRow = 1,   // row-major unpadded: VEC consecutive x values, one 16-byte load
+    kCol = 2,   // column-major unpadded: all VEC positions lie in one column, one value
+};
+
+template <typename VT, int XM> struct XVals {
+    static constexpr int VEC = V16<VT>::N;
+    VT v[XM == kCol ? 1 : VEC];
+    __device__ __forceinline__ void load(const VT *xb, const int (&jx)[VEC], const bool (&ok)[VEC]) {
+        if constexpr (XM == kRow) {
+            load16<VT, VEC, true>(xb + jx[0], v);
+        } else if constexpr (XM == kCol) {
+            v[0] = ld_keep(xb + jx[0]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) v[i] = ok[i] ? ld_keep(xb + jx[i]) : VT(0);
+        }
+    }
+    __device__ __forceinline__ void add(const VT (&a)[VEC], const bool (&ok)[VEC], VT (&acc)[VEC]) const {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i)
+            if (XM != kEach || ok[i]) acc[i] += a[i] * v[XM == kCol ? 0 : i];
+    }
+};
+
+// The rows a warp takes: order[w], order[w + W], ... of a grid of W warps
+// (longest first, so the long rows start first and the strided shares are
+// even).  A row's bounds are loaded while the row before it is summed.
+struct RowWalk {
+    const int *__restrict__ row_ptr;
+    const int *__restrict__ order;
+    int64_t n, w, W;
+    int row, b0, b1;  // the current row
+    int nrow, nb0, nb1;
+    __device__ __forceinline__ void fetch() {
+        nrow = -1;
+        nb0 = nb1 = 0;
+        if (w < n) {
+            nrow = order ? order[w] : (int)w;
+            nb0 = row_ptr[nrow];
+            nb1 = row_ptr[nrow + 1];
+        }
+        w += W;
+    }
+    __device__ __forceinline__ void next() {
+        row = nrow;
+        b0 = nb0;
+        b1 = nb1;
+        fetch();
+    }
+    __device__ RowWalk(const int *rp, const int *ord, int64_t n_rows) : row_ptr(rp), order(ord), n(n_rows) {
+        w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        W = (int64_t)gridDim.x * (blockDim.x >> 5);
+        fetch();
+        next();
+    }
+};
+
+// The stream loop, a warp per block row.  bs is a power of two here, so a
+// warp step covers a whole number of blocks and a lane's block advances by a
+// constant: no index division in the loop.  U steps' values and x entries are
+// loaded before any is used (the last steps of a row are masked, not looped
+// over one by one), and the column indices one iteration ahead -- the next
+// row's first ones during this row's last iteration -- so the x gathers wait
+// on no load of their own.  Bound by HBM and, between rows, by latency; four
+// steps on three CTAs an SM fill it (five CTAs spill: 168 us in the first
+// line).  B200, before (a warp per row, one step's indexes and gathers at a
+// time) and now, us: 27-point grid 48^3 in 4x4 blocks FP64 114 -> 78, FP32
+// 157 -> 54; 28^3 in 8x8 FP64 65 -> 55; 2^22 rows of lognormal length in 4x4
+// FP64 2080 -> 1557.
+template <typename VT, int XM, bool KEEP, int U, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) bcrs_stream_kernel(const int *__restrict__ row_ptr,
+                                                                const int *__restrict__ col,
+                                                                const VT *__restrict__ val, int64_t n_brows, int bh,
+                                                                int bw, int hpad, int wpad, int col_major,
+                                                                const VT *__restrict__ x, VT *__restrict__ y,
+                                                                const int *__restrict__ order) {
     constexpr int VEC = V16<VT>::N;
     __shared__ VT tile[8][kMaxBs];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t w = (int64_t)blockIdx.x * 8 + warp;
-    if (w >= n_brows) return;  // uniform per warp
-    const int64_t br = order ? order[w] : w;
     const int bs = hpad * wpad;
-    const int o = (lane * VEC) % bs;  // this lane's first in-block position
+    const int o = (lane * VEC) & (bs - 1);  // this lane's first in-block position
     int jx[VEC];
     bool ok[VEC];
 #pragma unroll
@@ -79,92 +153,141 @@ __device__ __forceinline__ void bcrs_stream_rows(const int *__restrict__ row_ptr
         jx[i] = col_major ? q / hpad : q % wpad;
         ok[i] = ix < bh && jx[i] < bw;
     }
-    VT acc[VEC];
+    const int per = 32 * VEC / bs;    // blocks of a warp step
+    const int sub = lane * VEC / bs;  // this lane's block of a step
+    const int groups = bs / VEC;      // lanes l and l + groups*m hold the same positions
+    RowWalk rows(row_ptr, order, n_brows);
+    int cn[U];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) acc[i] = VT(0);
-    const int64_t b0 = row_ptr[br], b1 = row_ptr[br + 1];
-    const int64_t end = b1 * bs;
-    constexpr int64_t STEP = 32 * VEC;
-    int64_t f = b0 * bs + lane * VEC;
-    // four steps' value and column loads first, then their x gathers, then
-    // the products in step order (the same sums as the one-step loop); for
-    // short block rows the registers this takes cost more occupancy than the
-    // overlap gains, so it is compiled out (UNROLL false)
-    // The column indices are loaded one iteration ahead, so an iteration's x
-    // gathers wait on no load of their own.
-    if constexpr (UNROLL) {
-    int cn[4] = {0, 0, 0, 0};
-    if (f + 3 * STEP < end)
+    for (int u = 0; u < U; ++u) {
+        const int j = rows.b0 + sub + u * per;
+        cn[u] = j < rows.b1 ? col[j] : 0;
+    }
+    while (rows.row >= 0) {  // uniform per warp
+        const int br = rows.row, b1 = rows.b1;
+        VT acc[VEC];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) cn[u] = col[(f + u * STEP) / bs];
-    for (; f + 3 * STEP < end; f += 4 * STEP) {
-        VT v[4][VEC];
-        int64_t c[4];
+        for (int i = 0; i < VEC; ++i) acc[i] = VT(0);
+        int j0 = rows.b0;
+        const VT *vp = val + (int64_t)(j0 + sub) * bs + o;
+        do {
+            const int j = j0 + sub;
+            VT v[U][VEC];
+            XVals<VT, XM> xv[U];
+            const VT *xb[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            load16<VT, VEC>(val + f + u * STEP, v[u]);
-            c[u] = (int64_t)cn[u] * wpad;
+            for (int u = 0; u < U; ++u)
+                if (j + u * per < b1) {
+                    load16<VT, VEC, KEEP>(vp + u * 32 * VEC, v[u]);
+                    xb[u] = x + (int64_t)cn[u] * wpad;
+                }
+            j0 += U * per;
+            const bool more = j0 < b1;
+            // the columns after these: of this row, or the first of the next
+            const int jn = (more ? j0 : rows.nb0) + sub, bn = more ? b1 : rows.nb1;
+#pragma unroll
+            for (int u = 0; u < U; ++u) cn[u] = jn + u * per < bn ? col[jn + u * per] : 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j + u * per < b1) xv[u].load(xb[u], jx, ok);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j + u * per < b1) xv[u].add(v[u], ok, acc);
+            vp += U * 32 * VEC;
+        } while (j0 < b1);
+        rows.next();
+        for (int s = groups; s < 32; s <<= 1)
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], s);
+        if (lane < groups)
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) tile[warp][o + i] = acc[i];
+        __syncwarp();
+        for (int ix = lane; ix < bh; ix += 32) {
+            VT s = VT(0);
+            for (int q = 0; q < bw; ++q) s += tile[warp][col_major ? q * hpad + ix : ix * wpad + q];
+            st_stream(y + (int64_t)br * hpad + ix, s);
         }
-        const int64_t fn = f + 4 * STEP;
-        if (fn + 3 * STEP < end)
-#pragma unroll
-            for (int u = 0; u < 4; ++u) cn[u] = col[(fn + u * STEP) / bs];
-        VT xv[4][VEC];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int i = 0; i < VEC; ++i) xv[u][i] = ok[i] ? ld_keep(x + c[u] + jx[i]) : VT(0);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int i = 0; i < VEC; ++i)
-                if (ok[i]) acc[i] += v[u][i] * xv[u][i];
+        __syncwarp();  // the tile is written again for the next row
     }
+}
+
+// Other block sizes up to kMaxBs, a lane per in-block position, so that the
+// loads of a step are contiguous.  NS == 1, blocks of at most 32 values: G
+// lanes per block row, G / bs blocks a step, 32 / G block rows a warp: the
+// whole warp, or for short block rows bs lanes each (several rows side by
+// side).  NS > 1: a block a step, NS positions a lane.  U steps' loads are in
+// flight, and the column indices come one iteration ahead.  3x3 blocks, before
+// (a thread per block row, its values strided) and now, us: 27-point grid 48^3
+// FP64 169 -> 91, FP32 125 -> 79; 7-point 64^3 FP64 84 -> 63.
+template <typename VT, int NS, int U>
+__global__ void __launch_bounds__(256) bcrs_lane_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col,
+                                                        const VT *__restrict__ val, int64_t n_brows, int bh, int bw,
+                                                        int hpad, int wpad, int col_major, const VT *__restrict__ x,
+                                                        VT *__restrict__ y, const int *__restrict__ order, int G) {
+    __shared__ VT tile[8][NS * 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int bs = hpad * wpad;
+    const int rows = 32 / G, g = lane / G, gl = lane - g * G;
+    const int64_t w = ((int64_t)blockIdx.x * 8 + warp) * rows + g;
+    const bool has = g < rows && w < n_brows;
+    const int64_t br = has ? (order ? order[w] : w) : 0;
+    const int per = NS == 1 ? G / bs : 1;  // blocks of a step
+    const int sub = NS == 1 ? gl / bs : 0;
+    int jx[NS];
+    bool ok[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        const int q = NS == 1 ? gl - sub * bs : lane + 32 * i;
+        const int ix = col_major ? q % hpad : q / wpad;
+        jx[i] = col_major ? q / hpad : q % wpad;
+        ok[i] = has && sub < per && q < bs && ix < bh && jx[i] < bw;
     }
-    for (; f < end; f += STEP) {
-        const int64_t c = (int64_t)col[f / bs] * wpad;
-        VT v[VEC];
-        load16<VT, VEC>(val + f, v);
+    VT acc[NS];
 #pragma unroll
-        for (int i = 0; i < VEC; ++i)
-            if (ok[i]) acc[i] += v[i] * ld_keep(x + c + jx[i]);
+    for (int i = 0; i < NS; ++i) acc[i] = VT(0);
+    int j0 = has ? row_ptr[br] : 0;
+    const int b1 = has ? row_ptr[br + 1] : 0;
+    int c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = j0 + u * per + sub < b1 ? col[j0 + u * per + sub] : -1;
+    for (; j0 < b1; j0 += U * per) {
+        VT v[U][NS], xv[U][NS];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const VT *p = val + (int64_t)(j0 + u * per) * bs + gl;
+#pragma unroll
+            for (int i = 0; i < NS; ++i)
+                if (ok[i] && c[u] >= 0) {
+                    v[u][i] = ld_stream(p + 32 * i);
+                    xv[u][i] = ld_keep(x + (int64_t)c[u] * wpad + jx[i]);
+                }
+        }
+        int cn[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + (U + u) * per + sub;
+            cn[u] = j < b1 ? col[j] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+            for (int i = 0; i < NS; ++i)
+                if (ok[i] && c[u] >= 0) acc[i] += v[u][i] * xv[u][i];
+            c[u] = cn[u];
+        }
     }
-    const int groups = bs / VEC;  // lanes l and l + groups*m hold the same positions
-    for (int s = groups; s < 32; s <<= 1)
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], s);
-    if (lane < groups)
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) tile[warp][o + i] = acc[i];
+    for (int i = 0; i < NS; ++i) tile[warp][lane + 32 * i] = acc[i];
     __syncwarp();
-    for (int ix = lane; ix < bh; ix += 32) {
-        VT s = VT(0);
-        for (int j = 0; j < bw; ++j) s += tile[warp][col_major ? j * hpad + ix : ix * wpad + j];
-        st_stream(y + br * hpad + ix, s);
-    }
-}
-
-template <typename VT, bool UNROLL>
-__global__ void __launch_bounds__(256) bcrs_stream_kernel(const int *__restrict__ row_ptr,
-                                                          const int *__restrict__ col, const VT *__restrict__ val,
-                                                          int64_t n_brows, int bh, int bw, int hpad, int wpad,
-                                                          int col_major, const VT *__restrict__ x,
-                                                          VT *__restrict__ y, const int *__restrict__ order) {
-    bcrs_stream_rows<VT, UNROLL>(row_ptr, col, val, n_brows, bh, bw, hpad, wpad, col_major, x, y, order);
-}
-
-// FP64: at most 48 registers, five CTAs per SM instead of four (the four-step
-// loop spills 32 bytes; 2^22 lognormal 4x4: 2.30 -> 2.26 ms; a bound of six
-// CTAs spilled 64 bytes and took 2.54 ms).  FP32 keeps the plain kernel: the
-// same bound spilled 88 bytes there.
-template <bool UNROLL>
-__global__ void __launch_bounds__(256, 5) bcrs_stream_kernel_f64(const int *__restrict__ row_ptr,
-                                                                 const int *__restrict__ col,
-                                                                 const double *__restrict__ val, int64_t n_brows,
-                                                                 int bh, int bw, int hpad, int wpad, int col_major,
-                                                                 const double *__restrict__ x, double *__restrict__ y,
-                                                                 const int *__restrict__ order) {
-    bcrs_stream_rows<double, UNROLL>(row_ptr, col, val, n_brows, bh, bw, hpad, wpad, col_major, x, y, order);
+    if (has)
+        for (int ix = gl; ix < bh; ix += G) {
+            VT s = VT(0);
+            for (int q = 0; q < bw; ++q)
+                for (int b = 0; b < per; ++b)
+                    s += tile[warp][g * G + b * bs + (col_major ? q * hpad + ix : ix * wpad + q)];
+            st_stream(y + br * hpad + ix, s);
+        }
 }
 
 // Short block rows: a group of G = bs / VEC lanes per block row (8 lanes for
@@ -239,7 +362,8 @@ __global__ void __launch_bounds__(256) bcrs_group_kernel(const int *__restrict__
         }
 }
 
-// generic block shapes: one thread per block row, the reference's loop order
+// block sizes beyond kMaxBs, and many short block rows: one thread per block
+// row, the reference's loop order
 template <typename VT>
 __global__ void bcrs_thread_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col,
                                    const VT *__restrict__ val, int64_t n_brows, int bh, int bw, int hpad, int wpad,
@@ -328,42 +452,72 @@ template <typename VT>
 void bcrs_spmv(const DevBCRS &m, const VT *x, VT *y, cudaStream_t st) {
     if (m.n_rows == 0) return;
     const int *order = m.order.p ? m.order.as<int>() : nullptr;
+    const int64_t bs = m.hpad * m.wpad;
+    constexpr int VEC = 16 / (int)sizeof(VT);
+    // a warp per block row, longest rows first; as many CTAs as are resident
+    auto go = [&](auto kern, int per_sm) {
+        const uint64_t grid = std::min<uint64_t>(((uint64_t)m.n_rows + 7) / 8, (uint64_t)per_sm * sm_count());
+        kern<<<(unsigned)grid, 256, 0, st>>>(m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows,
+                                             (int)m.bh, (int)m.bw, (int)m.hpad, (int)m.wpad, m.col_major ? 1 : 0, x, y,
+                                             order);
+    };
+    // Enough block rows to fill the chip with a thread each, and so short that a
+    // warp's rows stay in L1 while they are read: 3x3 blocks of a 7-point grid
+    // 64^3, FP32 (252 bytes a row) 46 us with a thread, 57 with a lane per
+    // position; FP64 (504 bytes) 84 and 63; 28^3 FP32 17.5 and 14.7.
+    const bool thread_rows = m.n_rows >= 1024ll * sm_count() &&
+                             m.n_blocks * bs * (int64_t)sizeof(VT) <= 256 * m.n_rows;
+    // a lane per in-block position, `lanes` lanes per block row
+    auto go_lanes = [&](auto kern, int lanes) {
+        kern<<<ceil_div_u(m.n_rows, 8 * (32 / lanes)), 256, 0, st>>>(
+            m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad,
+            (int)m.wpad, m.col_major ? 1 : 0, x, y, order, lanes);
+    };
     if (bcrs_stream_path(m.hpad, m.wpad, sizeof(VT))) {
         // mean warp steps per block row: below two a lane group per block row
-        // wastes fewer lanes; the four-step loop pays off from about three
-        const double steps = (double)m.n_blocks * (double)(m.hpad * m.wpad) /
-                             ((double)m.n_rows * 32.0 * (16.0 / sizeof(VT)));
-        const int64_t group = m.hpad * m.wpad / (16 / (int64_t)sizeof(VT));
+        // wastes fewer lanes; more loads in flight pay off from about three
+        const double steps = (double)m.n_blocks * (double)bs / ((double)m.n_rows * 32.0 * VEC);
         // values that fit in half of L2 are loaded with the default policy and
         // stay resident across repeated products (4x4 blocks of the 7-point
         // 64^3 Laplacian, 59 MB of values, in a loop of products: see the
         // BCRS notes); larger ones stream evict-first
-        const bool keep = (double)m.n_blocks * (double)(m.hpad * m.wpad) * sizeof(VT) <= 0.5 * (double)l2_bytes();
-        if (steps < 2.0 && keep)
-            bcrs_group_kernel<VT, true><<<ceil_div_u((uint64_t)m.n_rows * group, 256), 256, 0, st>>>(
-                m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad,
-                (int)m.wpad, m.col_major ? 1 : 0, x, y);
-        else if (steps < 2.0)
-            bcrs_group_kernel<VT, false><<<ceil_div_u((uint64_t)m.n_rows * group, 256), 256, 0, st>>>(
-                m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad,
-                (int)m.wpad, m.col_major ? 1 : 0, x, y);
-        else if (steps >= 3.0 && sizeof(VT) == 8)
-            bcrs_stream_kernel_f64<true><<<ceil_div_u(m.n_rows, 8), 256, 0, st>>>(
-                m.row_ptr.as<int>(), m.col.as<int>(), reinterpret_cast<const double *>(m.val.as<VT>()), m.n_rows,
-                (int)m.bh, (int)m.bw, (int)m.hpad, (int)m.wpad, m.col_major ? 1 : 0,
-                reinterpret_cast<const double *>(x), reinterpret_cast<double *>(y), order);
-        else if (steps >= 3.0)
-            bcrs_stream_kernel<VT, true><<<ceil_div_u(m.n_rows, 8), 256, 0, st>>>(
-                m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad,
-                (int)m.wpad, m.col_major ? 1 : 0, x, y, order);
-        else
-            bcrs_stream_kernel<VT, false><<<ceil_div_u(m.n_rows, 8), 256, 0, st>>>(
-                m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad,
-                (int)m.wpad, m.col_major ? 1 : 0, x, y, order);
-    } else
+        const bool keep = (double)m.n_blocks * (double)bs * sizeof(VT) <= 0.5 * (double)l2_bytes();
+        const bool whole = m.bh == m.hpad && m.bw == m.wpad;
+        const int xm = !whole ? kEach
+                       : m.col_major ? (m.hpad % VEC == 0 ? kCol : kEach)
+                       : (m.wpad % VEC == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) ? kRow : kEach;
+        auto with_x = [&](auto f) {
+            if (xm == kRow) f(std::integral_constant<int, kRow>());
+            else if (xm == kCol) f(std::integral_constant<int, kCol>());
+            else f(std::integral_constant<int, kEach>());
+        };
+        if (steps < 2.0) {
+            const uint64_t threads = (uint64_t)m.n_rows * (uint64_t)(bs / VEC);
+            auto kern = keep ? bcrs_group_kernel<VT, true> : bcrs_group_kernel<VT, false>;
+            kern<<<ceil_div_u(threads, 256), 256, 0, st>>>(m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(),
+                                                           m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad, (int)m.wpad,
+                                                           m.col_major ? 1 : 0, x, y);
+        } else {
+            with_x([&](auto XM) {
+                if (steps < 3.0 && keep) go(bcrs_stream_kernel<VT, XM.value, true, 2, 4>, 4);
+                else if (steps < 3.0) go(bcrs_stream_kernel<VT, XM.value, false, 2, 4>, 4);
+                else if (keep) go(bcrs_stream_kernel<VT, XM.value, true, 4, 3>, 3);
+                else go(bcrs_stream_kernel<VT, XM.value, false, 4, 3>, 3);
+            });
+        }
+    } else if (bs <= 32 && !thread_rows) {
+        // fewer than three warp steps a block row: several block rows a warp
+        const int per = 32 / (int)bs;
+        go_lanes(bcrs_lane_kernel<VT, 1, 4>, m.n_blocks < 3 * per * m.n_rows ? (int)bs : 32);
+    } else if (bs <= 64 && !thread_rows) {
+        go_lanes(bcrs_lane_kernel<VT, 2, 2>, 32);
+    } else if (bs <= kMaxBs && !thread_rows) {
+        go_lanes(bcrs_lane_kernel<VT, 4, 1>, 32);
+    } else {
         bcrs_thread_kernel<VT><<<ceil_div_u(m.n_rows, 128), 128, 0, st>>>(
             m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad,
             (int)m.wpad, m.col_major ? 1 : 0, x, y);
+    }
     SMAX_CUDA(cudaGetLastError());
 }
 
