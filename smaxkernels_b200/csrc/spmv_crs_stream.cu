@@ -19,7 +19,9 @@
 // more than 32 entries, a slice instead sums the head of its first row (the
 // entries before the slice, at most 31) itself, one entry per lane, and
 // neither carries nor the fix-up launch are needed.  Rows without
-// entries get y = 0 from a separate list.  HBM traffic: val, col, one bit per
+// entries get y = 0 from a separate list.  Short rows of nearly one length are
+// summed by a few lanes each instead (crs_rows_kernel): one launch, no carries,
+// no scan.  HBM traffic: val, col, one bit per
 // entry, one int per 512 entries, y; x is gathered through L2.
 #include "spmv_crs.cuh"
 
@@ -180,6 +182,44 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
     }
 }
 
+// Short rows (at most 32 entries) of nearly one length, G lanes a row: lane l
+// takes the row's entries l, l + G, ..., at most U of them (G * U >= the longest
+// row), all loaded before any is used.  The lanes of a warp read neighbouring
+// rows, so every line of col and val is used up from L1, and the x entries that
+// neighbouring rows of a grid share are found there too.  Bound by HBM: 190^3
+// 7-point FP64 171 -> 136 us (5.2 TB/s of val, col, row_ptr, x and y).
+template <typename VT, int G, int U>
+__global__ void __launch_bounds__(256) crs_rows_kernel(const int *__restrict__ col, const VT *__restrict__ val,
+                                                       const int *__restrict__ row_ptr, int64_t n,
+                                                       const VT *__restrict__ x, VT *__restrict__ y) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t row = i / G;
+    const int gl = (int)(i % G);
+    int s = 0, e = 0;
+    if (row < n) {
+        s = row_ptr[row] + gl;
+        e = row_ptr[row + 1];
+    }
+    int c[U];
+    VT v[U], xv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (s + u * G < e) {
+            c[u] = __ldg(col + s + u * G);
+            v[u] = __ldg(val + s + u * G);
+        }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (s + u * G < e) xv[u] = __ldg(x + c[u]);
+    VT sum = VT(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (s + u * G < e) sum += v[u] * xv[u];
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (row < n && gl == 0) st_stream(y + row, sum);
+}
+
 // y[row] += the run of carries of one row, summed in task order.
 template <typename VT>
 __global__ void crs_stream_fixup(const VT *__restrict__ carry_val, const int *__restrict__ carry_rank,
@@ -203,13 +243,17 @@ __global__ void row_flags_kernel(const int *__restrict__ row_ptr, int64_t n, uns
                                  unsigned char *__restrict__ nonempty, uint32_t *__restrict__ endbits,
                                  int *__restrict__ max_len) {
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const int s = row_ptr[r], e = row_ptr[r + 1];
-    const bool em = e == s;
-    empty[r] = em;
-    nonempty[r] = !em;
-    if (!em) atomicOr(endbits + ((e - 1) >> 5), 1u << ((e - 1) & 31));
-    if (e - s > 32) atomicMax(max_len, e - s);  // only "more than 32" matters
+    int len = 0;
+    if (r < n) {
+        const int s = row_ptr[r], e = row_ptr[r + 1];
+        const bool em = e == s;
+        empty[r] = em;
+        nonempty[r] = !em;
+        if (!em) atomicOr(endbits + ((e - 1) >> 5), 1u << ((e - 1) & 31));
+        len = e - s;
+    }
+    len = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
+    if ((threadIdx.x & 31) == 0 && len > 0) atomicMax(max_len, len);
 }
 
 // rank of the row holding entry t*W: the largest r with row_ptr[r] <= t*W
@@ -250,7 +294,7 @@ void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vby
     n_empty = 0;
     n_nonempty = 0;
     row_ptr = d_row_ptr;
-    short_rows = true;
+    longest = 0;
     if (n > 0) {
         DevBuf fe(n), fne(n), cnt(sizeof(int) * 3);
         SMAX_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes, st));
@@ -270,7 +314,7 @@ void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vby
         SMAX_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, st));
         SMAX_CUDA(cudaStreamSynchronize(st));
         n_empty = h[0];
-        short_rows = h[2] == 0;
+        longest = h[2];
         n_nonempty = n - n_empty;
         if (n_empty > 0) {
             row_list.alloc(sizeof(int) * (n_nonempty > 0 ? n_nonempty : 1));
@@ -295,6 +339,24 @@ void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vby
 
 template <typename VT>
 void crs_spmv_stream(const CrsStreamPlan &p, const int *col, const VT *val, const VT *x, VT *y, cudaStream_t st) {
+    // Rows of nearly one length, up to 32: a lane (or 2, 4) per row.  Lanes left
+    // without entries cost as much as the others, so only where rows are two
+    // thirds full on average.  B200, us, stream -> rows: 128^3 7-point FP64
+    // (98% full) 54.8 -> 48.1, 96^3 27-point 86.3 -> 70.9, 2^20 rows of 5, one in
+    // 100 of 7 (72%) 32.3 -> 25.0; 2^22 rows of 0 to 32 evenly (50%) 299 -> 318,
+    // of 2, one in 100 of 32 (7%) 57 -> 229.
+    if (p.n_rows > 0 && p.longest <= 32 && 3 * p.nnz >= 2 * p.n_rows * p.longest) {
+        // rows without entries get their zero here as well
+        auto rows = [&](auto kern, int g) {
+            kern<<<ceil_div_u((uint64_t)p.n_rows * g, 256), 256, 0, st>>>(col, val, p.row_ptr, p.n_rows, x, y);
+            SMAX_CUDA(cudaGetLastError());
+        };
+        if (p.longest <= 4) rows(crs_rows_kernel<VT, 1, 4>, 1);
+        else if (p.longest <= 8) rows(crs_rows_kernel<VT, 1, 8>, 1);
+        else if (p.longest <= 16) rows(crs_rows_kernel<VT, 2, 8>, 2);
+        else rows(crs_rows_kernel<VT, 4, 8>, 4);
+        return;
+    }
     const int *rl = p.row_list.p ? p.row_list.as<int>() : nullptr;
     if (p.n_tasks > 0) {
         unsigned grid = ceil_div_u(p.n_tasks, kWarpsPerCta);
@@ -304,7 +366,7 @@ void crs_spmv_stream(const CrsStreamPlan &p, const int *col, const VT *val, cons
                                                      p.carry_val.as<VT>(), p.carry_rank.as<int>());
             SMAX_CUDA(cudaGetLastError());
         };
-        if (p.short_rows) {
+        if (p.longest <= 32) {
             launch(crs_stream_kernel<VT, true>);  // no carries: one launch
         } else {
             launch(crs_stream_kernel<VT, false>);
