@@ -60,8 +60,10 @@ static_assert(kLevels >= kGroups && kSlots >= kWindow + kGroups, "mbarriers for 
 // to i + kWindow - 1: the mbarrier must not have been used again by then.
 static_assert(kSlots > 2 * kWindow + kCopyWarps - 2, "mbarriers for the copying warps' lead");
 constexpr int kRecChunks = 32;             // chunks of a record, at most
-constexpr long long kWaitLimit = 1 << 18;  // polls of a copy's mbarrier (each blocks for a while) before giving up
-constexpr int kLevelLimit = 1 << 22; // polls of a level's mbarrier before giving up
+// Polls before a wait gives up: seconds, since the threads of a run wait while
+// one of them goes through a row of a million entries.
+constexpr long long kWaitLimit = 1 << 25;  // of a copy's mbarrier (each may sleep for a while)
+constexpr int kLevelLimit = 1 << 28;       // of a level's, 10 ns each at least
 
 // header flags (the width is above them)
 constexpr int kFlagBits = 4;
@@ -518,23 +520,41 @@ __device__ __forceinline__ void sw_store(const ChunkView &c, int t, VT x, unsign
     xp[p] = x;
 }
 
+// Sum of a row too wide for the stage, from the blob, eight entries in flight.
+// A function of its own, for its registers.
+template <typename VT>
+__device__ __noinline__ VT sw_sum_direct(const unsigned char *__restrict__ data, int w, int mp, int t, const VT *xp) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const unsigned char *ring = smem + kSharedBytes;
+    const VT *pv = reinterpret_cast<const VT *>(data) + t;
+    const int *ps = reinterpret_cast<const int *>(data + (int64_t)(w + 1) * mp * (int)sizeof(VT)) + t;
+    VT sum = VT(0);
+    constexpr int U = 8;
+    int i = 0;
+#pragma unroll 1
+    for (; i + U <= w; i += U, pv += (int64_t)U * mp, ps += (int64_t)U * mp) {
+        VT v[U], x[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            v[q] = pv[(int64_t)q * mp];
+            x[q] = sw_solution<VT>(ps[(int64_t)q * mp], ring, xp);
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) sum += v[q] * x[q];
+    }
+#pragma unroll 1
+    for (; i < w; ++i, pv += mp, ps += mp) sum += *pv * sw_solution<VT>(*ps, ring, xp);
+    return sum;
+}
+
 // sum of the entries' products of row t of a chunk of wider rows
 template <typename VT>
 __device__ VT sw_sum_any(const unsigned char *stage, int at, const ChunkView &c, int t, const RowOps<VT> &R,
                          const unsigned char *ring, const VT *xp, const unsigned char *__restrict__ blob) {
     VT sum = VT(0);
     const int w = c.wf >> kFlagBits;
-    if (c.wf & kDirect) {
-        const int off = sw_blob_offset(stage, at);
-        const VT *pv = reinterpret_cast<const VT *>(blob + (int64_t)off * 16 + kHeader);
-        const int *ps = reinterpret_cast<const int *>(pv + (int64_t)(w + 1) * c.mp());
-#pragma unroll 1
-        for (int i = 0; i < w; ++i) {
-            const int64_t u = (int64_t)i * c.mp() + t;
-            sum += pv[u] * sw_solution<VT>(ps[u], ring, xp);
-        }
-        return sum;
-    }
+    if (c.wf & kDirect)
+        return sw_sum_direct<VT>(blob + (int64_t)sw_blob_offset(stage, at) * 16 + kHeader, w, c.mp(), t, xp);
     const VT *pv = reinterpret_cast<const VT *>(stage + at + kHeader);
     const int *ps = reinterpret_cast<const int *>(pv + (w + 1) * c.mp());
     // four entries at a time: their solutions are read before any is used
@@ -945,6 +965,9 @@ bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *v
         for (int s = step.first; s < step.first + step.count; ++s) {
             const int m = count[s];
             if (m == 0) continue;
+            // a level near the waits' limit (in polls: an entry after the other in
+            // its rows, and what the SM takes in) is left to the plain kernels
+            if (25ll * w[s] * (m / (kGroups * T) + 1) + (long long)m * w[s] / 4 > kLevelLimit / 4) return false;
             const int layout = w[s] <= 2 ? kTwo : (w[s] == 3 ? kThree : 0);
             const long long each = (long long)row_bytes(layout, w[s], vb) + vb;  // with its right-hand side
             // two rows a thread, but one where a division each is the longest part

@@ -130,6 +130,22 @@ def test_sweep_rows_too_wide_for_the_stage(vt):
     assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
 
 
+def test_sweep_waits_for_a_very_long_row():
+    """A row of 400000 entries, read in place by one thread while the others
+    wait for its level: as long as it takes."""
+    n0, chain = 400000, 60
+    n = n0 + 1 + chain
+    rows = [np.array([r]) for r in range(n0)] + [np.arange(n0 + 1)] + [np.array([r - 1, r]) for r in range(n0 + 1, n)]
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    col = np.concatenate(rows).astype(np.int32)
+    rng = np.random.default_rng(11)
+    val = rng.uniform(-1, 1, len(col)) / 1000
+    val[rp[1:] - 1] = rng.uniform(1, 2, n)
+    b = rng.uniform(-1, 1, n)
+    x = _solve("SPTRSV", rp, col, val, b)
+    assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(np.float64)
+
+
 MERGED = 2
 
 
