@@ -589,12 +589,14 @@ def wl_spmm(b: Bench):
                 t, reps = b.time(k.apply)
             cpu = b.cpu(lambda: b.ref.time_spmm(rp, col, val, X, kv, True, warm=1, reps=5), nbytes,
                         "5 applies after 1 warm-up (reference OpenMP row-major SpMM)") if var == variants[0] else None
-            vname = {0: "", 1: "_grid", 2: "_walk"}[var]
+            vname = {0: "", 1: "_grid", 2: "_groups"}[var]
+            kname = {0: "spmm_group_kernel or spmm_row_major_kernel", 1: "spmm_row_major_kernel",
+                     2: "spmm_group_kernel"}[var]
             b.emit(f"spmm_rowmajor_k{kv}_{_dt(vt)}_stencil27_128{vname}", "SpMM GB/s", nbytes / t / 1e9, "GB/s", t,
                    reps, _dt(vt), {"n_rows": n, "nnz": nnz, "k": kv, "layout": "row-major X, Y",
                                    "l2": "inputs larger than L2 (no flush)",
-                                   "kernel": "spmm_row_major_kernel" if var == 1 else "spmm_walk_kernel"},
-                   clk.summary(), b.hbm(nbytes, t, "spmm_row_major_kernel" if var == 1 else "spmm_walk_kernel"),
+                                   "kernel": kname},
+                   clk.summary(), b.hbm(nbytes, t, kname),
                    cpu, launches=reps,
                    gflops=round(2 * nnz * kv / t / 1e9, 3))
             smax.close()
@@ -684,7 +686,7 @@ def wl_sptrsv(b: Bench):
                         "3 solves after 1 warm-up (reference naive_crs_sptrsv, serial)")
         b.emit(f"sptrsv_f64_laplace2d_{side}_natural_{names[mode]}", "SpTRSV GB/s", nbytes / t / 1e9, "GB/s", t,
                reps, "f64", {"n_rows": n, "nnz": nnz, "levels": n_lv, "scheme": names[mode]}, clk.summary(),
-               b.hbm(nbytes, t, "syncfree_kernel" if mode == 5 else "wide_level_kernel/sweep_kernel"), cpu,
+               b.hbm(nbytes, t, "syncfree_kernel" if mode == 5 else "sw_wide_kernel/sweep_kernel"), cpu,
                launches=n_lv * reps if mode == 1 else (reps if mode == 4 else (2 * reps if mode == 5 else None)),
                us_per_level=round(t * 1e6 / n_lv, 4), bitwise_equal_to_graph=same)
         smax.close()
@@ -729,7 +731,7 @@ def wl_sptrsv(b: Bench):
             b.emit(f"sptrsv_f64_laplace2d_{side}_permuted_{names[mode]}", "SpTRSV GB/s", nbytes / t / 1e9, "GB/s", t,
                    reps, "f64", {"n_rows": n, "nnz": len(lcol), "levels": nl, "scheme": names[mode],
                                  "ordering": "random symmetric permutation (seed 3), RS level order"},
-                   clk.summary(), b.hbm(nbytes, t, "syncfree_kernel" if mode in (0, 5) else "wide_level_kernel/sweep_kernel"),
+                   clk.summary(), b.hbm(nbytes, t, "syncfree_kernel" if mode in (0, 5) else "sw_wide_kernel/sweep_kernel"),
                    cpu, launches=reps if mode == 4 else (2 * reps if mode in (0, 5) else None),
                    us_per_level=round(t * 1e6 / max(nl, 1), 4), bitwise_equal_to_graph=same)
         smax.close()
@@ -1032,7 +1034,7 @@ def wl_solvers(b: Bench):
             cpu = {"value": round(nbytes / tc / 1e9, 3), "unit": "GB/s", "cores": b.threads, "kind": "reference",
                    "sample": f"{k_cpu} iterations of the program's loop through the reference's kernels",
                    "ms_per_iteration": round(tc * 1e3, 4)}
-        kern = "jacobi_kernel" if kind == "jacobi" else "rhs_kernel + level-pack SpTRSV (sweep_kernel)"
+        kern = "jacobi_kernel" if kind == "jacobi" else "rhs_kernel + SpTRSV sweeps (sweep_kernel)"
         b.emit(f"solver_{kind}_poisson2d_{side}", "solver iteration GB/s (algorithmic bytes)", nbytes / t_it / 1e9,
                "GB/s", t_it, reps, "f64", {"n_rows": n, "nnz": nnz, "iterations": iters, "check_length": cl,
                                           "driver": b.args.solver_mode, "inputs": "larger than L2"},

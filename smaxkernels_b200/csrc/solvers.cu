@@ -16,7 +16,7 @@
 //    device, so a block of iterations is one replayable launch sequence.
 //  * Gauss-Seidel: a row-group kernel forms tmp = b - U x, then the platform's
 //    level-scheduled SpTRSV (an internal kernel object on D+L, merged single-
-//    CTA runs on its level pack) solves (D+L) x = tmp.
+//    CTA runs on its sweep pack) solves (D+L) x = tmp.
 //  * The residual max_r |b_r - (A x)_r| is a row-group kernel with a block
 //    maximum and one atomicMax on the bit pattern (non-negative doubles order
 //    like their bits); a one-thread kernel records it, advances the iteration
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kSmallThreads)
     for (int r = threadIdx.x; r < n; r += blockDim.x) {
         x[r] = xg[r];
         b[r] = bg[r];
-        D[r] = VT(1) / Dg[r];  // the sweep multiplies by 1/D, as the level-pack SpTRSV does
+        D[r] = VT(1) / Dg[r];  // the sweep multiplies by 1/D, as the SpTRSV sweeps do
     }
     // with stage, the level sweep's arrays follow the vectors in shared memory:
     // its chain of dependent loads per level then never leaves the SM
