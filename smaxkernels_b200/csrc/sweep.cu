@@ -24,15 +24,15 @@
 // same pack through L2.
 //
 // What bounds it: narrow levels by the chain wait, ring read, sum, store,
-// arrive, 0.25 us a level; wide ones by what one SM takes in, 48 bytes a row
-// of a 5-point FP64 matrix at 83 GB/s (2048 rows a level).  B200, 5-point D+L
+// arrive, 0.22 us a level; wide ones by the SM's issue slots (62% busy at up to
+// 1024 rows a level) and L1 (67%).  B200, 5-point D+L
 // in natural order, FP64; before: one CTA whose threads load every level from
 // global memory two levels ahead and meet at a barrier.
-//     100^2 (199 levels)             127 -> 51 us
-//     512^2                          727 -> 260 us
-//     2048^2 (4095 levels)          5020 -> 2450 us
-//     1024^2, 32 right-hand sides   2900 -> 1510 us
-//     48 matrices in one batch       919 -> 397 us
+//     100^2 (199 levels)             124 -> 48 us
+//     512^2                          727 -> 223 us
+//     2048^2 (4095 levels)          5020 -> 2370 us
+//     1024^2, 32 right-hand sides   2900 -> 1450 us
+//     48 matrices in one batch       919 -> 362 us
 #include "sweep.cuh"
 
 #include <algorithm>
@@ -62,8 +62,9 @@ static_assert(kSlots > 2 * kWindow + kCopyWarps - 2, "mbarriers for the copying 
 constexpr int kRecChunks = 32;             // chunks of a record, at most
 // Polls before a wait gives up: seconds, since the threads of a run wait while
 // one of them goes through a row of a million entries.
-constexpr long long kWaitLimit = 1 << 25;  // of a copy's mbarrier (each may sleep for a while)
-constexpr int kLevelLimit = 1 << 28;       // of a level's, 10 ns each at least
+constexpr long long kWaitLimit = 1 << 27;  // 20 ns each at least
+// Time of a level, in steps of 10 ns, up to which it is swept.
+constexpr long long kLevelTime = 1 << 26;
 
 // header flags (the width is above them)
 constexpr int kFlagBits = 4;
@@ -623,28 +624,13 @@ __device__ __forceinline__ void sw_arrive(unsigned long long *bar, int count) {
     asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 
-// The wait of one level for the one before it is on the critical path: polled
-// without the blocking of mbarrier.try_wait.
-__device__ __forceinline__ bool sw_wait_level(unsigned long long *bar, unsigned parity) {
-#pragma unroll 1
-    for (int it = 0; it < kLevelLimit; ++it) {
-        unsigned ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-
+// The wait for the level before.  The thread sleeps in mbarrier.try_wait: polling
+// with test_wait took issue slots from the groups at work (512^2 natural FP64
+// 260 us against 223, 2048^2 2.45 ms against 2.37).
 __device__ __forceinline__ bool sw_wait_before(SweepShared *sh, const ChunkView &c, int level0) {
     if (c.level == 0) return true;
     const int l = level0 + c.level - 1;
-    return sw_wait_level(&sh->level[l % kLevels], (unsigned)(l / kLevels) & 1u);
+    return mbar_wait_bounded(as_bar(&sh->level[l % kLevels]), (unsigned)(l / kLevels) & 1u, kWaitLimit);
 }
 
 // Chunk c of layout W for a group: operands, the wait for the level before, RW
@@ -965,9 +951,9 @@ bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *v
         for (int s = step.first; s < step.first + step.count; ++s) {
             const int m = count[s];
             if (m == 0) continue;
-            // a level near the waits' limit (in polls: an entry after the other in
-            // its rows, and what the SM takes in) is left to the plain kernels
-            if (25ll * w[s] * (m / (kGroups * T) + 1) + (long long)m * w[s] / 4 > kLevelLimit / 4) return false;
+            // a level near the waits' limit (an entry after the other in its rows,
+            // and what the SM takes in) is left to the plain kernels
+            if (25ll * w[s] * (m / (kGroups * T) + 1) + (long long)m * w[s] / 4 > kLevelTime) return false;
             const int layout = w[s] <= 2 ? kTwo : (w[s] == 3 ? kThree : 0);
             const long long each = (long long)row_bytes(layout, w[s], vb) + vb;  // with its right-hand side
             // two rows a thread, but one where a division each is the longest part
