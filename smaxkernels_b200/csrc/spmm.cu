@@ -558,10 +558,14 @@ void SpmmPlan::build(const DevCRS &a, cudaStream_t st) {
 // 1997; k = 16 FP64 276 / 257), or rows too short to pay for the groups' work
 // per row (7-point 100^3: k = 16 FP64 134 / 154 us, k = 16 FP32 79 / 83; k = 4
 // FP64 73 / 48), or rows of X of one 16-byte FP64 vector (27-point 96^3, k = 2:
-// 239 / 495 us).  Rows of uneven length always take the groups (lognormal
-// 500000, k = 64 FP64: 946 against 1543 us).
+// 239 / 495 us).  Rows of uneven length take the groups (lognormal 500000,
+// k = 64 FP64: 946 against 1543 us), except in small matrices of few entries,
+// where a CTA's start counts (20000 rows, nine in ten empty, k = 32 FP64: 25 us,
+// the grid 16; of 2 entries, one in 100 of 32: 19.6 and 16.9).
 static bool grid_suits(const DevCRS &a, const SpmmPlan &p, int64_t nvec, int vbytes) {
-    if (!p.regular || nvec <= 0 || nvec > 128 || (nvec & (nvec - 1))) return false;
+    if (nvec <= 0 || nvec > 128 || (nvec & (nvec - 1))) return false;
+    if (nvec >= 8 && a.nnz < 4 * a.n_rows && a.n_rows < (1 << 17)) return true;
+    if (!p.regular) return false;
     return nvec >= 16 || (nvec >= 4 && a.nnz <= 12 * a.n_rows) || (nvec == 1 && vbytes == 8);
 }
 
@@ -598,6 +602,18 @@ void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStre
                 a.rp(), a.ci(), a.val.template as<VT>(), a.n_rows, k, X, Y);
     }
     SMAX_CUDA(cudaGetLastError());
+}
+
+// Whether a column-major block runs as one product per column: rows so short
+// that transposing X costs more than reading A again.  2^19 rows of 2 entries,
+// one in 100 of 32, FP64: k = 3 37 us as products, 52 as a block; k = 8 89 and
+// 70; below 2^17 rows the products' launches cost more (20000 rows, k = 3: 27
+// and 21).  With rows of more than 64 times the average length also k = 8 (of 1
+// entry, one in 1000 of 500: 137 and 173 us): a product spreads a long row over
+// the chip.
+bool spmm_by_columns(const DevCRS &a, int64_t k, int64_t longest) {
+    const bool skewed = longest * a.n_rows > 64 * a.nnz;
+    return a.nnz < 4 * a.n_rows && ((k < 8 && a.n_rows >= (1 << 17)) || (k <= 8 && skewed));
 }
 
 int64_t spmm_col_major_work(int64_t n_cols, int64_t k, int vbytes) {
