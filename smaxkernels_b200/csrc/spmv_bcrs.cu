@@ -465,8 +465,11 @@ void bcrs_spmv(const DevBCRS &m, const VT *x, VT *y, cudaStream_t st) {
     // warp's rows stay in L1 while they are read: 3x3 blocks of a 7-point grid
     // 64^3, FP32 (252 bytes a row) 46 us with a thread, 57 with a lane per
     // position; FP64 (504 bytes) 84 and 63; 28^3 FP32 17.5 and 14.7.
+    // Blocks of more than 16 values leave a fifth of a warp's lanes idle: 2^19
+    // block rows of five 5x5 blocks, FP32 (500 bytes) 248 and 292 us.
+    const int64_t short_row = bs > 16 && m.n_blocks >= 4 * m.n_rows ? 512 : 256;
     const bool thread_rows = m.n_rows >= 1024ll * sm_count() &&
-                             m.n_blocks * bs * (int64_t)sizeof(VT) <= 256 * m.n_rows;
+                             m.n_blocks * bs * (int64_t)sizeof(VT) <= short_row * m.n_rows;
     // a lane per in-block position, `lanes` lanes per block row
     auto go_lanes = [&](auto kern, int lanes) {
         kern<<<ceil_div_u(m.n_rows, 8 * (32 / lanes)), 256, 0, st>>>(
