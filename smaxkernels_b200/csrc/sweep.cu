@@ -31,7 +31,7 @@
 //     100^2 (199 levels)             124 -> 48 us
 //     512^2                          727 -> 223 us
 //     2048^2 (4095 levels)          5020 -> 2370 us
-//     1024^2, 32 right-hand sides   2900 -> 1450 us
+//     1024^2, 32 right-hand sides   2900 -> 1480 us
 //     48 matrices in one batch       919 -> 362 us
 #include "sweep.cuh"
 

@@ -70,8 +70,10 @@ struct SweepStep {
 // diagonal) whose sweep step s solves the rows order[src_begin[s] ..
 // src_begin[s] + count[s]) (order == nullptr: the identity); `steps` groups the
 // sweep steps.  div: divide by the diagonal instead of multiplying by its
-// reciprocal.  batch: the runs are independent matrices (sweep_solve_batch).  Returns false (building nothing) when the padding would make the
-// pack more than about three times the off-diagonal entries.  Synchronises.
+// reciprocal.  batch: the runs are independent matrices (sweep_solve_batch).  Returns false when the
+// padding would make the pack more than about three times the off-diagonal
+// entries, or a level takes so long that others' waits for it could give up.
+// Synchronises.
 bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *val, const void *D, int vbytes,
                       int64_t n, const int *order, const std::vector<int> &src_begin, const std::vector<int> &count,
                       const std::vector<SweepStep> &steps, bool div, bool batch, cudaStream_t st);
