@@ -62,8 +62,11 @@ DevStatus *dstatus(smax_kernel_s *k) { return k->status.as<DevStatus>(); }
 
 bool is_tri(const smax_kernel_s *k) { return k->ktype == SMAX_KERNEL_SPTRSV || k->ktype == SMAX_KERNEL_SPTRSM; }
 
+SweepWait sweep_wait(const smax_kernel_s *k) { return {k->spin_limit * SweepWait::kPollNs, k->force_timeout}; }
+
 void tri_plan(smax_kernel_s *k) {
     k->tri.status = dstatus(k);
+    k->tri.wait = sweep_wait(k);
     if (k->f_perm) {
         require(k->ctx != nullptr && k->ctx->n_levels > 0, SMAX_ERR_STATE,
                 "level-scheduled solve needs the levels of generate_perm in the context");

@@ -16,6 +16,8 @@ smax_kernel_s *K(smax_kernel k);
 void read_status(smax_kernel_s *k);
 DevStatus *dstatus(smax_kernel_s *k);
 bool is_tri(const smax_kernel_s *k);
+// how long the waits of a solve's sweeps last
+SweepWait sweep_wait(const smax_kernel_s *k);
 // builds (or reuses) the level schedule of a triangular solve
 void tri_plan(smax_kernel_s *k);
 // device addresses of the registered B and C (+ element offsets)

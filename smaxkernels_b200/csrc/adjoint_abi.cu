@@ -46,6 +46,7 @@ void ensure_adjoint(smax_kernel_s *k) {
         k->adj_plan_serial = k->tri_plan_serial;
     }
     k->adj_plan.status = dstatus(k);
+    k->adj_plan.wait = sweep_wait(k);
 }
 
 template <typename VT> void adjoint_t(smax_kernel_s *k, const VT *x, const VT *g, VT *din, VT *dval) {

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "sweep.cuh"
 
 namespace smax {
 
@@ -17,6 +18,7 @@ struct RefineState {
     int g_steps = -1, g_merge = -1;
     uint64_t g_serial = ~0ull, g_aver = ~0ull;  // level plan and A upload the graph was captured for
     const void *g_pack = nullptr;                // sweep pack the graph reads
+    SweepWait g_wait;                            // and how long its waits last
     int steps_done = 0;
     double last_rel = 0.0;          // max|d| / max|x| of the last correction
     void release_graph() {

@@ -371,7 +371,7 @@ void tri_solve_raw(TriPlan &p, const int *rp, const int *ci, const VT *val, cons
     if (p.n_rows == 0) return;
     const int64_t rs = row_major ? k : 1, vs = row_major ? 1 : ld;
     if (k == 1 && p.pack_is(val, D, sizeof(VT), merge_rows, tag, 1)) {
-        sweep_solve<VT>(p.pack, B, X, 1, rs, vs, p.status, st);
+        sweep_solve<VT>(p.pack, B, X, 1, rs, vs, p.status, p.wait, st);
         return;
     }
     if (p.scheduled_k != k || p.scheduled_merge != merge_rows) p.schedule(k, merge_rows);
@@ -429,7 +429,8 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
     if (!packed && (p.scheduled_k != k || p.scheduled_merge != merge_rows)) p.schedule(k, merge_rows);
     const void *key[4] = {B, X, D, a.val.p};
     if (!p.graph_valid || p.graph_key[0] != key[0] || p.graph_key[1] != key[1] || p.graph_key[2] != key[2] ||
-        p.graph_key[3] != key[3] || p.graph_row_major != row_major || p.graph_ld != ld || p.graph_k != k || p.graph_packed != packed) {
+        p.graph_key[3] != key[3] || p.graph_row_major != row_major || p.graph_ld != ld || p.graph_k != k || p.graph_packed != packed ||
+        p.graph_wait != p.wait) {
         if (!packed && !p.ranges_uploaded && !p.seg_ranges.empty()) {
             SMAX_CUDA(cudaMemcpyAsync(p.d_ranges.p, p.seg_ranges.data(), sizeof(int2) * p.seg_ranges.size(),
                                       cudaMemcpyHostToDevice, st));
@@ -441,7 +442,7 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
         SMAX_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         try {
             if (packed)
-                sweep_solve<VT>(p.pack, B, X, k, row_major ? k : 1, row_major ? 1 : ld, p.status, st);
+                sweep_solve<VT>(p.pack, B, X, k, row_major ? k : 1, row_major ? 1 : ld, p.status, p.wait, st);
             else
                 tri_solve_raw<VT>(p, a.rp(), a.ci(), a.val.as<VT>(), D, B, X, k, row_major, ld, merge_rows, tag, st);
         } catch (...) {
@@ -464,6 +465,7 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
         p.graph_ld = ld;
         p.graph_k = k;
         p.graph_packed = packed;
+        p.graph_wait = p.wait;
     }
     SMAX_CUDA(cudaGraphLaunch(p.graph, st));
 }

@@ -47,6 +47,7 @@ struct TriPlan {
     bool graph_row_major = false;
     int64_t graph_ld = 0, graph_k = 0;
     bool graph_packed = false;
+    SweepWait graph_wait;
     AuxStream aux;  // capture stream when the caller's stream cannot be captured
 
     // level-ordered pack (sweep.cu), built for the value arrays, their version
@@ -57,6 +58,7 @@ struct TriPlan {
     uint64_t pack_tag = ~0ull;
     int pack_merge = -1, pack_vbytes = 0;
     DevStatus *status = nullptr;  // where a sweep reports a wait that gave up
+    SweepWait wait;               // how long its waits last
     // (re)builds the pack when its key changed (new values of the same arrays
     // are filled in); false when the matrix does not pack compactly and the
     // plain kernels must be used.  k > 1: rows divide by D, as the plain

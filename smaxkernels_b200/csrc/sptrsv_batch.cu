@@ -251,7 +251,7 @@ template <typename VT>
 void TriBatch::solve_persistent(const VT *B, VT *X, cudaStream_t st) {
     if (n_mats == 0) return;
     if (pack_ok) {
-        sweep_solve_batch<VT>(pack, queue_order.as<int>(), n_mats, queue.as<int>(), B, X, st);
+        sweep_solve_batch<VT>(pack, queue_order.as<int>(), n_mats, queue.as<int>(), B, X, SweepWait(), st);
         return;
     }
     int per_sm = 0;

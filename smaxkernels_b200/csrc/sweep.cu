@@ -60,11 +60,12 @@ static_assert(kLevels >= kGroups && kSlots >= kWindow + kGroups, "mbarriers for 
 // to i + kWindow - 1: the mbarrier must not have been used again by then.
 static_assert(kSlots > 2 * kWindow + kCopyWarps - 2, "mbarriers for the copying warps' lead");
 constexpr int kRecChunks = 32;             // chunks of a record, at most
-// Polls before a wait gives up: seconds, since the threads of a run wait while
-// one of them goes through a row of a million entries.
-constexpr long long kWaitLimit = 1 << 27;  // 20 ns each at least
-// Time of a level, in steps of 10 ns, up to which it is swept.
+// Time of a level, in steps of 10 ns, up to which it is swept: a quarter of
+// the waits' default limit, since the threads of a run wait while one of them
+// goes through a row of a million entries.
 constexpr long long kLevelTime = 1 << 26;
+// An arrived copy takes microseconds; a CTA does not end before its own have.
+constexpr long long kDrainNs = 2000000000ll;
 
 // header flags (the width is above them)
 constexpr int kFlagBits = 4;
@@ -364,6 +365,7 @@ struct SweepShared {
     unsigned long long full[kSlots];   // a record has arrived
     unsigned long long empty[kSlots];  // its operands are no longer needed
     unsigned long long level[kLevels]; // a level is solved
+    long long wait_ns;  // a wait gives up after this time
     int failed;  // a wait gave up
     int mat, rec0, level0;  // batch: the matrix taken, records and levels before it
 };
@@ -380,12 +382,74 @@ __device__ __forceinline__ void bulk_copy(unsigned dst, const void *src, unsigne
 
 __device__ __forceinline__ uint64_t *as_bar(unsigned long long *p) { return reinterpret_cast<uint64_t *>(p); }
 
+__device__ __forceinline__ long long sw_now() {
+    long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+constexpr int kPolls = 16;  // polls of a wait between two looks at the time
+constexpr unsigned kWarp = 0xffffffffu;
+
+__device__ __forceinline__ int sw_failed(const SweepShared *sh) { return *(const volatile int *)&sh->failed; }
+
+// Whether a wait that began at t0 (0: begins now) is over without what it waits
+// for: its time is up or another thread's was.  Returns when it began, 0 when it
+// is over.
+__device__ __noinline__ long long sw_patience(SweepShared *sh, long long t0) {
+    const long long now = sw_now();
+    if (t0 == 0) t0 = now;
+    if (now - t0 > sh->wait_ns) *(volatile int *)&sh->failed = 1;
+    return sw_failed(sh) ? 0 : t0;
+}
+
+// Waits of a whole warp for phase `parity` of bar, with one answer for all its
+// lanes: the warp's next __syncwarp has them all or none.  false: the wait gave
+// up, and the warp leaves the run without an arrival: the level mbarriers may
+// be in an earlier phase, where a wait returns at once and an arrival for more
+// than is pending is an error.  The vote costs 1 % (2048^2 natural FP64 2.40 ms
+// against 2.37); letting a warp go on without one and keeping back its arrivals
+// cost more (2.42 and 2.51).  The threads sleep in mbarrier.try_wait: polling
+// with test_wait took issue slots from the groups at work (512^2 natural FP64
+// 260 us against 223).
+__device__ __forceinline__ bool sw_wait(SweepShared *sh, unsigned long long *bar, unsigned parity) {
+    long long t0 = 0;
+#pragma unroll 1
+    for (int i = 1;; ++i) {
+        if (__all_sync(kWarp, mbar_try_wait(as_bar(bar), parity))) return true;
+        if (i % kPolls == 0) {
+            t0 = sw_patience(sh, t0);
+            if (__any_sync(kWarp, t0 == 0)) return false;
+        }
+    }
+}
+
+// The same for one lane.
+__device__ __forceinline__ bool sw_wait_lane(SweepShared *sh, unsigned long long *bar, unsigned parity) {
+    long long t0 = 0;
+#pragma unroll 1
+    for (int i = 1;; ++i) {
+        if (mbar_try_wait(as_bar(bar), parity)) return true;
+        if (i % kPolls == 0) {
+            t0 = sw_patience(sh, t0);
+            if (t0 == 0) return false;
+        }
+    }
+}
+
+// Until an issued copy has arrived, whatever else gave up.
+__device__ __forceinline__ void sw_drain(unsigned long long *bar, unsigned parity) {
+    const long long t0 = sw_now();
+    while (!mbar_try_wait(as_bar(bar), parity) && sw_now() - t0 < kDrainNs) {
+    }
+}
+
 // The copying warps take the run's records in turn, each once the records
 // whose room it needs are given back.  Issuing a record is a chain of about 500
 // cycles whatever its size, which with one warp held a run of wide levels to
 // 36 GB/s; so there are kCopyWarps of them.  Returns when the warp's copies have
 // arrived.
-__device__ __forceinline__ bool sw_copy(SweepShared *sh, unsigned stage, const Record *__restrict__ recs, int n_rec,
+__device__ __forceinline__ void sw_copy(SweepShared *sh, unsigned stage, const Record *__restrict__ recs, int n_rec,
                                         int base, const unsigned char *__restrict__ blob,
                                         const unsigned char *__restrict__ bp, int vbytes, int warp) {
     const int lane = threadIdx.x & 31;
@@ -396,7 +460,7 @@ __device__ __forceinline__ bool sw_copy(SweepShared *sh, unsigned stage, const R
             b = *(reinterpret_cast<const int4 *>(recs + i) + 1);
         }
     };
-    bool good = true;  // no wait has given up: after one, no further copy is issued
+    bool good = true;  // no wait has given up, here or elsewhere: after one, no further copy is issued
     int last = -1;     // the warp's last record issued
     fetch(kCopyWarps * lane + warp);
 #pragma unroll 1
@@ -409,7 +473,8 @@ __device__ __forceinline__ bool sw_copy(SweepShared *sh, unsigned stage, const R
             if (lane == j) {
 #pragma unroll 1
                 for (int f = base + cb.z; f < base + cb.y && good; ++f)
-                    good = mbar_wait_bounded(as_bar(&sh->empty[f % kSlots]), (unsigned)(f / kSlots) & 1u, kWaitLimit);
+                    good = sw_wait_lane(sh, &sh->empty[f % kSlots], (unsigned)(f / kSlots) & 1u);
+                good = good && !sw_failed(sh);
                 if (good) {
                     unsigned long long *bar = &sh->full[i % kSlots];
                     mbar_arrive_expect_tx(as_bar(bar), (unsigned)(ca.y + ca.w));
@@ -425,8 +490,7 @@ __device__ __forceinline__ bool sw_copy(SweepShared *sh, unsigned stage, const R
     // none of the warp's copies in flight: those before the last kSlots records were used
 #pragma unroll 1
     for (int i = last; i >= base && i > last - kSlots; i -= kCopyWarps)
-        mbar_wait_bounded(as_bar(&sh->full[i % kSlots]), (unsigned)(i / kSlots) & 1u, kWaitLimit);
-    return good;
+        sw_drain(&sh->full[i % kSlots], (unsigned)(i / kSlots) & 1u);
 }
 
 // A chunk's header.
@@ -624,13 +688,11 @@ __device__ __forceinline__ void sw_arrive(unsigned long long *bar, int count) {
     asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 
-// The wait for the level before.  The thread sleeps in mbarrier.try_wait: polling
-// with test_wait took issue slots from the groups at work (512^2 natural FP64
-// 260 us against 223, 2048^2 2.45 ms against 2.37).
+// The wait for the level before.
 __device__ __forceinline__ bool sw_wait_before(SweepShared *sh, const ChunkView &c, int level0) {
     if (c.level == 0) return true;
     const int l = level0 + c.level - 1;
-    return mbar_wait_bounded(as_bar(&sh->level[l % kLevels]), (unsigned)(l / kLevels) & 1u, kWaitLimit);
+    return sw_wait(sh, &sh->level[l % kLevels], (unsigned)(l / kLevels) & 1u);
 }
 
 // Chunk c of layout W for a group: operands, the wait for the level before, RW
@@ -697,16 +759,15 @@ __device__ void sw_run(const SweepPack::Run &run, const Record *__restrict__ rec
     unsigned char *ring = smem + kSharedBytes;
     const unsigned char *stage = smem + kSharedBytes + ring_bytes<VT>();
     if (threadIdx.x >= kGroups * T) {
-        if (!sw_copy(sh, smem_u32(stage), recs + run.rec0, run.n_rec, rec0, blob,
-                     reinterpret_cast<const unsigned char *>(bp), (int)sizeof(VT), (int)(threadIdx.x - kGroups * T) / 32))
-            *(volatile int *)&sh->failed = 1;
+        sw_copy(sh, smem_u32(stage), recs + run.rec0, run.n_rec, rec0, blob,
+                reinterpret_cast<const unsigned char *>(bp), (int)sizeof(VT), (int)(threadIdx.x - kGroups * T) / 32);
     } else {
         const int g = threadIdx.x / T, t = threadIdx.x % T;
         int at = run.at[g], rec = rec0 + run.rec[g];
         bool good = true;
 #pragma unroll 1
         while (at >= 0 && good) {
-            good = mbar_wait_bounded(as_bar(&sh->full[rec % kSlots]), (unsigned)(rec / kSlots) & 1u, kWaitLimit);
+            good = sw_wait(sh, &sh->full[rec % kSlots], (unsigned)(rec / kSlots) & 1u);
             if (!good) break;
             const ChunkView c = sw_view(stage, at);
             const int kind = c.wf & (kTwo | kThree | kRingOnly);
@@ -723,7 +784,6 @@ __device__ void sw_run(const SweepPack::Run &run, const Record *__restrict__ rec
             at = c.next;
             rec = rec0 + c.next_rec;
         }
-        if (!good) *(volatile int *)&sh->failed = 1;
     }
     __syncthreads();
 }
@@ -735,7 +795,8 @@ template <typename VT> __device__ __forceinline__ void sw_no_solution(const Swee
 }
 
 // level_arrivals, rec_arrivals: what completes a level and gives a record back
-template <typename VT> __device__ __forceinline__ void sw_init(unsigned char *smem, int level_arrivals, int rec_arrivals) {
+template <typename VT>
+__device__ __forceinline__ void sw_init(unsigned char *smem, int level_arrivals, int rec_arrivals, const SweepWait &wait) {
     SweepShared *sh = reinterpret_cast<SweepShared *>(smem);
     if (threadIdx.x == 0) {
 #pragma unroll 1
@@ -743,7 +804,8 @@ template <typename VT> __device__ __forceinline__ void sw_init(unsigned char *sm
             mbar_init(as_bar(&sh->full[i]), 1);
             mbar_init(as_bar(&sh->empty[i]), rec_arrivals);
         }
-        for (int i = 0; i < kLevels; ++i) mbar_init(as_bar(&sh->level[i]), level_arrivals);
+        for (int i = 0; i < kLevels; ++i) mbar_init(as_bar(&sh->level[i]), level_arrivals + (wait.never ? 1 : 0));
+        sh->wait_ns = wait.ns;
         sh->failed = 0;
         mbar_fence_init();
         reinterpret_cast<VT *>(smem + kSharedBytes)[kRing] = VT(0);  // the slot of padding
@@ -754,9 +816,9 @@ template <typename VT> __device__ __forceinline__ void sw_init(unsigned char *sm
 template <typename VT, int T, bool DIV>
 __global__ void __launch_bounds__(kGroups * T + 32 * kCopyWarps, 1)
     sweep_kernel(const SweepPack::Run run, const Record *__restrict__ recs, const unsigned char *__restrict__ blob,
-                 int64_t npos, const VT *__restrict__ bp, VT *xp, DevStatus *status) {
+                 int64_t npos, const VT *__restrict__ bp, VT *xp, DevStatus *status, const SweepWait wait) {
     extern __shared__ __align__(128) unsigned char smem[];
-    sw_init<VT>(smem, run.level_chunks * (T / 32), kRecChunks * (T / 32));
+    sw_init<VT>(smem, run.level_chunks * (T / 32), kRecChunks * (T / 32), wait);
     __syncthreads();
     bp += blockIdx.x * npos;
     xp += blockIdx.x * npos;
@@ -772,10 +834,10 @@ template <typename VT, int T>
 __global__ void __launch_bounds__(kGroups * T + 32 * kCopyWarps, T <= 32 ? 2 : 1)
     sweep_batch_kernel(const SweepPack::Run *__restrict__ runs, const int *__restrict__ queue_order, int n_mats,
                        int *queue, const Record *__restrict__ recs, const unsigned char *__restrict__ blob,
-                       const VT *__restrict__ bp, VT *xp) {
+                       const VT *__restrict__ bp, VT *xp, const SweepWait wait) {
     extern __shared__ __align__(128) unsigned char smem[];
     SweepShared *sh = reinterpret_cast<SweepShared *>(smem);
-    sw_init<VT>(smem, runs[0].level_chunks * (T / 32), kRecChunks * (T / 32));
+    sw_init<VT>(smem, runs[0].level_chunks * (T / 32), kRecChunks * (T / 32), wait);
     // what the CTA keeps from one matrix to the next is in shared memory: the
     // sweep needs the registers
     volatile SweepShared *vs = sh;
@@ -829,12 +891,12 @@ int group_threads(int max_rows) { return max_rows <= 32 ? 32 : (max_rows <= 64 ?
 
 template <typename VT, bool DIV>
 void launch_run(const SweepPack &pk, const SweepPack::Run &run, int threads, int64_t k, const VT *bp, VT *xp,
-                DevStatus *status, cudaStream_t st) {
+                DevStatus *status, const SweepWait &wait, cudaStream_t st) {
     const size_t sm = sweep_smem(pk);
     const Record *recs = pk.recs.as<Record>();
     const unsigned char *blob = pk.blob.as<unsigned char>();
     auto go = [&](auto kern, int t) {
-        kern<<<(unsigned)k, kGroups * t + 32 * kCopyWarps, sm, st>>>(run, recs, blob, pk.npos, bp, xp, status);
+        kern<<<(unsigned)k, kGroups * t + 32 * kCopyWarps, sm, st>>>(run, recs, blob, pk.npos, bp, xp, status, wait);
     };
     if (threads == 32) go(sweep_kernel<VT, 32, DIV>, 32);
     else if (threads == 64) go(sweep_kernel<VT, 64, DIV>, 64);
@@ -1139,7 +1201,7 @@ void sweep_reserve(SweepPack &pk, int64_t k) {
 
 template <typename VT>
 void sweep_solve(const SweepPack &pk, const VT *B, VT *X, int64_t k, int64_t rs, int64_t vs, DevStatus *status,
-                 cudaStream_t st) {
+                 const SweepWait &wait, cudaStream_t st) {
     if (pk.n == 0 || k == 0) return;
     if (pk.vectors < 1) fail(SMAX_ERR_STATE, "the sweep has no workspace");
     VT *bp = pk.bp.as<VT>(), *xp = pk.xp.as<VT>();
@@ -1156,9 +1218,9 @@ void sweep_solve(const SweepPack &pk, const VT *B, VT *X, int64_t k, int64_t rs,
                 if (pk.div) sw_wide_kernel<VT, true><<<g, 256, 0, st>>>(L, blob, pk.npos, bp, xp);
                 else sw_wide_kernel<VT, false><<<g, 256, 0, st>>>(L, blob, pk.npos, bp, xp);
             } else if (pk.div) {
-                launch_run<VT, true>(pk, pk.runs[it.index], it.threads, kv, bp, xp, status, st);
+                launch_run<VT, true>(pk, pk.runs[it.index], it.threads, kv, bp, xp, status, wait, st);
             } else {
-                launch_run<VT, false>(pk, pk.runs[it.index], it.threads, kv, bp, xp, status, st);
+                launch_run<VT, false>(pk, pk.runs[it.index], it.threads, kv, bp, xp, status, wait, st);
             }
         }
         sw_scatter<VT>(pk, Xv, kv, rs, vs, st);
@@ -1168,7 +1230,7 @@ void sweep_solve(const SweepPack &pk, const VT *B, VT *X, int64_t k, int64_t rs,
 
 template <typename VT>
 void sweep_solve_batch(const SweepPack &pk, const int *queue_order, int n_mats, int *queue, const VT *B, VT *X,
-                       cudaStream_t st) {
+                       const SweepWait &wait, cudaStream_t st) {
     if (pk.n == 0 || n_mats == 0) return;
     VT *bp = pk.bp.as<VT>(), *xp = pk.xp.as<VT>();
     sw_gather<VT>(pk, B, X, 1, 1, 1, st);
@@ -1179,7 +1241,7 @@ void sweep_solve_batch(const SweepPack &pk, const int *queue_order, int n_mats, 
     const size_t sm = sweep_smem(pk);
     auto go = [&](auto kern, int t) {
         kern<<<ctas, kGroups * t + 32 * kCopyWarps, sm, st>>>(pk.drun.as<SweepPack::Run>(), queue_order, n_mats, queue, pk.recs.as<Record>(),
-                                       pk.blob.as<unsigned char>(), bp, xp);
+                                       pk.blob.as<unsigned char>(), bp, xp, wait);
     };
     if (threads == 32) go(sweep_batch_kernel<VT, 32>, 32);
     else if (threads == 64) go(sweep_batch_kernel<VT, 64>, 64);
@@ -1189,12 +1251,12 @@ void sweep_solve_batch(const SweepPack &pk, const int *queue_order, int n_mats, 
 }
 
 template void sweep_solve<double>(const SweepPack &, const double *, double *, int64_t, int64_t, int64_t, DevStatus *,
-                                  cudaStream_t);
+                                  const SweepWait &, cudaStream_t);
 template void sweep_solve<float>(const SweepPack &, const float *, float *, int64_t, int64_t, int64_t, DevStatus *,
-                                 cudaStream_t);
+                                 const SweepWait &, cudaStream_t);
 template void sweep_solve_batch<double>(const SweepPack &, const int *, int, int *, const double *, double *,
-                                        cudaStream_t);
+                                        const SweepWait &, cudaStream_t);
 template void sweep_solve_batch<float>(const SweepPack &, const int *, int, int *, const float *, float *,
-                                       cudaStream_t);
+                                       const SweepWait &, cudaStream_t);
 
 }  // namespace smax

@@ -62,6 +62,14 @@ struct SweepPack {
     bool needs_x_init = false;  // some entry reads a solution not computed before it
 };
 
+// How long the waits of a sweep last.
+struct SweepWait {
+    static constexpr long long kPollNs = 128;  // a limit given in polls counts this many nanoseconds for each
+    long long ns = 20000000 * kPollNs;
+    bool never = false;  // test: the levels wait for an arrival that never comes
+    bool operator!=(const SweepWait &o) const { return ns != o.ns || never != o.never; }
+};
+
 struct SweepStep {
     int first, count, kind;  // first sweep step, steps, kind 0: a wide level (grid) / 1: a run (one CTA)
 };
@@ -86,16 +94,16 @@ void refill_sweep_pack(SweepPack &pk, const int *rp, const void *val, const void
 void sweep_reserve(SweepPack &pk, int64_t k);
 
 // Solves k right-hand sides, element (r, v) of B and X at r * rs + v * vs.
-// status (may be null) gets SMAX_ERR_TIMEOUT if a bounded wait gives up; the
-// solutions not computed are then NaN.
+// status (may be null) gets SMAX_ERR_TIMEOUT if a wait gives up; the solutions
+// of its run are then NaN.
 template <typename VT>
 void sweep_solve(const SweepPack &pk, const VT *B, VT *X, int64_t k, int64_t rs, int64_t vs, DevStatus *status,
-                 cudaStream_t st);
+                 const SweepWait &wait, cudaStream_t st);
 
 // One CTA per run, runs (independent matrices) taken from a device work queue
 // in the order queue_order.
 template <typename VT>
 void sweep_solve_batch(const SweepPack &pk, const int *queue_order, int n_mats, int *queue, const VT *B, VT *X,
-                       cudaStream_t st);
+                       const SweepWait &wait, cudaStream_t st);
 
 }  // namespace smax

@@ -249,7 +249,7 @@ class Kernel:
         return self._flag("solve_mode", mode)
 
     def set_spin_limit(self, kilo_polls: int):
-        """Polls (x 1000) before a wait of the persistent or sync-free solve gives up with TIMEOUT."""
+        """Polls (x 1000) before a wait of a solve gives up with TIMEOUT (a level sweep counts 128 ns a poll)."""
         return self._flag("spin_limit", kilo_polls)
 
     def set_sweep_cluster(self, v: bool):

@@ -209,3 +209,27 @@ def test_batches(vt, count, most):
         a, e = tb.row_offset(m), tb.row_offset(m + 1)
         assert normwise(x[a:e], O.sptrsv(rp, col, val, b[a:e])) <= tol(vt), m
     tb.close()
+
+
+@pytest.mark.parametrize("kind,k,mode", [("SPTRSV", 1, 0), ("SPTRSV", 1, MERGED), ("SPTRSM", 3, 0)])
+@pytest.mark.parametrize("most", [30, 60, 400])
+def test_a_wait_that_runs_out_is_an_error_and_recoverable(kind, k, mode, most):
+    """A level waits for an arrival that never comes: the sweep ends, reports
+    TIMEOUT and leaves no number behind, and the same kernel solves afterwards."""
+    from smaxkernels_b200 import SmaxError, _lib
+    rp, col, val = level_matrix([most, most - 3, 2] * 20, 4, most, np.float64)
+    n = len(rp) - 1
+    b = np.random.default_rng(12).uniform(-1, 1, n * k)
+    smax, kern, x = _kernel(kind, rp, col, val, b, k=k, mode=mode)
+    kern.set_spin_limit(5)
+    kern._flag("test_force_timeout", 1)
+    with pytest.raises(SmaxError) as e:
+        kern.run()
+    assert e.value.code == _lib.ERR_TIMEOUT
+    assert np.isnan(x).all()
+    kern._flag("test_force_timeout", 0)
+    kern.run()
+    smax.close()
+    B = b.reshape(n, k)
+    ref = np.stack([O.sptrsv(rp, col, val, np.ascontiguousarray(B[:, v])) for v in range(k)], 1)
+    assert normwise(x.reshape(n, k), ref) <= tol(np.float64)
