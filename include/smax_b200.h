@@ -293,8 +293,8 @@ smax_status smax_utils_tune_spmv_format(int float_type, uint64_t n_rows, uint64_
  * its diagonal; no counterpart in the reference, which solves one matrix per
  * kernel) solved together: one persistent kernel whose CTAs take matrices from
  * a device work queue (longest critical path first) and sweep each matrix's
- * dependency levels with the CTA barrier as the level barrier.  The batch owns
- * device copies; the caller's arrays are not modified. */
+ * dependency levels.  The batch owns device copies; the caller's arrays are not
+ * modified. */
 typedef struct smax_batch_s *smax_batch;
 smax_status smax_batch_sptrsv_create(smax_batch *out, int float_type, int n_mats, const uint64_t *n_rows,
                                      const uint64_t *nnz, void *const *row_ptr, void *const *col, void *const *val);
@@ -302,8 +302,15 @@ smax_status smax_batch_sptrsv_create(smax_batch *out, int float_type, int n_mats
  * smax_batch_row_offset(b, m)); mode: SMAX_SOLVE_GRAPH (persistent kernel
  * replayed from a CUDA graph), SMAX_SOLVE_MERGED (persistent kernel, direct
  * launch) or SMAX_SOLVE_PER_LEVEL (one launch per level of every matrix, the
- * plain baseline).  stream: a cudaStream_t (NULL = legacy default stream). */
+ * plain baseline).  stream: a cudaStream_t (NULL = legacy default stream).
+ * Returns when the solve is queued.  A wait of the sweeps that gives up leaves NaN
+ * in its matrix and SMAX_ERR_TIMEOUT, returned by smax_batch_sync or else by a
+ * later solve (which is then not queued). */
 smax_status smax_batch_sptrsv_solve(smax_batch b, const void *rhs, void *x, int mode, void *stream);
+/* waits for the solves queued on the stream and returns their error */
+smax_status smax_batch_sync(smax_batch b, void *stream);
+/* SMAX_FLAG_SPIN_LIMIT, SMAX_FLAG_TEST_FORCE_TIMEOUT */
+smax_status smax_batch_set_flag(smax_batch b, int flag, int value);
 uint64_t smax_batch_row_offset(smax_batch b, int m);
 /* total packed rows, sum of the matrices' level counts, largest level count */
 smax_status smax_batch_info(smax_batch b, uint64_t *n_rows, int *total_levels, int *max_levels);

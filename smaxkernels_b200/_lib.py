@@ -59,6 +59,8 @@ SIGNATURES = {
     "smax_utils_tune_spmv_format": (I32, [I32, U64, U64, U64, P, P, P, P]),
     "smax_batch_sptrsv_create": (I32, [PP, I32, I32, PU64, PU64, PP, PP, PP]),
     "smax_batch_sptrsv_solve": (I32, [P, P, P, I32, P]),
+    "smax_batch_sync": (I32, [P, P]),
+    "smax_batch_set_flag": (I32, [P, I32, I32]),
     "smax_batch_row_offset": (U64, [P, I32]),
     "smax_batch_info": (I32, [P, PU64, C.POINTER(I32), C.POINTER(I32)]),
     "smax_batch_destroy": (I32, [P]),

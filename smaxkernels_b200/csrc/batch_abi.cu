@@ -61,6 +61,27 @@ smax_status smax_batch_sptrsv_solve(smax_batch b, const void *rhs, void *x, int 
     });
 }
 
+smax_status smax_batch_sync(smax_batch b, void *stream) {
+    return guarded([&] {
+        if (!b) fail(SMAX_ERR_BAD_ARG, "null batch");
+        b->tb.sync(static_cast<cudaStream_t>(stream));
+    });
+}
+
+smax_status smax_batch_set_flag(smax_batch b, int flag, int value) {
+    return guarded([&] {
+        if (!b) fail(SMAX_ERR_BAD_ARG, "null batch");
+        switch (flag) {
+        case SMAX_FLAG_SPIN_LIMIT:
+            if (value <= 0) fail(SMAX_ERR_BAD_ARG, "spin limit must be positive");
+            b->tb.wait.ns = (long long)value * 1000 * SweepWait::kPollNs;
+            break;
+        case SMAX_FLAG_TEST_FORCE_TIMEOUT: b->tb.wait.never = value != 0; break;
+        default: fail(SMAX_ERR_BAD_ARG, "not a flag of a batch");
+        }
+    });
+}
+
 uint64_t smax_batch_row_offset(smax_batch b, int m) {
     if (!b || m < 0 || m > b->tb.n_mats) return 0;
     return m == b->tb.n_mats ? (uint64_t)b->tb.n_rows : (uint64_t)b->tb.row_off[m];

@@ -4,13 +4,12 @@
 //    persistent launch.  The matrices are packed back to back (global row
 //    numbering, their rows sorted by dependency level).  Each CTA takes the
 //    next matrix from a device work queue (an atomic counter over the matrices
-//    in longest-first order) and sweeps that matrix's levels, with
-//    __syncthreads() as the level barrier; when done it takes the next one.
-//    The sweep runs on the level-ordered pack of the batch (sweep.cu:
-//    per-level ELL blocks copied ahead into shared memory, a ring of recent
-//    solutions); matrices that would pack too sparsely use the plain kernel
-//    below.  The queue is a fetch-add, the level barrier is the CTA barrier,
-//    and the waits on the copies are bounded.  The launch (queue reset + kernel) is
+//    in longest-first order) and sweeps that matrix's levels; when done it takes
+//    the next one.  The sweep runs on the level-ordered pack of the batch
+//    (sweep.cu: operands copied ahead into shared memory, a ring of recent
+//    solutions, an mbarrier per level; every wait is bounded and one that gives up
+//    is reported).  Matrices that would pack too sparsely use the plain kernel
+//    below, whose level barrier is the CTA barrier.  The launch (queue reset + kernel) is
 //    captured once into a CUDA graph and replayed.
 // 2. Grid-wide persistent (one matrix, wide levels): a cooperative launch of
 //    co-resident CTAs sweeps all levels, with a software grid barrier between
@@ -243,6 +242,8 @@ void TriBatch::build(int vbytes_, const std::vector<RegCRS> &mats, cudaStream_t 
         }
         steps.push_back(SweepStep{moff[m], moff[m + 1] - moff[m], 1});
     }
+    SMAX_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&error.p), sizeof(int), cudaHostAllocMapped));
+    *error.p = 0;
     pack_ok = build_sweep_pack(pack, A.rp(), A.ci(), A.val.p, D.p, vbytes, n_rows, order.as<int>(), src_begin, count,
                                steps, false, true, st);
 }
@@ -250,8 +251,9 @@ void TriBatch::build(int vbytes_, const std::vector<RegCRS> &mats, cudaStream_t 
 template <typename VT>
 void TriBatch::solve_persistent(const VT *B, VT *X, cudaStream_t st) {
     if (n_mats == 0) return;
+    check_status();
     if (pack_ok) {
-        sweep_solve_batch<VT>(pack, queue_order.as<int>(), n_mats, queue.as<int>(), B, X, SweepWait(), st);
+        sweep_solve_batch<VT>(pack, queue_order.as<int>(), n_mats, queue.as<int>(), B, X, error.p, wait, st);
         return;
     }
     int per_sm = 0;
@@ -267,6 +269,7 @@ void TriBatch::solve_persistent(const VT *B, VT *X, cudaStream_t st) {
 template <typename VT>
 void TriBatch::solve_graph(const VT *B, VT *X, cudaStream_t caller) {
     if (n_mats == 0) return;
+    check_status();
     const bool fenced = !is_capturable(caller);
     cudaStream_t st = fenced ? aux.enter(caller) : caller;
     struct Leave {
@@ -280,7 +283,7 @@ void TriBatch::solve_graph(const VT *B, VT *X, cudaStream_t caller) {
             }
         }
     } leave{aux, fenced, caller};
-    if (!graph || graph_b != B || graph_x != X) {
+    if (!graph || graph_b != B || graph_x != X || graph_wait != wait) {
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
         SMAX_CUDA(cudaStreamSynchronize(st));
@@ -299,6 +302,7 @@ void TriBatch::solve_graph(const VT *B, VT *X, cudaStream_t caller) {
         cuda_check(e, "cudaGraphInstantiate");
         graph_b = B;
         graph_x = X;
+        graph_wait = wait;
     }
     SMAX_CUDA(cudaGraphLaunch(graph, st));
 }
@@ -312,6 +316,19 @@ void TriBatch::solve_per_level(const VT *B, VT *X, cudaStream_t st) {
                                                                     order.as<int>(), a, b, B, X);
         }
     SMAX_CUDA(cudaGetLastError());
+}
+
+void TriBatch::check_status() {
+    if (!error.p) return;
+    const int code = *(volatile int *)error.p;
+    if (code == 0) return;
+    *(volatile int *)error.p = 0;
+    fail(code, "a wait of a batched solve gave up: the solutions of its matrix are NaN");
+}
+
+void TriBatch::sync(cudaStream_t st) {
+    SMAX_CUDA(cudaStreamSynchronize(st));
+    check_status();
 }
 
 TriBatch::~TriBatch() {

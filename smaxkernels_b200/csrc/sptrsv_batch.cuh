@@ -12,6 +12,15 @@ namespace smax {
 // A batch of independent lower-triangular matrices packed as one
 // block-diagonal CRS (global row numbers), with per-matrix level sets.
 struct TriBatch {
+    // Error word of the sweeps in pinned host memory: solves are asynchronous, so
+    // a wait that gave up is reported by the next solve or by sync().  (The
+    // first member: freed after the device buffers, which waits for the device.)
+    struct HostWord {
+        int *p = nullptr;
+        ~HostWord() {
+            if (p) cudaFreeHost(p);
+        }
+    } error;
     int vbytes = 8;
     int n_mats = 0;
     int64_t n_rows = 0, nnz = 0;
@@ -23,6 +32,7 @@ struct TriBatch {
     DevBuf D, order, mat_lvl_off, lvl_rows, queue_order, queue;
     SweepPack pack;          // level-ordered pack, one single-CTA run per matrix
     bool pack_ok = false;    // false: the plain batch kernel (the pack would be too sparse)
+    SweepWait wait, graph_wait;
     cudaGraphExec_t graph = nullptr;
     const void *graph_b = nullptr, *graph_x = nullptr;
     AuxStream aux;  // capture stream when the caller's stream cannot be captured
@@ -31,6 +41,8 @@ struct TriBatch {
     template <typename VT> void solve_persistent(const VT *B, VT *X, cudaStream_t st);
     template <typename VT> void solve_graph(const VT *B, VT *X, cudaStream_t st);
     template <typename VT> void solve_per_level(const VT *B, VT *X, cudaStream_t st);
+    void check_status();  // fails if a solve has reported an error, and forgets it
+    void sync(cudaStream_t st);
     ~TriBatch();
 };
 

@@ -834,7 +834,7 @@ template <typename VT, int T>
 __global__ void __launch_bounds__(kGroups * T + 32 * kCopyWarps, T <= 32 ? 2 : 1)
     sweep_batch_kernel(const SweepPack::Run *__restrict__ runs, const int *__restrict__ queue_order, int n_mats,
                        int *queue, const Record *__restrict__ recs, const unsigned char *__restrict__ blob,
-                       const VT *__restrict__ bp, VT *xp, const SweepWait wait) {
+                       const VT *__restrict__ bp, VT *xp, int *status, const SweepWait wait) {
     extern __shared__ __align__(128) unsigned char smem[];
     SweepShared *sh = reinterpret_cast<SweepShared *>(smem);
     sw_init<VT>(smem, runs[0].level_chunks * (T / 32), kRecChunks * (T / 32), wait);
@@ -852,7 +852,10 @@ __global__ void __launch_bounds__(kGroups * T + 32 * kCopyWarps, T <= 32 ? 2 : 1
         if (vs->mat < 0) return;
         if (!vs->failed) sw_run<VT, T, false>(runs[vs->mat], recs, blob, bp, xp, smem, vs->rec0, vs->level0);
         const SweepPack::Run &run = runs[vs->mat];
-        if (vs->failed) sw_no_solution<VT>(run, xp);
+        if (vs->failed) {
+            if (threadIdx.x == 0) *(volatile int *)status = SMAX_ERR_TIMEOUT;
+            sw_no_solution<VT>(run, xp);
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
             vs->rec0 = vs->rec0 + run.n_rec;
@@ -1230,7 +1233,7 @@ void sweep_solve(const SweepPack &pk, const VT *B, VT *X, int64_t k, int64_t rs,
 
 template <typename VT>
 void sweep_solve_batch(const SweepPack &pk, const int *queue_order, int n_mats, int *queue, const VT *B, VT *X,
-                       const SweepWait &wait, cudaStream_t st) {
+                       int *status, const SweepWait &wait, cudaStream_t st) {
     if (pk.n == 0 || n_mats == 0) return;
     VT *bp = pk.bp.as<VT>(), *xp = pk.xp.as<VT>();
     sw_gather<VT>(pk, B, X, 1, 1, 1, st);
@@ -1241,7 +1244,7 @@ void sweep_solve_batch(const SweepPack &pk, const int *queue_order, int n_mats, 
     const size_t sm = sweep_smem(pk);
     auto go = [&](auto kern, int t) {
         kern<<<ctas, kGroups * t + 32 * kCopyWarps, sm, st>>>(pk.drun.as<SweepPack::Run>(), queue_order, n_mats, queue, pk.recs.as<Record>(),
-                                       pk.blob.as<unsigned char>(), bp, xp, wait);
+                                       pk.blob.as<unsigned char>(), bp, xp, status, wait);
     };
     if (threads == 32) go(sweep_batch_kernel<VT, 32>, 32);
     else if (threads == 64) go(sweep_batch_kernel<VT, 64>, 64);
@@ -1255,8 +1258,8 @@ template void sweep_solve<double>(const SweepPack &, const double *, double *, i
 template void sweep_solve<float>(const SweepPack &, const float *, float *, int64_t, int64_t, int64_t, DevStatus *,
                                  const SweepWait &, cudaStream_t);
 template void sweep_solve_batch<double>(const SweepPack &, const int *, int, int *, const double *, double *,
-                                        const SweepWait &, cudaStream_t);
+                                        int *, const SweepWait &, cudaStream_t);
 template void sweep_solve_batch<float>(const SweepPack &, const int *, int, int *, const float *, float *,
-                                       const SweepWait &, cudaStream_t);
+                                       int *, const SweepWait &, cudaStream_t);
 
 }  // namespace smax

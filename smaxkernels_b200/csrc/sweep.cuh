@@ -101,9 +101,11 @@ void sweep_solve(const SweepPack &pk, const VT *B, VT *X, int64_t k, int64_t rs,
                  const SweepWait &wait, cudaStream_t st);
 
 // One CTA per run, runs (independent matrices) taken from a device work queue
-// in the order queue_order.
+// in the order queue_order.  *status (which the host can read) becomes
+// SMAX_ERR_TIMEOUT if a wait gives up; the solutions of that matrix and of those
+// its CTA takes after it are then NaN.
 template <typename VT>
 void sweep_solve_batch(const SweepPack &pk, const int *queue_order, int n_mats, int *queue, const VT *B, VT *X,
-                       const SweepWait &wait, cudaStream_t st);
+                       int *status, const SweepWait &wait, cudaStream_t st);
 
 }  // namespace smax

@@ -390,6 +390,14 @@ class TriangularBatch:
         (0, the default, is torch's default stream)."""
         check(lib.smax_batch_sptrsv_solve(self._h, _ptr(rhs), _ptr(x), int(mode), _stream_arg(stream)))
 
+    def sync(self, stream: int = 0):
+        """Waits for the solves queued on the stream; TIMEOUT if a wait in one of them gave up
+        (solve() is asynchronous: without this call the next solve() raises it)."""
+        check(lib.smax_batch_sync(self._h, _stream_arg(stream)))
+
+    def _flag(self, name, v):
+        check(lib.smax_batch_set_flag(self._h, FLAG[name], int(v)))
+
     def close(self):
         if self._h:
             lib.smax_batch_destroy(self._h)

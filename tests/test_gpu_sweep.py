@@ -211,6 +211,35 @@ def test_batches(vt, count, most):
     tb.close()
 
 
+@pytest.mark.parametrize("mode", [0, MERGED])
+def test_a_wait_that_runs_out_in_a_batch_is_reported(mode):
+    """solve() is asynchronous: sync() raises TIMEOUT, or else the next solve() does."""
+    import torch
+    from smaxkernels_b200 import SmaxError, _lib
+    from smaxkernels_b200.interface import TriangularBatch
+    rng = np.random.default_rng(13)
+    mats = [level_matrix([40, 3, 90] * 6, 3, m, np.float64) for m in range(200)]
+    tb = TriangularBatch(mats)
+    b = rng.uniform(-1, 1, sum(len(m[0]) - 1 for m in mats))
+    bd, xd = torch.from_numpy(b).cuda(), torch.zeros(len(b), dtype=torch.float64, device="cuda")
+    tb._flag("spin_limit", 5)
+    tb._flag("test_force_timeout", 1)
+    for report in (tb.sync, lambda: (torch.cuda.synchronize(), tb.solve(bd, xd, mode))):
+        tb.solve(bd, xd, mode)
+        with pytest.raises(SmaxError) as e:
+            report()
+        assert e.value.code == _lib.ERR_TIMEOUT
+        assert torch.isnan(xd).all()
+    tb._flag("test_force_timeout", 0)
+    tb.solve(bd, xd, mode)
+    tb.sync()
+    x = xd.cpu().numpy()
+    for m, (rp, col, val) in enumerate(mats):
+        a, e = tb.row_offset(m), tb.row_offset(m + 1)
+        assert normwise(x[a:e], O.sptrsv(rp, col, val, b[a:e])) <= tol(np.float64), m
+    tb.close()
+
+
 @pytest.mark.parametrize("kind,k,mode", [("SPTRSV", 1, 0), ("SPTRSV", 1, MERGED), ("SPTRSM", 3, 0)])
 @pytest.mark.parametrize("most", [30, 60, 400])
 def test_a_wait_that_runs_out_is_an_error_and_recoverable(kind, k, mode, most):
