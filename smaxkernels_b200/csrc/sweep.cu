@@ -9,7 +9,9 @@
 // what its successor has to wait for:
 //
 //   * solutions a row needs are read from the shared-memory ring of the last
-//     kRing positions (a slot is safe while q >= level_end - kRing);
+//     kRing positions (a slot is safe while q >= level_end - kRing; in a level of
+//     more than kRing positions, whose chunks are stored in no order, only its
+//     first kRing have a slot that no other of the level writes);
 //   * every other operand is in shared memory already: some warps issue bulk
 //     copies (cp.async.bulk, completion on an mbarrier) of whole records, as
 //     far ahead as the stage has room, and needs no register of the others;
@@ -164,13 +166,14 @@ template <typename VT> struct RowSlots {
 };
 
 // One position's entries.  PATTERN: source codes too (and which chunks read
-// global solutions); otherwise new values only.
+// global solutions); otherwise new values only.  wraps: some level of a run has
+// more than kRing positions.
 template <typename VT, bool PATTERN>
 __global__ void sw_fill_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT *__restrict__ val,
                                const VT *__restrict__ D, int64_t npos, const int *__restrict__ prow,
                                const int *__restrict__ pchunk, const int *__restrict__ pos_of_row,
                                const ChunkDesc *__restrict__ ch, unsigned char *__restrict__ blob, bool div,
-                               int *__restrict__ reads_global, int *__restrict__ needs_init) {
+                               bool wraps, int *__restrict__ reads_global, int *__restrict__ needs_init) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < npos; p += stride) {
         const int r = prow[p];
@@ -186,7 +189,8 @@ __global__ void sw_fill_kernel(const int *__restrict__ rp, const int *__restrict
                 if (i < len) {
                     const int q = pos_of_row[ci[j0 + i]];
                     if (q >= c.lpos) atomicExch(needs_init, 1);
-                    const bool ring = q >= c.rpos && q < c.lpos && q >= c.lend - kRing;
+                    bool ring = q >= c.rpos && q < c.lpos && q >= c.lend - kRing;
+                    if (ring && wraps) ring = q - ch[pchunk[q]].lpos < kRing;
                     code = ring ? (q & (kRing - 1)) * (int)sizeof(VT) : ~q;
                     if (!ring) reads_global[pchunk[p]] = 1;
                 }
@@ -974,6 +978,7 @@ bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *v
     // 3.37 (a copy costs its issue), a tenth 3.11, a fifth 2.47
     const int chunk_cap = S / 6 / 16 * 16, rec_cap = S / 8 / 16 * 16;
     int64_t off = 0, pos = 0;  // blob bytes, positions
+    bool wraps = false;
     auto add_chunk = [&](int s, int t0, int m, int lpos, int lend, int rpos, int flags, int level,
                          int pad = 4) {
         ChunkDesc d{};
@@ -1016,6 +1021,7 @@ bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *v
         for (int s = step.first; s < step.first + step.count; ++s) {
             const int m = count[s];
             if (m == 0) continue;
+            wraps = wraps || m > kRing - 4;
             // a level near the waits' limit (an entry after the other in its rows,
             // and what the SM takes in) is left to the plain kernels
             if (25ll * w[s] * (m / (kGroups * T) + 1) + (long long)m * w[s] / 4 > kLevelTime) return false;
@@ -1160,8 +1166,8 @@ bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *v
         using VT = decltype(zero);
         sw_fill_kernel<VT, true><<<grid_for(pos), 256, 0, st>>>(
             rp, ci, static_cast<const VT *>(val), static_cast<const VT *>(D), pos, pk.prow.as<int>(),
-            pk.pchunk.as<int>(), pos_of_row.as<int>(), dch, pk.blob.as<unsigned char>(), div, glob.as<int>(),
-            flag.as<int>());
+            pk.pchunk.as<int>(), pos_of_row.as<int>(), dch, pk.blob.as<unsigned char>(), div, wraps,
+            glob.as<int>(), flag.as<int>());
     };
     if (vbytes == 8) fill(0.0);
     else fill(0.0f);
@@ -1182,8 +1188,8 @@ void refill_sweep_pack(SweepPack &pk, const int *rp, const void *val, const void
         using VT = decltype(zero);
         sw_fill_kernel<VT, false><<<grid_for(pk.npos), 256, 0, st>>>(
             rp, nullptr, static_cast<const VT *>(val), static_cast<const VT *>(D), pk.npos, pk.prow.as<int>(),
-            pk.pchunk.as<int>(), nullptr, pk.chunks.as<ChunkDesc>(), pk.blob.as<unsigned char>(), pk.div, nullptr,
-            nullptr);
+            pk.pchunk.as<int>(), nullptr, pk.chunks.as<ChunkDesc>(), pk.blob.as<unsigned char>(), pk.div, false,
+            nullptr, nullptr);
     };
     if (pk.vbytes == 8) fill(0.0);
     else fill(0.0f);

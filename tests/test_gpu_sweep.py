@@ -189,6 +189,40 @@ def test_new_values_sync_free():
     smax.close()
 
 
+def wide_levels(sizes, width, seed, vt):
+    """level_matrix with exactly `width` sources a row, all in the level before."""
+    rng = np.random.default_rng(seed)
+    starts = np.concatenate([[0], np.cumsum(sizes)])
+    cols, lens = [], []
+    for s, m in enumerate(sizes):
+        r = np.arange(starts[s], starts[s + 1])[:, None]
+        c = rng.integers(starts[s - 1], starts[s], (m, width)) if s else np.zeros((m, 0), np.int64)
+        cols.append(np.concatenate([c, r], 1).ravel())
+        lens.append(np.full(m, c.shape[1] + 1))
+    rp = np.concatenate([[0], np.cumsum(np.concatenate(lens))]).astype(np.int32)
+    val = rng.uniform(-1, 1, rp[-1]) / width
+    val[rp[1:] - 1] = rng.uniform(1, 2, len(rp) - 1)
+    return rp, np.concatenate(cols).astype(np.int32), val.astype(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("width", [1, 3, 5, 23])
+@pytest.mark.parametrize("sizes", [[8188, 8189, 8192, 8193] * 5, [20000, 8500, 300, 9001, 16390] * 4])
+def test_levels_wider_than_the_ring(vt, width, sizes):
+    """Swept in one run, such a level writes some slots of the ring twice."""
+    rp, col, val = wide_levels(sizes, width, width, vt)
+    b = np.random.default_rng(width).uniform(-1, 1, len(rp) - 1).astype(vt)
+    smax, kern, x = _kernel("SPTRSV", rp, col, val, b)
+    kern.set_level_merge(1 << 20)
+    kern.run()
+    assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
+    first = x.copy()
+    for _ in range(10):
+        kern.run()
+        np.testing.assert_array_equal(x, first)
+    smax.close()
+
+
 @pytest.mark.parametrize("vt", [np.float64, np.float32])
 @pytest.mark.parametrize("count,most", [(3, 900), (170, 60)])
 def test_batches(vt, count, most):
