@@ -66,6 +66,8 @@ constexpr int kRecChunks = 32;             // chunks of a record, at most
 // the waits' default limit, since the threads of a run wait while one of them
 // goes through a row of a million entries.
 constexpr long long kLevelTime = 1 << 26;
+// Arrivals of a phase that an mbarrier counts, one of them the test's that never comes.
+constexpr int kMaxArrivals = (1 << 20) - 2;
 // An arrived copy takes microseconds; a CTA does not end before its own have.
 constexpr long long kDrainNs = 2000000000ll;
 
@@ -1111,6 +1113,7 @@ bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *v
         for (int c = c_run, in_level = 0; c < c_end; ++c) {
             ++in_level;
             if (c + 1 < c_end && ch[c + 1].level == ch[c].level) continue;
+            if (in_level > kMaxArrivals / (T / 32)) return false;  // tens of millions of rows: the plain kernels
             run.level_chunks = std::max(run.level_chunks, in_level);
             ch[c].lev_arrive = in_level;  // made good below
             in_level = 0;

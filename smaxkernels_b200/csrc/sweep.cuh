@@ -80,7 +80,8 @@ struct SweepStep {
 // sweep steps.  div: divide by the diagonal instead of multiplying by its
 // reciprocal.  batch: the runs are independent matrices (sweep_solve_batch).  Returns false when the
 // padding would make the pack more than about three times the off-diagonal
-// entries, or a level takes so long that others' waits for it could give up.
+// entries, or a level takes so long that others' waits for it could give up, or
+// has more chunks than an mbarrier counts arrivals.
 // Synchronises.
 bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *val, const void *D, int vbytes,
                       int64_t n, const int *order, const std::vector<int> &src_begin, const std::vector<int> &count,

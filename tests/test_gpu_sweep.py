@@ -296,3 +296,20 @@ def test_a_wait_that_runs_out_is_an_error_and_recoverable(kind, k, mode, most):
     B = b.reshape(n, k)
     ref = np.stack([O.sptrsv(rp, col, val, np.ascontiguousarray(B[:, v])) for v in range(k)], 1)
     assert normwise(x.reshape(n, k), ref) <= tol(np.float64)
+
+
+def test_batch_of_a_level_with_more_chunks_than_a_barrier_counts():
+    """One diagonal matrix of 2^18 chunks of 256 rows and a little more, and a small one."""
+    import torch
+    from smaxkernels_b200.interface import FloatType, TriangularBatch
+    n = (1 << 26) + 3000
+    d = (np.arange(n) % 7 + 1).astype(np.float32)
+    small = level_matrix([3, 5], 2, 0, np.float32)
+    tb = TriangularBatch([(np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), d), small], FloatType.FLOAT32)
+    b = torch.ones(n + 8, dtype=torch.float32, device="cuda")
+    x = torch.zeros_like(b)
+    tb.solve(b, x)
+    tb.sync()
+    assert torch.equal(x[:n], 1 / torch.from_numpy(d).cuda())
+    assert normwise(x[n:].cpu().numpy(), O.sptrsv(*small, np.ones(8, np.float32))) <= tol(np.float32)
+    tb.close()
