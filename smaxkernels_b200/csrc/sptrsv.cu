@@ -203,7 +203,7 @@ void TriPlan::assign_reverse(const TriPlan &src, cudaStream_t st) {
 void TriPlan::finish(cudaStream_t) {
     graph_valid = false;
     pack_ok = false;
-    pack_unfit = false;
+    pack_refused.clear();
     pack = SweepPack();
     sf_ok = false;
     sf_unfit = false;
@@ -212,7 +212,7 @@ void TriPlan::finish(cudaStream_t) {
 
 bool TriPlan::ensure_pack(const int *rp, const int *ci, const void *val, const void *D, int vbytes, int merge_rows,
                           uint64_t tag, cudaStream_t st, int64_t k) {
-    if (pack_unfit) return false;  // a property of the pattern and the level sets
+    if (pack_unfit(merge_rows, k)) return false;
     if (!pack_is(val, D, vbytes, merge_rows, pack_tag, k)) {
         if (scheduled_k != 1 || scheduled_merge != merge_rows) schedule(1, merge_rows);
         const int L = n_levels();
@@ -232,7 +232,7 @@ bool TriPlan::ensure_pack(const int *rp, const int *ci, const void *val, const v
         const bool ok = build_sweep_pack(pack, rp, ci, val, D, vbytes, n_rows, has_order ? order.as<int>() : nullptr,
                                          src_begin, count, sweep, k > 1, false, st);
         if (!ok) {
-            pack_unfit = true;
+            pack_refused.push_back({merge_rows, k > 1});
             return false;
         }
         pack_ok = true;
@@ -401,7 +401,7 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
     if (p.n_rows == 0) return;
     // the pack is built outside the capture (it synchronises); a rebuild drops the graph
     bool packed = false;
-    if (k == 1 || sweep_suits(p)) {
+    if (k == 1 || sweep_suits(p, merge_rows)) {
         try {
             packed = p.ensure_pack(a.rp(), a.ci(), a.val.p, D, sizeof(VT), merge_rows, tag, caller, k);
         } catch (const Error &e) {
@@ -478,14 +478,14 @@ void TriPlan::release_graph() {
 
 TriPlan::~TriPlan() { release_graph(); }
 
-bool sweep_suits(const TriPlan &p) {
+bool sweep_suits(const TriPlan &p, int merge_rows) {
     const int64_t L = p.n_levels();
-    return L > 0 && !p.pack_unfit && p.n_rows <= L * 2048;
+    return L > 0 && !p.pack_unfit(merge_rows, 2) && p.n_rows <= L * 2048;
 }
 
-bool syncfree_suits(const TriPlan &p, int64_t k) {
+bool syncfree_suits(const TriPlan &p, int64_t k, int merge_rows) {
     const int64_t L = p.n_levels();
-    if (L <= 0 || (k > 1 && sweep_suits(p))) return false;
+    if (L <= 0 || (k > 1 && sweep_suits(p, merge_rows))) return false;
     if (k == 1) return p.n_rows >= (1 << 17) && p.n_rows >= L * 32768;
     return p.n_rows >= (1 << 16) && L >= 64 && p.n_rows <= L * 16384;
 }

@@ -1,6 +1,8 @@
 // sptrsv.cuh -- level-scheduled triangular solves (sptrsv.cu).
 #pragma once
 
+#include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "levelpack.cuh"
@@ -53,7 +55,14 @@ struct TriPlan {
     // level-ordered pack (sweep.cu), built for the value arrays, their version
     // tag, the merge threshold and one or several right-hand sides below
     SweepPack pack;
-    bool pack_ok = false, pack_unfit = false;
+    bool pack_ok = false;
+    // merge thresholds (and one or several right-hand sides) whose pack was
+    // refused: the levels swept in runs, and so the limits on a run, are theirs
+    std::vector<std::pair<int, bool>> pack_refused;
+    bool pack_unfit(int merge_rows, int64_t k) const {
+        return std::find(pack_refused.begin(), pack_refused.end(), std::make_pair(merge_rows, k > 1)) !=
+               pack_refused.end();
+    }
     const void *pack_key[2] = {nullptr, nullptr};
     uint64_t pack_tag = ~0ull;
     int pack_merge = -1, pack_vbytes = 0;
@@ -115,8 +124,8 @@ template <typename VT>
 void tri_solve_raw(TriPlan &p, const int *rp, const int *ci, const VT *val, const VT *D, const VT *B, VT *X,
                    int64_t k, bool row_major, int64_t ld, int merge_rows, uint64_t tag, cudaStream_t st);
 // Whether blocks of k > 1 right-hand sides run as sweeps of the pack, one CTA
-// each: levels of at most 2048 rows on average.
-bool sweep_suits(const TriPlan &p);
+// each: levels of at most 2048 rows on average, and a pack not yet refused.
+bool sweep_suits(const TriPlan &p, int merge_rows);
 // The sync-free solve of one right-hand side (pack_solve_syncfree).  Returns
 // false, launching nothing, when it does not apply: the matrix does not pack,
 // an entry reads a row not solved before it, or B and X overlap.
@@ -125,7 +134,7 @@ bool sweep_suits(const TriPlan &p);
 // average (few wide levels, whose launches the sync-free solve saves).  k > 1:
 // at least 2^16 rows in 64 levels or more of at most 16384 rows on average
 // (many narrow levels, launch-bound as level launches).
-bool syncfree_suits(const TriPlan &p, int64_t k = 1);
+bool syncfree_suits(const TriPlan &p, int64_t k, int merge_rows);
 // k > 1 runs the row kernel (solve_syncfree_rows), in either block layout.
 template <typename VT>
 bool tri_solve_syncfree(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *X, uint64_t tag, DevBuf &ctl,

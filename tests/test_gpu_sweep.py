@@ -313,3 +313,37 @@ def test_batch_of_a_level_with_more_chunks_than_a_barrier_counts():
     assert torch.equal(x[:n], 1 / torch.from_numpy(d).cuda())
     assert normwise(x[n:].cpu().numpy(), O.sptrsv(*small, np.ones(8, np.float32))) <= tol(np.float32)
     tb.close()
+
+
+def test_a_refused_merge_threshold_closes_no_other():
+    """A level of 5200 rows of up to 43500 entries is too much for one run: the
+    plain kernels solve with the threshold that would sweep it, and the pack, which
+    multiplies by 1/D where they divide, with one that leaves it to a grid."""
+    sources, m, tail = 45000, 5200, 2000
+    rng = np.random.default_rng(14)
+    lens = np.concatenate([[0, 0, 0], np.ones(sources), np.full(m, 14500), np.ones(tail)]).astype(np.int64)
+    lens[3 + sources] = 43500
+    n = len(lens)
+    rp = np.concatenate([[0], np.cumsum(lens + 1)]).astype(np.int32)
+    col = np.empty(rp[-1], np.int32)
+    col[rp[1:] - 1] = np.arange(n)
+    off = np.ones(len(col), bool)
+    off[rp[1:] - 1] = False
+    wide = np.arange(rp[3 + sources], rp[3 + sources + m])
+    col[rp[3]:rp[3 + sources]][::2] = rng.integers(0, 3, sources)
+    w = wide[off[wide]]
+    col[w] = 3 + (np.arange(len(w)) * 7 + np.arange(len(w)) // sources) % sources
+    t0 = 3 + sources + m
+    col[rp[t0]:][::2] = np.arange(t0 - 1, n - 1)
+    val = rng.uniform(-1, 1, len(col)).astype(np.float32) / 1000
+    val[rp[1:] - 1] = rng.uniform(1, 2, n)
+    b = rng.uniform(-1, 1, n).astype(np.float32)
+    fresh = _solve("SPTRSV", rp, col, val, b)
+    smax, kern, x = _kernel("SPTRSV", rp, col, val, b)
+    kern.set_level_merge(1 << 20)
+    kern.run()
+    assert normwise(x, fresh) <= tol(np.float32) and not np.array_equal(x, fresh)
+    kern.set_level_merge(4096)
+    kern.run()
+    np.testing.assert_array_equal(x, fresh)
+    smax.close()
