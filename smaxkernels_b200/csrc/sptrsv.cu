@@ -246,9 +246,10 @@ bool TriPlan::ensure_pack(const int *rp, const int *ci, const void *val, const v
         refill_sweep_pack(pack, rp, val, D, st);
         pack_tag = tag;
     }
-    const void *before = pack.bp.p;
+    const void *before[2] = {pack.bp.p, pack.xp.p};
+    const int vectors = pack.vectors;
     sweep_reserve(pack, k);
-    if (pack.bp.p != before) release_graph();
+    if (pack.bp.p != before[0] || pack.xp.p != before[1] || pack.vectors != vectors) release_graph();
     return true;
 }
 
@@ -405,10 +406,12 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
         try {
             packed = p.ensure_pack(a.rp(), a.ci(), a.val.p, D, sizeof(VT), merge_rows, tag, caller, k);
         } catch (const Error &e) {
-            // a block without room for the sweep's workspace runs the level launches
+            // a block without room for the pack, or for the workspace of one vector,
+            // runs the level launches, now and later
             if (k == 1 || e.code != SMAX_ERR_OOM) throw;
             p.pack = SweepPack();
             p.pack_ok = false;
+            p.pack_refused.push_back({merge_rows, true});
             p.release_graph();
         }
     }

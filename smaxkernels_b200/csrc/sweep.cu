@@ -1203,11 +1203,21 @@ void sweep_reserve(SweepPack &pk, int64_t k) {
     // right-hand sides solved at a time: one CTA each and one CTA per SM, and
     // at most 4 GiB of workspace
     const int64_t each = 2ll * pk.vbytes * std::max<int64_t>(1, pk.npos);
-    k = std::max<int64_t>(1, std::min<int64_t>({k, sm_count(), (4ll << 30) / each}));
+    k = std::max<int64_t>(1, std::min<int64_t>({k, sm_count(), (4ll << 30) / each, pk.most_vectors}));
     if (k <= pk.vectors) return;
     pk.vectors = 0;
-    pk.bp.ensure((size_t)(each / 2 * k));
-    pk.xp.ensure((size_t)(each / 2 * k));
+    for (;; k = (k + 1) / 2) {
+        try {
+            pk.bp.ensure((size_t)(each / 2 * k));
+            pk.xp.ensure((size_t)(each / 2 * k));
+            break;
+        } catch (const Error &e) {
+            if (k == 1 || e.code != SMAX_ERR_OOM) throw;
+            pk.bp.release();
+            pk.xp.release();
+            pk.most_vectors = (int)((k + 1) / 2);
+        }
+    }
     pk.vectors = (int)k;
 }
 

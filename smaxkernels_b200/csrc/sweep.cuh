@@ -59,6 +59,7 @@ struct SweepPack {
     DevBuf blob, recs, drun;
     DevBuf bp, xp;  // VT[vectors][npos]: right-hand sides and solutions in position order
     int vectors = 0;  // right-hand sides solved at a time
+    int most_vectors = 1 << 30;  // as many as there was memory for
     bool needs_x_init = false;  // some entry reads a solution not computed before it
 };
 
@@ -91,7 +92,8 @@ bool build_sweep_pack(SweepPack &pk, const int *rp, const int *ci, const void *v
 void refill_sweep_pack(SweepPack &pk, const int *rp, const void *val, const void *D, cudaStream_t st);
 
 // Workspace for solves of up to k right-hand sides (allocates: call outside
-// stream capture).  Solves take as many at a time as it holds.
+// stream capture).  Solves take as many at a time as it holds: half as many, and
+// so on, if there is no memory for k.
 void sweep_reserve(SweepPack &pk, int64_t k);
 
 // Solves k right-hand sides, element (r, v) of B and X at r * rs + v * vs.

@@ -159,3 +159,56 @@ def test_injection_disarms_itself_and_can_be_cleared():
     assert normwise(result(), ref) <= 1e-12
     smax.close()
     assert _lib().lib.smax_test_fail_device_alloc(-1) == _lib().ERR_BAD_ARG
+
+
+def test_a_block_solve_without_room_for_its_workspace_rebuilds_nothing():
+    """Each allocation of the first solve of a block fails once: those before the
+    sweep's are errors, the sweep's leave a solve that is bit for bit the level
+    launches' and that later solves repeat without an allocation."""
+    from smaxkernels_b200 import FloatType, Interface, IntType, KernelType, PlatformType, SmaxError
+    import torch
+    rp, col, val = rand_crs(2500, 8, 98, lower=True)
+    n, kk = len(rp) - 1, 12
+    b = torch.from_numpy(np.random.default_rng(99).uniform(-1, 1, n * kk)).cuda()
+    MERGED = 2
+
+    def solver(mode):
+        smax = Interface()
+        smax.register_kernel("k", KernelType.SPTRSM, PlatformType.CUDA, IntType.INT32, FloatType.FLOAT64)
+        k = smax.kernel("k")
+        k.set_solve_mode(mode)
+        k.set_vec_row_major(True)
+        x = torch.zeros_like(b)
+        k.register_A(n, n, len(col), col.copy(), rp, val.copy())
+        k.register_B(n, kk, x)
+        k.register_C(n, kk, b)
+        k.initialize()
+        return smax, k, x
+
+    smax, k, ref = solver(MERGED)
+    k.apply()
+    k.sync()
+    smax.close()
+    swept = 0
+    for nth in range(1, 100):
+        smax, k, x = solver(0)
+        _arm(nth)
+        try:
+            k.apply()
+            k.sync()
+        except SmaxError as e:
+            assert e.code == _lib().ERR_OOM
+            _arm(0)
+            smax.close()
+            continue
+        _arm(0)
+        swept += 1
+        x.zero_()
+        for _ in range(2):
+            c0 = _count()
+            k.apply()
+            k.sync()
+            assert _count() == c0, nth
+        assert torch.equal(x, ref), nth
+        smax.close()
+    assert swept > 3
