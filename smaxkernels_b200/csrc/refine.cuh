@@ -17,7 +17,7 @@ struct RefineState {
     const void *gkey[2] = {nullptr, nullptr};
     int g_steps = -1, g_merge = -1;
     uint64_t g_serial = ~0ull, g_aver = ~0ull;  // level plan and A upload the graph was captured for
-    const void *g_pack = nullptr;                // sweep pack the graph reads
+    uint64_t g_pack = ~0ull;                     // sweep pack the graph reads
     SweepWait g_wait;                            // and how long its waits last
     int steps_done = 0;
     double last_rel = 0.0;          // max|d| / max|x| of the last correction

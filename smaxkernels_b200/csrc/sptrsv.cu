@@ -228,6 +228,7 @@ bool TriPlan::ensure_pack(const int *rp, const int *ci, const void *val, const v
             sweep.push_back(SweepStep{s.sweep_first, s.sweep_count, s.kind});
         }
         release_graph();
+        ++pack_serial;
         pack_ok = false;
         const bool ok = build_sweep_pack(pack, rp, ci, val, D, vbytes, n_rows, has_order ? order.as<int>() : nullptr,
                                          src_begin, count, sweep, k > 1, false, st);
@@ -249,7 +250,10 @@ bool TriPlan::ensure_pack(const int *rp, const int *ci, const void *val, const v
     const void *before[2] = {pack.bp.p, pack.xp.p};
     const int vectors = pack.vectors;
     sweep_reserve(pack, k);
-    if (pack.bp.p != before[0] || pack.xp.p != before[1] || pack.vectors != vectors) release_graph();
+    if (pack.bp.p != before[0] || pack.xp.p != before[1] || pack.vectors != vectors) {
+        release_graph();
+        ++pack_serial;
+    }
     return true;
 }
 

@@ -65,6 +65,7 @@ struct TriPlan {
     }
     const void *pack_key[2] = {nullptr, nullptr};
     uint64_t pack_tag = ~0ull;
+    uint64_t pack_serial = 0;  // bumped whenever the pack or its workspace moves
     int pack_merge = -1, pack_vbytes = 0;
     DevStatus *status = nullptr;  // where a sweep reports a wait that gave up
     SweepWait wait;               // how long its waits last

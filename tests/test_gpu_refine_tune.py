@@ -167,3 +167,19 @@ def test_tune_spmv_format():
     assert 0 < c["seconds"] <= c["crs_seconds"]
     if c["format"] == 1:
         assert c["C"] in (8, 16, 32, 64)
+
+
+def test_refine_after_solves_in_between():
+    """The plan keeps one pack: FP64 solves and other merge thresholds in between
+    replace it, and the captured refinement follows."""
+    rp, col, val = _lower_laplace(90)
+    b = np.random.default_rng(5).uniform(-1, 1, len(rp) - 1)
+    ref = O.sptrsv(rp, col, val, b)
+    smax, k, x = _tri_kernel(rp, col, val, b)
+    for steps, merge in [(2, 4096), (0, 4096), (2, 4096), (2, 40), (2, 4096), (0, 20), (2, 4096), (2, 4096)]:
+        k.set_refine(steps)
+        k.set_level_merge(merge)
+        x[:] = 0
+        k.run()
+        assert normwise(x, ref) <= 1e-12, (steps, merge)
+    smax.close()
