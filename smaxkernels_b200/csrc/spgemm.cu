@@ -47,6 +47,9 @@ constexpr int kSmallWarps = 4;                 // warps per CTA: 16 teams, 1.8 K
 constexpr int kWarpBins = 5;
 __host__ __device__ constexpr int warp_slots(int b) { return 512 << b; }
 __host__ __device__ constexpr int warp_products(int b) { return b == 0 ? 256 : warp_slots(b) * 3 / 4; }
+template <typename VT> constexpr size_t warp_table_bytes(int b) {
+    return (size_t)warp_slots(b) * (sizeof(VT) + sizeof(int)) + sizeof(unsigned short) * warp_products(b);
+}
 constexpr int kCtaThreads = 512;               // CTA of the global-table path
 constexpr int kMergeLists = 8;                 // merge path: at most this many entries in the row of A
 constexpr int kBinGlobal = 1 + kWarpBins, kBinMerge = kBinGlobal + 1;
@@ -799,9 +802,11 @@ void spgemm(const DevCRS &A, const DevCRS &B, DevCRS &C, SpgemmWork &w, SpgemmTi
     for (int b = kWarpBins - 1; b >= 0; --b) {  // the longest rows first
         const int nw = h.counts[1 + b];
         if (nw == 0) continue;
-        const size_t sm = (size_t)warp_slots(b) * (sizeof(VT) + sizeof(int)) + sizeof(unsigned short) * warp_products(b);
-        // set on every call: the attribute belongs to the current device
-        SMAX_CUDA(cudaFuncSetAttribute(gustavson_warp<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        const size_t sm = warp_table_bytes<VT>(b);
+        // set on every call: the attribute belongs to the current device; always for the largest
+        // bin: it is one for all threads, and another's launch may come between this and the launch below
+        SMAX_CUDA(cudaFuncSetAttribute(gustavson_warp<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)warp_table_bytes<VT>(kWarpBins - 1)));
         // as many one-warp CTAs as an SM's shared memory holds (1 KB of it is reserved per CTA), at most 32
         const int per_sm = (int)std::min<size_t>(32, (size_t)227 * 1024 / (sm + 1024));
         const unsigned grid = (unsigned)std::min<int64_t>(nw, (int64_t)per_sm * sm_count());

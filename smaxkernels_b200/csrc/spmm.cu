@@ -149,6 +149,9 @@ template <typename VT> __host__ __device__ constexpr int stage_bytes(int rw, int
     return rw * (ch + kStagePad) * (int)(sizeof(VT) + sizeof(int));
 }
 
+// the most that the two stages of a CTA's warps take: launch_groups gives them 256 entries at most, or 32 rows of 4
+template <typename VT> constexpr int stages_most(int warps) { return warps * 2 * stage_bytes<VT>(32, 8); }
+
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async4(unsigned dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
@@ -493,8 +496,10 @@ void launch_groups(const DevCRS &a, const SpmmPlan &p, int64_t k, int64_t ldx, c
         }
         auto go = [&](auto kern, int warps) {
             const size_t sm = (size_t)warps * 2 * stage_bytes<VT>(rw, 1 << shift);
-            // set on every call: the attribute belongs to the current device
-            SMAX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            // set on every call: the attribute belongs to the current device; always to the most
+            // that a call can need: it is one for all threads, and another's launch
+            // may come between this and the launch below
+            SMAX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, stages_most<VT>(warps)));
             kern<<<p.grid, warps * 32, sm, st>>>(a.rp(), a.ci(), a.val.template as<VT>(), p.ranges.as<int64_t>(), G,
                                                  shift, nvec, kcols, (int)ldx, X + v0 * VEC,
                                                  COL ? Y + v0 * VEC * ldy : Y + v0 * VEC, ldy);
