@@ -185,7 +185,7 @@ void spmm_upload(smax_kernel_s *k) {
     validate_crs(k->dA, dstatus(k), k->stream);
     read_status(k);
     k->crs_stream = CrsStreamPlan();
-    k->spmm_plan.build(k->dA, k->stream);
+    k->spmm_plan.build(k->dA, !k->f_row_major, k->stream);
     if (!k->f_row_major) k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, k->stream);
 }
 
@@ -198,7 +198,8 @@ template <typename VT> void spmm_apply_t(smax_kernel_s *k, const VT *X, VT *Y) {
         // of both X and Y (src/kernels/spmm/spmm_cpu/spmm_cpu_crs_impl.hpp:29,44)
         const int64_t ld = k->dA.n_rows;
         if (kk > 1 && !spmm_by_columns(k->dA, kk, k->crs_stream.longest) &&
-            (int64_t)k->spmm_plan.work.bytes >= spmm_col_major_work(k->dA.n_cols, kk, k->vbytes)) {
+            (int64_t)k->spmm_plan.work.bytes >= spmm_col_major_work(k->dA.n_cols, kk, k->vbytes) &&
+            (int64_t)k->spmm_plan.part.bytes >= k->spmm_plan.part_bytes(kk)) {
             crs_spmm_col_major<VT>(k->dA, kk, X, Y, ld, k->spmm_plan.work.as<VT>(), k->stream, k->spmm_plan);
             return;
         }
@@ -474,13 +475,15 @@ void do_initialize(smax_kernel_s *k, bool wait = true) {
         ++k->a_version;
         ++k->vals_version;
     }
-    // column-major SpMM: the workspace of X's row-major copy, allocated here so
-    // that applies allocate nothing; without room for it they run one product
-    // per column
+    // column-major SpMM: the workspaces of X's row-major copy and of long rows'
+    // pieces, allocated here so that applies allocate nothing; without room for
+    // them they run one product per column
     if (k->ktype == SMAX_KERNEL_SPMM && !k->f_row_major && k->B.n_cols > 1 &&
         !spmm_by_columns(k->dA, (int64_t)k->B.n_cols, k->crs_stream.longest)) {
+        const int64_t kk = (int64_t)k->B.n_cols;
         try {
-            k->spmm_plan.work.ensure((size_t)spmm_col_major_work(k->dA.n_cols, (int64_t)k->B.n_cols, k->vbytes));
+            k->spmm_plan.part.ensure((size_t)k->spmm_plan.part_bytes(kk));
+            k->spmm_plan.work.ensure((size_t)spmm_col_major_work(k->dA.n_cols, kk, k->vbytes));
         } catch (const Error &e) {
             if (e.code != SMAX_ERR_OOM) throw;
         }

@@ -19,7 +19,13 @@
 //
 // Column-major blocks are transposed into a row-major workspace (one pass over
 // X) and run the group kernel, which writes Y column-major: A is read once
-// and not once per vector.
+// and not once per vector.  The products per vector that it replaces spread a long
+// row over the chip and add it up in slices.  So a row far longer than the
+// others is not left to one group, which takes 0.1 us an entry, but cut into
+// pieces, a warp each (spmm_piece_kernel, spmm_combine_kernel), and four products
+// at a time are added to a sum that loses less: 64 bits wide for FP32,
+// compensated for FP64.  (A row-major block is added up in stored order, by
+// whichever kernel.)
 //
 // Measured before and after (before: the grid kernel, a warp per row for
 // widths that are no power of two, k SpMVs for column-major blocks):
@@ -31,11 +37,17 @@
 #include "spmv_formats.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <type_traits>
+
+#include <cub/device/device_scan.cuh>
 
 namespace smax {
 
 namespace {
+
+constexpr int kPiece = 128, kBigPiece = 512;  // entries of a piece, and of one of a row of over kPiece * 1024
+__host__ __device__ constexpr int piece_size(int len) { return len > kPiece * 1024 ? kBigPiece : kPiece; }
 
 template <typename VT> struct V16;
 template <> struct V16<double> { using T = double2; static constexpr int N = 2; };
@@ -194,10 +206,29 @@ template <typename VT> __device__ __forceinline__ void read4(const VT *p, VT (&v
     }
 }
 
+// The sums of a column-major block: 64 bits for FP32; for FP64, the rounding errors
+// of the additions beside the sum.
+struct Wide {
+    double sum;
+    __device__ __forceinline__ void add(float x) { sum += x; }
+    __device__ __forceinline__ float value() const { return (float)sum; }
+};
+struct Compensated {
+    double sum, err;
+    __device__ __forceinline__ void add(double x) {
+        const double s = sum + x, b = s - sum;
+        err += (sum - (s - b)) + (x - b);
+        sum = s;
+    }
+    // (infinities and NaN are the sum's: what stands beside them is no error)
+    __device__ __forceinline__ double value() const { return isfinite(err) ? sum + err : sum; }
+};
+
 // U staged entries: their rows of X are all loaded before the first is used.
-template <typename VT, int VB, int NV, int U>
+// AT: VT itself, or one of the sums above, which takes the U products together.
+template <typename VT, typename AT, int VB, int NV, int U>
 __device__ __forceinline__ void take(const int *sc, const VT *sv, const VT *const (&xl)[NV], int ldx,
-                                     VT (&acc)[NV][XVec<VT, VB>::N]) {
+                                     AT (&acc)[NV][XVec<VT, VB>::N]) {
     XVec<VT, VB> x[U][NV];
     int c[U];
     if constexpr (U % 4 == 0) {
@@ -227,26 +258,40 @@ __device__ __forceinline__ void take(const int *sc, const VT *sv, const VT *cons
 #pragma unroll
         for (int u = 0; u < U; ++u) v[u] = sv[u];
     }
+    if constexpr (std::is_same<VT, AT>::value) {
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int m = 0; m < NV; ++m)
+#pragma unroll
+                for (int i = 0; i < XVec<VT, VB>::N; ++i) acc[m][i] += v[u] * x[u][m].v[i];
+    } else {
 #pragma unroll
         for (int m = 0; m < NV; ++m)
 #pragma unroll
-            for (int i = 0; i < XVec<VT, VB>::N; ++i) acc[m][i] += v[u] * x[u][m].v[i];
+            for (int i = 0; i < XVec<VT, VB>::N; ++i) {
+                VT sum = v[0] * x[0][m].v[i];
+#pragma unroll
+                for (int u = 1; u < U; ++u) sum += v[u] * x[u][m].v[i];
+                acc[m][i].add(sum);
+            }
+    }
 }
 
 // Columns [0, kcols) of one panel: nvec vectors of a row of X (row stride ldx
 // values).  COL: Y is column-major, element (row, v) at row + v * ldy, else
 // row-major with row stride ldy.
 // REG: no row has more than CH entries; rows are then dealt out in turn and a
-// row is one chunk.  Otherwise the groups take rows from a shared counter.
+// row is one chunk.  Otherwise the groups take rows from a shared counter, and
+// leave out those of more than `limit` entries.
 template <typename VT, int VB, int NV, bool COL, bool REG>
 __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
     spmm_group_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col, const VT *__restrict__ val,
                       const int64_t *__restrict__ ranges, int G, int ch_shift, int nvec, int kcols, int ldx,
-                      const VT *__restrict__ X, VT *__restrict__ Y, int64_t ldy) {
+                      const VT *__restrict__ X, VT *__restrict__ Y, int64_t ldy, int limit) {
     using XV = XVec<VT, VB>;
     constexpr int VEC = XV::N;
+    using AT = typename std::conditional<!COL, VT, typename std::conditional<sizeof(VT) == 8, Compensated, Wide>::type>::type;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int next_row;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -282,6 +327,10 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
             if (row < r1) {
                 s = row_ptr[row];
                 e = row_ptr[row + 1];
+                if (COL && e - s > limit) {  // left out: e < s
+                    s = 0;
+                    e = -1;
+                }
             }
         }
     };
@@ -290,7 +339,7 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
         VT *sv = reinterpret_cast<VT *>(reinterpret_cast<unsigned char *>(sv0) + b * stage);
         int *sc = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(sc0) + b * stage);
         if (worker)
-            for (int j = gl; j < CH && at + j < e; j += G) {
+            for (int j = gl; j < CH && j < e - at; j += G) {
                 cp_async4(smem_u32(sc + j), col + at + j);
                 if constexpr (sizeof(VT) == 8) cp_async8(smem_u32(sv + j), val + at + j);
                 else cp_async4(smem_u32(sv + j), val + at + j);
@@ -298,11 +347,11 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
         cp_async_commit();
     };
 
-    VT acc[NV][VEC];
+    AT acc[NV][VEC];
 #pragma unroll
     for (int m = 0; m < NV; ++m)
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) acc[m][i] = VT(0);
+        for (int i = 0; i < VEC; ++i) acc[m][i] = AT{};
 
     // the entries of a staged chunk, n of them, into acc
     auto chunk = [&](int b, int n) {
@@ -312,24 +361,24 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
         // lane, fewer entries at a time, for the same bytes in flight
         constexpr int U = group_unroll(NV);
         int j = 0;
-        for (; j + U <= n; j += U) take<VT, VB, NV, U>(sc + j, sv + j, xl, ldx, acc);
+        for (; j + U <= n; j += U) take<VT, AT, VB, NV, U>(sc + j, sv + j, xl, ldx, acc);
         if constexpr (U > 2)
             if (j + 2 <= n) {
-                take<VT, VB, NV, 2>(sc + j, sv + j, xl, ldx, acc);
+                take<VT, AT, VB, NV, 2>(sc + j, sv + j, xl, ldx, acc);
                 j += 2;
             }
-        if (j < n) take<VT, VB, NV, 1>(sc + j, sv + j, xl, ldx, acc);
+        if (j < n) take<VT, AT, VB, NV, 1>(sc + j, sv + j, xl, ldx, acc);
     };
-    // the finished row to Y, and acc back to zero
-    auto finish = [&](int row) {
+    // the finished row to Y (store: it was not left out), and acc back to zero
+    auto finish = [&](int row, bool store) {
 #pragma unroll
         for (int m = 0; m < NV; ++m) {
             const int off = (m * G + gl) * VEC;
-            if (worker && row < r1 && m * G + gl < nvec) {
+            if (worker && (!COL || store) && row < r1 && m * G + gl < nvec) {
                 if constexpr (COL) {
 #pragma unroll
                     for (int i = 0; i < VEC; ++i)
-                        if (off + i < kcols) __stcs(Y + (int64_t)(off + i) * ldy + row, acc[m][i]);
+                        if (off + i < kcols) __stcs(Y + (int64_t)(off + i) * ldy + row, acc[m][i].value());
                 } else {
                     VT *y = Y + (int64_t)row * ldy + off;
                     if constexpr (VB == 16 && sizeof(VT) == 8)
@@ -344,7 +393,7 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
                 }
             }
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) acc[m][i] = VT(0);
+            for (int i = 0; i < VEC; ++i) acc[m][i] = AT{};
         }
     };
 
@@ -371,7 +420,7 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
             __syncwarp();
             chunk(b, e - s);
             __syncwarp();
-            finish(row);
+            finish(row, true);
             s = s1;
             e = e1;
             s1 = s2;
@@ -394,7 +443,7 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
             if (more) {
                 s += CH;
             } else {
-                finish(row);
+                finish(row, e >= s);
                 row = row1;
                 s = s1;
                 e = e1;
@@ -409,17 +458,142 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
     cp_async_wait<0>();
 }
 
-// ranges[b] = first row r with row_ptr[r] + r >= b * (nnz + n) / grid
-// (nonzeros and rows balanced: a row costs its entries plus its Y write)
-__global__ void row_ranges_kernel(const int *__restrict__ row_ptr, int64_t n, int grid, int64_t *__restrict__ ranges) {
+// One warp per piece of a long row, for up to 32 vectors (a panel, blockIdx.y):
+// a lane per vector and 32 / G entries side by side, four of them in flight a
+// lane; then the lanes of one vector are added up.  part: kq sums a piece.
+// Bound by the gathers of X, as the group kernel is.  10^6 rows of 5 entries, one
+// of 10^6, k = 8 column-major FP64: 112 ms by one group, see spmm_by_columns.
+template <typename VT>
+__global__ void __launch_bounds__(256) spmm_piece_kernel(const int2 *__restrict__ pieces, int64_t n_pieces,
+                                                         const int *__restrict__ col, const VT *__restrict__ val,
+                                                         int64_t nvec, int64_t ldx, const VT *__restrict__ X,
+                                                         int64_t kq, double *__restrict__ part) {
+    using XV = XVec<VT, 16>;
+    constexpr int VEC = XV::N, U = 4;
+    const int lane = threadIdx.x & 31;
+    const int64_t p = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (p >= n_pieces) return;
+    const int2 piece = pieces[p];
+    const int64_t panels = (nvec + 31) / 32;
+    for (int64_t pn = blockIdx.y; pn < panels; pn += gridDim.y) {
+        const int64_t v0 = nvec * pn / panels;
+        const int G = (int)(nvec * (pn + 1) / panels - v0), R = 32 / G;
+        const int slot = lane / G, gl = lane - slot * G;
+        const VT *xl = X + (v0 + gl) * VEC;
+        double acc[VEC];
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) acc[i] = 0;
+        if (slot < R) {
+            // (left counts the entries: an entry's number plus a step may pass 2^31)
+            int left = piece.y - piece.x - slot;
+            const int *cp = col + piece.x + slot;
+            const VT *vp = val + piece.x + slot;
+            for (; left > 0; left -= U * R, cp += U * R, vp += U * R) {
+                int c[U];
+                VT v[U];
+                XV x[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const bool ok = u * R < left;
+                    c[u] = ok ? ld_stream(cp + u * R) : -1;
+                    v[u] = ok ? ld_stream(vp + u * R) : VT(0);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (c[u] >= 0) x[u].load(xl + (int64_t)c[u] * ldx);
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) {
+                    VT sum = VT(0);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (c[u] >= 0) sum += v[u] * x[u].v[i];
+                    acc[i] += sum;
+                }
+            }
+        }
+        int o = 1;
+        while (o < R) o <<= 1;
+        for (o >>= 1; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) {
+                const double other = __shfl_down_sync(0xffffffffu, acc[i], o * G);
+                if (slot < o && slot + o < R) acc[i] += other;
+            }
+        if (slot == 0)
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) part[p * kq + (v0 + gl) * VEC + i] = acc[i];
+    }
+}
+
+// The pieces of a long row (blockIdx.x), added up: W vectors side by side, 256 / W
+// stretches of pieces, those in order.  long_rows: row, first piece, pieces.
+template <typename VT>
+__global__ void __launch_bounds__(256) spmm_combine_kernel(const int4 *__restrict__ long_rows,
+                                                           const double *__restrict__ part, int64_t k, int64_t kq,
+                                                           int W, VT *__restrict__ Y, int64_t ldy) {
+    __shared__ Compensated sums[256];
+    const int4 L = long_rows[blockIdx.x];
+    const int t = threadIdx.x % W, stretch = threadIdx.x / W, S = 256 / W;
+    const int p0 = (int)((int64_t)L.z * stretch / S), p1 = (int)((int64_t)L.z * (stretch + 1) / S);
+    for (int64_t v0 = (int64_t)blockIdx.y * W; v0 < k; v0 += (int64_t)gridDim.y * W) {
+        const int64_t v = v0 + t;
+        Compensated s{0, 0};
+        if (v < k) {
+            const double *q = part + (int64_t)L.y * kq + v;
+#pragma unroll 4
+            for (int p = p0; p < p1; ++p) s.add(q[p * kq]);
+        }
+        sums[threadIdx.x] = s;
+        __syncthreads();
+        if (stretch == 0 && v < k) {
+            for (int i = 1; i < S; ++i) {
+                s.add(sums[i * W + t].sum);
+                s.err += sums[i * W + t].err;
+            }
+            Y[v * ldy + L.x] = (VT)s.value();
+        }
+        __syncthreads();
+    }
+}
+
+// weight[r]: a row's entries (none for one cut into pieces) and its Y write
+__global__ void row_weights_kernel(const int *__restrict__ row_ptr, int64_t n, int limit, int64_t *__restrict__ weight) {
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    const int len = row_ptr[r + 1] - row_ptr[r];
+    weight[r] = 1 + (len > limit ? 0 : len);
+}
+
+// The rows of more than `limit` entries (row, first piece, pieces) and their
+// pieces, rows in any order.  next: rows << 40 | pieces taken so far (2^31 entries are
+// less than 2^24 rows of more than 128).
+__global__ void long_rows_kernel(const int *__restrict__ row_ptr, int64_t n, int limit, unsigned long long *next,
+                                 int4 *__restrict__ long_rows, int2 *__restrict__ pieces) {
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    const int s = row_ptr[r], len = row_ptr[r + 1] - s;
+    if (len <= limit) return;
+    const int size = piece_size(len), m = (len - 1) / size + 1;
+    const unsigned long long at = atomicAdd(next, (1ull << 40) | (unsigned long long)m);
+    const int first = (int)(at & ((1ull << 40) - 1));
+    long_rows[at >> 40] = make_int4((int)r, first, m, 0);
+    for (int i = 0; i < m; ++i)
+        pieces[first + i] = make_int2(s + i * size, i + 1 < m ? s + (i + 1) * size : s + len);
+}
+
+// ranges[b] = first row r with w[r] >= b * w[n] / grid, where w[r] is what the rows
+// before r weigh: their entries and their Y writes, row_ptr[r] + r unless
+// given (without the rows cut into pieces)
+__global__ void row_ranges_kernel(const int *__restrict__ row_ptr, const int64_t *__restrict__ weights, int64_t n,
+                                  int grid, int64_t *__restrict__ ranges) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b > grid) return;
-    const int64_t total = (int64_t)row_ptr[n] + n;
-    const int64_t target = total * b / grid;
+    auto w = [&](int64_t r) { return weights ? (r > 0 ? weights[r - 1] : 0) : (int64_t)row_ptr[r] + r; };
+    const int64_t target = w(n) * b / grid;
     int64_t lo = 0, hi = n;
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
-        if ((int64_t)row_ptr[mid] + mid < target) lo = mid + 1;
+        if (w(mid) < target) lo = mid + 1;
         else hi = mid;
     }
     ranges[b] = b == grid ? n : lo;
@@ -470,6 +644,22 @@ void group_shape(int nvec, int &G, int &NV) {
     }
 }
 
+// the long rows of a column-major Y; X: rows of ldx values, whole vectors
+template <typename VT>
+void launch_pieces(const DevCRS &a, const SpmmPlan &p, int64_t k, int64_t ldx, const VT *X, VT *Y, int64_t ldy,
+                   cudaStream_t st) {
+    const int64_t nvec = ldx / V16<VT>::N;
+    const unsigned panels = (unsigned)std::min<int64_t>((nvec + 31) / 32, 65535);
+    spmm_piece_kernel<VT><<<dim3(ceil_div_u(p.n_pieces, 8), panels), 256, 0, st>>>(
+        p.pieces.as<int2>(), p.n_pieces, a.ci(), a.val.template as<VT>(), nvec, ldx, X, ldx, p.part.as<double>());
+    SMAX_CUDA(cudaGetLastError());
+    int W = 1;
+    while (W < 32 && W < k) W <<= 1;
+    const dim3 grid(p.n_long, (unsigned)std::min<int64_t>((k + W - 1) / W, 65535));
+    spmm_combine_kernel<VT><<<grid, 256, 0, st>>>(p.long_rows.as<int4>(), p.part.as<double>(), k, ldx, W, Y, ldy);
+    SMAX_CUDA(cudaGetLastError());
+}
+
 template <typename VT, int VB, bool COL>
 void launch_groups(const DevCRS &a, const SpmmPlan &p, int64_t k, int64_t ldx, const VT *X, VT *Y, int64_t ldy,
                    cudaStream_t st) {
@@ -502,7 +692,8 @@ void launch_groups(const DevCRS &a, const SpmmPlan &p, int64_t k, int64_t ldx, c
             SMAX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, stages_most<VT>(warps)));
             kern<<<p.grid, warps * 32, sm, st>>>(a.rp(), a.ci(), a.val.template as<VT>(), p.ranges.as<int64_t>(), G,
                                                  shift, nvec, kcols, (int)ldx, X + v0 * VEC,
-                                                 COL ? Y + v0 * VEC * ldy : Y + v0 * VEC, ldy);
+                                                 COL ? Y + v0 * VEC * ldy : Y + v0 * VEC, ldy,
+                                                 p.limit);
             SMAX_CUDA(cudaGetLastError());
         };
         auto pick = [&](auto NVc) {
@@ -534,26 +725,56 @@ __global__ void spmm_row_major_generic(const int *__restrict__ row_ptr, const in
 
 }  // namespace
 
-static __global__ void longest_row_kernel(const int *__restrict__ row_ptr, int64_t n, int *__restrict__ longest) {
+// found[0]: entries of the longest row, [1]: rows of more than `limit`, [2]: their pieces
+static __global__ void longest_row_kernel(const int *__restrict__ row_ptr, int64_t n, int limit,
+                                          int *__restrict__ found) {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int len = r < n ? row_ptr[r + 1] - row_ptr[r] : 0;
+    if (len > limit) {
+        atomicAdd(found + 1, 1);
+        atomicAdd(found + 2, (len - 1) / piece_size(len) + 1);
+    }
     len = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
-    if ((threadIdx.x & 31) == 0 && len > 0) atomicMax(longest, len);
+    if ((threadIdx.x & 31) == 0 && len > 0) atomicMax(found, len);
 }
 
-void SpmmPlan::build(const DevCRS &a, cudaStream_t st) {
-    DevBuf d(sizeof(int));
-    SMAX_CUDA(cudaMemsetAsync(d.p, 0, sizeof(int), st));
-    if (a.n_rows > 0)
-        longest_row_kernel<<<ceil_div_u(a.n_rows, 256), 256, 0, st>>>(a.rp(), a.n_rows, d.as<int>());
-    SMAX_CUDA(cudaMemcpyAsync(&longest, d.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+void SpmmPlan::build(const DevCRS &a, bool col_major, cudaStream_t st) {
+    const int64_t n = a.n_rows;
+    // cut: rows of more than a piece and four times the average
+    limit = !col_major ? INT_MAX : (int)std::min<int64_t>(INT_MAX, std::max<int64_t>(kPiece, n > 0 ? 4 * a.nnz / n : 0));
+    DevBuf d(sizeof(int) * 3);
+    int h[3] = {0, 0, 0};
+    SMAX_CUDA(cudaMemsetAsync(d.p, 0, sizeof(h), st));
+    if (n > 0) longest_row_kernel<<<ceil_div_u(n, 256), 256, 0, st>>>(a.rp(), n, limit, d.as<int>());
+    SMAX_CUDA(cudaMemcpyAsync(h, d.p, sizeof(h), cudaMemcpyDeviceToHost, st));
     SMAX_CUDA(cudaStreamSynchronize(st));
-    regular = (int64_t)longest * a.n_rows <= 2 * a.nnz + 8 * a.n_rows;
+    longest = h[0];
+    n_long = h[1];
+    n_pieces = h[2];
+    regular = (int64_t)longest * n <= 2 * a.nnz + 8 * n;
+    DevBuf weights, tmp, next;
+    if (n_long > 0) {
+        long_rows.ensure(sizeof(int4) * n_long);
+        pieces.ensure(sizeof(int2) * n_pieces);
+        next.alloc(sizeof(unsigned long long));
+        SMAX_CUDA(cudaMemsetAsync(next.p, 0, sizeof(unsigned long long), st));
+        long_rows_kernel<<<ceil_div_u(n, 256), 256, 0, st>>>(a.rp(), n, limit, next.as<unsigned long long>(),
+                                                             long_rows.as<int4>(), pieces.as<int2>());
+        weights.alloc(sizeof(int64_t) * n);
+        int64_t *w = weights.as<int64_t>();
+        row_weights_kernel<<<ceil_div_u(n, 256), 256, 0, st>>>(a.rp(), n, limit, w);
+        SMAX_CUDA(cudaGetLastError());
+        size_t tb = 0;
+        SMAX_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, w, w, n, st));
+        tmp.alloc(tb ? tb : 1);
+        SMAX_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, tb, w, w, n, st));
+    }
     grid = sm_count();
     ranges.ensure(sizeof(int64_t) * (grid + 1));
-    row_ranges_kernel<<<ceil_div_u((uint64_t)grid + 1, 256), 256, 0, st>>>(a.rp(), a.n_rows, grid,
+    row_ranges_kernel<<<ceil_div_u((uint64_t)grid + 1, 256), 256, 0, st>>>(a.rp(), weights.as<int64_t>(), n, grid,
                                                                            ranges.as<int64_t>());
     SMAX_CUDA(cudaGetLastError());
+    if (n_long > 0) SMAX_CUDA(cudaStreamSynchronize(st));  // the temporaries die here
 }
 
 // Whether a row-major product runs on the grid of all rows: rows of nearly
@@ -635,6 +856,7 @@ void crs_spmm_col_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, int64_t 
     to_row_major_kernel<VT><<<dim3(ceil_div_u(a.n_cols, kTrRows), ceil_div_u(kp, 64)), 256, 0, st>>>(
         X, a.n_cols, (int)k, (int)kp, ld, work);
     SMAX_CUDA(cudaGetLastError());
+    if (plan.n_long > 0) launch_pieces<VT>(a, plan, k, kp, work, Y, ld, st);
     launch_groups<VT, 16, true>(a, plan, k, kp, work, Y, ld, st);
 }
 

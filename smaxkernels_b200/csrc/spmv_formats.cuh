@@ -67,8 +67,15 @@ struct SpmmPlan {
     int grid = 0;
     int longest = 0;       // entries of the longest row
     bool regular = false;  // ... at most twice the mean plus 8
+    // column-major blocks: rows of more than `limit` entries, cut into pieces (spmm.cu)
+    int limit = 0, n_long = 0;
+    int64_t n_pieces = 0;
+    DevBuf long_rows;  // int4[n_long]: row, first piece, pieces
+    DevBuf pieces;     // int2[n_pieces]: entries [x, y)
+    DevBuf part;       // double[n_pieces][k rounded up]: their sums
     DevBuf work;    // column-major blocks: X as a row-major block
-    void build(const DevCRS &a, cudaStream_t st);
+    int64_t part_bytes(int64_t k) const { return n_pieces * ((k + 3) / 4 * 4) * (int64_t)sizeof(double); }
+    void build(const DevCRS &a, bool col_major, cudaStream_t st);
 };
 // variant 0: chosen by the matrix and the block's width; 1: a grid of all
 // rows; 2: lane groups going through a range of rows per SM
