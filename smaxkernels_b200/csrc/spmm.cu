@@ -835,11 +835,15 @@ void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStre
 // one in 100 of 32, FP64: k = 3 37 us as products, 52 as a block; k = 8 89 and
 // 70; below 2^17 rows the products' launches cost more (20000 rows, k = 3: 27
 // and 21).  With rows of more than 64 times the average length also k = 8 (of 1
-// entry, one in 1000 of 500: 137 and 173 us): a product spreads a long row over
-// the chip.
+// entry, one in 1000 of 500: 137 and 173 us).  Of longer rows, two vectors
+// where their lengths differ (products and block, lognormal 30000 rows FP64 28 and 47 us, 300000
+// 66 and 141; 2^19 rows of 8, one in 100 of 64: 60 and 89; 20000 of these 27 and
+// 23) and three where some are far longer (lognormal 30000 FP32 37 and 47, 300000 92 and 105).
 bool spmm_by_columns(const DevCRS &a, int64_t k, int64_t longest) {
     const bool skewed = longest * a.n_rows > 64 * a.nnz;
-    return a.nnz < 4 * a.n_rows && ((k < 8 && a.n_rows >= (1 << 17)) || (k <= 8 && skewed));
+    const bool uneven = longest * a.n_rows > 2 * a.nnz + 8 * a.n_rows;
+    if (a.nnz < 4 * a.n_rows) return (k < 8 && a.n_rows >= (1 << 17)) || (k <= 8 && skewed);
+    return a.nnz >= (1 << 18) && ((k == 2 && uneven) || (k == 3 && longest * a.n_rows > 32 * a.nnz));
 }
 
 int64_t spmm_col_major_work(int64_t n_cols, int64_t k, int vbytes) {

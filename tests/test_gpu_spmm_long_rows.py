@@ -84,3 +84,17 @@ def test_sums_no_worse_than_the_products_per_column(vt, lens):
     ref = np.stack([np.add.reduceat(val.astype(np.longdouble) * xl[v][col], rp[:-1]) for v in range(k)])
     block, products = (np.sqrt(np.mean((A - ref).astype(np.float64) ** 2)) for A in (Y, P))
     assert block <= products, (block, products)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("k", [2, 3, 4])
+@pytest.mark.parametrize("n,most", [(32767, 90), (32768, 90), (32768, 600), (50000, 8)])
+def test_few_vectors_where_the_products_begin(vt, k, n, most):
+    """2^18 entries, less and more, rows uneven, far longer or all equal."""
+    lens = np.full(n, 8)
+    lens[0] = most
+    lens[1:1 + most] -= most > 8
+    rp, col, val = _matrix(lens, k, vt)
+    X = np.random.default_rng(9).uniform(-1, 1, n * k).astype(vt)
+    Y = gpu_spmm(rp, col, val, X, k, False)
+    assert normwise(Y, O.spmm(rp, col, val, X, k, row_major=False)) <= tol(vt)
