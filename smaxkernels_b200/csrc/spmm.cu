@@ -673,9 +673,14 @@ void launch_groups(const DevCRS &a, const SpmmPlan &p, int64_t k, int64_t ldx, c
         int G = 1, NV = 1;
         group_shape(nvec, G, NV);
         const int rw = 32 / G;
-        // a chunk holds a row of mean length, a warp's stage at most 256 entries
+        // a chunk holds a row of mean length, and of far longer rows, which are a
+        // chain of chunks, a sixteenth; a warp's stage at most 256 entries (rows of 1
+        // entry, one in 1000 of 500, 20000 rows, k = 3 FP32: 88 us with chunks of 4, 56
+        // with 16; lognormal 600000 rows, k = 20 FP32: 195 with 16, 182 with 32)
         int shift = 2;
-        while (shift < 5 && (rw << (shift + 1)) <= 256 && (int64_t)a.n_rows << shift < a.nnz) ++shift;
+        while (shift < 5 && (rw << (shift + 1)) <= 256 &&
+               ((int64_t)a.n_rows << shift < a.nnz || p.longest > 16 << shift))
+            ++shift;
         // rows of nearly equal length: a chunk that holds the longest
         bool reg = false;
         if (p.regular) {
@@ -777,7 +782,7 @@ void SpmmPlan::build(const DevCRS &a, bool col_major, cudaStream_t st) {
     if (n_long > 0) SMAX_CUDA(cudaStreamSynchronize(st));  // the temporaries die here
 }
 
-// Whether a row-major product runs on the grid of all rows: rows of nearly
+// Whether a row-major product runs on the grid of all rows.  Rows of nearly
 // equal length, a power of two of 16-byte vectors, and either a wide block,
 // whose rows of X are more than an SM keeps (27-point 96^3, grid against
 // groups: k = 64 FP64 655 / 801 us, k = 64 FP32 359 / 396, k = 128 FP64 1199 /
@@ -785,14 +790,29 @@ void SpmmPlan::build(const DevCRS &a, bool col_major, cudaStream_t st) {
 // per row (7-point 100^3: k = 16 FP64 134 / 154 us, k = 16 FP32 79 / 83; k = 4
 // FP64 73 / 48), or rows of X of one 16-byte FP64 vector (27-point 96^3, k = 2:
 // 239 / 495 us).  Rows of uneven length take the groups (lognormal 500000,
-// k = 64 FP64: 946 against 1543 us), except in small matrices of few entries,
-// where a CTA's start counts (20000 rows, nine in ten empty, k = 32 FP64: 25 us,
-// the grid 16; of 2 entries, one in 100 of 32: 19.6 and 16.9).
+// k = 64 FP64: 946 against 1543 us), except (grid / groups, us):
+//  * one FP64 vector, if no row is long (2^17 rows of 2, one in 100 of 32: 18 / 23;
+//    2^19 of 8, one in 100 of 64: 55 / 69; but of 3, one in 1000 of 100: 40 / 37) or if
+//    there are many that are not short (lognormal 600000: 300 / 370; 150000: 131 / 109;
+//    2^19 of 10, one in 1000 of 3000: 600 / 528);
+//  * rows of fewer than four entries on average and none long, where the groups'
+//    work per row and a CTA's start count: small matrices whatever the width (20000
+//    rows, nine in ten empty, k = 32 FP64 16 / 26, k = 5 FP32 14 / 20; of 2 entries, one in
+//    100 of 32, k = 20 FP32 14 / 16), wide blocks up to 2^18 rows, and beyond if few
+//    rows are longer than the rest (2^19 of 2, one in 100 of 32, k = 32 FP64 115 / 122;
+//    nine in ten empty 190 / 160); of fewer than 2.5 also narrow ones (2^17 of 2, one in
+//    100 of 32, k = 8 FP64 20 / 24, FP32 20 / 22; 2^19: 40 / 40, 35 / 33).
+// nvec: 16-byte vectors of a row of X, 0 if it is not whole vectors (the grid's
+// kernel for such rows is a warp each).
 static bool grid_suits(const DevCRS &a, const SpmmPlan &p, int64_t nvec, int vbytes) {
-    if (nvec <= 0 || nvec > 128 || (nvec & (nvec - 1))) return false;
-    if (nvec >= 8 && a.nnz < 4 * a.n_rows && a.n_rows < (1 << 17)) return true;
+    const int64_t n = a.n_rows;
+    const bool short_rows = a.nnz < 4 * n && p.longest <= 64;
+    if (nvec <= 0 || nvec > 128 || (nvec & (nvec - 1))) return short_rows && n < (1 << 16);
+    if (nvec == 1 && vbytes == 8) return p.regular || p.longest <= 64 || (n >= (1 << 18) && a.nnz >= 15 * n);
+    if (nvec >= 8 && short_rows && (n < (1 << 18) || p.longest * n > 12 * a.nnz)) return true;
+    if (short_rows && 2 * a.nnz < 5 * n && n >= (1 << 16) && n < (1 << 18)) return true;
     if (!p.regular) return false;
-    return nvec >= 16 || (nvec >= 4 && a.nnz <= 12 * a.n_rows) || (nvec == 1 && vbytes == 8);
+    return nvec >= 16 || (nvec >= 4 && a.nnz <= 12 * a.n_rows);
 }
 
 template <typename VT>
