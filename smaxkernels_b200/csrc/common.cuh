@@ -115,6 +115,10 @@ struct DevBuf {
 
 inline unsigned ceil_div_u(uint64_t a, uint64_t b) { return (unsigned)((a + b - 1) / b); }
 
+// Whether an int that counts to n may pass 2^31 in the steps of a kernel that goes
+// a little beyond its end before it looks.
+inline bool near_int_end(int64_t n) { return n > (1ll << 31) - 4096; }
+
 // number of SMs of the current device (148 on B200), cached per device
 int sm_count();
 int64_t l2_bytes();  // L2 capacity of the current device

@@ -468,15 +468,16 @@ void bcrs_spmv(const DevBCRS &m, const VT *x, VT *y, cudaStream_t st) {
     // Blocks of more than 16 values leave a fifth of a warp's lanes idle: 2^19
     // block rows of five 5x5 blocks, FP32 (500 bytes) 248 and 292 us.
     const int64_t short_row = bs > 16 && m.n_blocks >= 4 * m.n_rows ? 512 : 256;
-    const bool thread_rows = m.n_rows >= 1024ll * sm_count() &&
-                             m.n_blocks * bs * (int64_t)sizeof(VT) <= short_row * m.n_rows;
+    const bool int_end = near_int_end(m.n_blocks);
+    const bool thread_rows = int_end || (m.n_rows >= 1024ll * sm_count() &&
+                                         m.n_blocks * bs * (int64_t)sizeof(VT) <= short_row * m.n_rows);
     // a lane per in-block position, `lanes` lanes per block row
     auto go_lanes = [&](auto kern, int lanes) {
         kern<<<ceil_div_u(m.n_rows, 8 * (32 / lanes)), 256, 0, st>>>(
             m.row_ptr.as<int>(), m.col.as<int>(), m.val.as<VT>(), m.n_rows, (int)m.bh, (int)m.bw, (int)m.hpad,
             (int)m.wpad, m.col_major ? 1 : 0, x, y, order, lanes);
     };
-    if (bcrs_stream_path(m.hpad, m.wpad, sizeof(VT))) {
+    if (bcrs_stream_path(m.hpad, m.wpad, sizeof(VT)) && !int_end) {
         // mean warp steps per block row: below two a lane group per block row
         // wastes fewer lanes; more loads in flight pay off from about three
         const double steps = (double)m.n_blocks * (double)bs / ((double)m.n_rows * 32.0 * VEC);
