@@ -607,14 +607,17 @@ __global__ void __launch_bounds__(256) to_row_major_kernel(const VT *__restrict_
     // 32 rows by up to 64 columns through shared memory: both sides coalesced
     __shared__ VT tile[64][kTrRows + 1];
     const int64_t r0 = (int64_t)blockIdx.x * kTrRows;
-    const int v0 = blockIdx.y * 64, nv = min(64, kp - v0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int v = w; v < nv; v += 8)
-        tile[v][lane] = (v0 + v < k && r0 + lane < n) ? ld_stream(X + (int64_t)(v0 + v) * ld + r0 + lane) : VT(0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < kTrRows * nv; i += 256) {
-        const int r = i / nv, v = i - r * nv;
-        if (r0 + r < n) T[(r0 + r) * kp + v0 + v] = tile[v][r];
+    for (int v0 = blockIdx.y * 64; v0 < kp; v0 += gridDim.y * 64) {
+        const int nv = min(64, kp - v0);
+        for (int v = w; v < nv; v += 8)
+            tile[v][lane] = (v0 + v < k && r0 + lane < n) ? ld_stream(X + (int64_t)(v0 + v) * ld + r0 + lane) : VT(0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTrRows * nv; i += 256) {
+            const int r = i / nv, v = i - r * nv;
+            if (r0 + r < n) T[(r0 + r) * kp + v0 + v] = tile[v][r];
+        }
+        __syncthreads();
     }
 }
 
@@ -822,7 +825,7 @@ void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStre
     constexpr int VEC = V16<VT>::N;
     const uintptr_t bits = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y) | (k * sizeof(VT));
     const bool grid = variant == 1 || (variant == 0 && grid_suits(a, plan, (bits & 15) == 0 ? k / VEC : 0, sizeof(VT)));
-    if (!grid && k > 1 && k < (1 << 30)) {
+    if (!grid && k > 1 && k < (1 << 30) && !near_int_end(a.n_rows)) {
         if ((bits & 15) == 0) launch_groups<VT, 16, false>(a, plan, k, k, X, Y, k, st);
         else if ((bits & 7) == 0 || sizeof(VT) == 8) launch_groups<VT, 8, false>(a, plan, k, k, X, Y, k, st);
         else launch_groups<VT, sizeof(VT), false>(a, plan, k, k, X, Y, k, st);
@@ -860,6 +863,7 @@ void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStre
 // 66 and 141; 2^19 rows of 8, one in 100 of 64: 60 and 89; 20000 of these 27 and
 // 23) and three where some are far longer (lognormal 30000 FP32 37 and 47, 300000 92 and 105).
 bool spmm_by_columns(const DevCRS &a, int64_t k, int64_t longest) {
+    if (near_int_end(a.n_rows) || k >= (1 << 30)) return true;
     const bool skewed = longest * a.n_rows > 64 * a.nnz;
     const bool uneven = longest * a.n_rows > 2 * a.nnz + 8 * a.n_rows;
     if (a.nnz < 4 * a.n_rows) return (k < 8 && a.n_rows >= (1 << 17)) || (k <= 8 && skewed);
@@ -877,7 +881,7 @@ void crs_spmm_col_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, int64_t 
     if (a.n_rows == 0 || k == 0) return;
     constexpr int VEC = V16<VT>::N;
     const int64_t kp = (k + VEC - 1) / VEC * VEC;
-    to_row_major_kernel<VT><<<dim3(ceil_div_u(a.n_cols, kTrRows), ceil_div_u(kp, 64)), 256, 0, st>>>(
+    to_row_major_kernel<VT><<<dim3(ceil_div_u(a.n_cols, kTrRows), std::min(ceil_div_u(kp, 64), 65535u)), 256, 0, st>>>(
         X, a.n_cols, (int)k, (int)kp, ld, work);
     SMAX_CUDA(cudaGetLastError());
     if (plan.n_long > 0) launch_pieces<VT>(a, plan, k, kp, work, Y, ld, st);

@@ -37,3 +37,26 @@ def test_block_product_of_two_billion_blocks():
     k.sync()
     smax.close()
     assert torch.equal(y, (rp[1:] - rp[:-1]).float() * 2)
+
+
+def test_column_major_block_of_more_vectors_than_a_grid_is_high():
+    """4.3 million vectors of 6 rows."""
+    import torch
+    n, kk = 6, 65535 * 64 + 70000
+    rp = np.array([0, 2, 4, 5, 6, 8, 9], np.int32)
+    col = np.array([0, 5, 1, 2, 2, 3, 4, 0, 5], np.int32)
+    val = np.arange(1, 10, dtype=np.float32)
+    A = torch.zeros(n, n, device="cuda")
+    A[torch.from_numpy(np.repeat(np.arange(n), np.diff(rp))).cuda(), torch.from_numpy(col).long().cuda()] = torch.from_numpy(val).cuda()
+    X = (torch.arange(n * kk, device="cuda") % 17).float()
+    Y = torch.zeros_like(X)
+    smax, k = _kernel("SPMM", np.float32)
+    k.set_vec_row_major(False)
+    k.register_A(n, n, len(col), col, rp, val)
+    k.register_B(n, kk, X)
+    k.register_C(n, kk, Y)
+    k.initialize()
+    k.apply()
+    k.sync()
+    smax.close()
+    assert torch.equal(Y.view(kk, n), (X.view(kk, n).double() @ A.double().t()).float())
