@@ -461,16 +461,21 @@ void bcrs_spmv(const DevBCRS &m, const VT *x, VT *y, cudaStream_t st) {
                                              (int)m.bh, (int)m.bw, (int)m.hpad, (int)m.wpad, m.col_major ? 1 : 0, x, y,
                                              order);
     };
-    // Enough block rows to fill the chip with a thread each, and so short that a
-    // warp's rows stay in L1 while they are read: 3x3 blocks of a 7-point grid
-    // 64^3, FP32 (252 bytes a row) 46 us with a thread, 57 with a lane per
-    // position; FP64 (504 bytes) 84 and 63; 28^3 FP32 17.5 and 14.7.
-    // Blocks of more than 16 values leave a fifth of a warp's lanes idle: 2^19
-    // block rows of five 5x5 blocks, FP32 (500 bytes) 248 and 292 us.
-    const int64_t short_row = bs > 16 && m.n_blocks >= 4 * m.n_rows ? 512 : 256;
+    // A thread or a lane per position (block sizes off the stream path): a thread's
+    // time grows with a row's values, which its warp reads strided and must find in
+    // L1 again; that of the lanes with the number of rows, a warp each above 16 values
+    // a block, of which every chunk of rows pays its latency.  Blocks of up to 16
+    // values, thread / lanes, us: 3x3, one a row, 20000 rows FP32 10 / 12, 80000 12 / 20; five a
+    // row, 20000 16 / 14, 80000 22 / 24; FP64 of 2^19 rows, four a row 100 / 92, seven 194 / 117.
+    // Larger ones: 5x5, one a row, 8000 rows FP32 12 / 14, 20000 12 / 18; three a row, 8000
+    // 17 / 14, 20000 18 / 19, 40000 22 / 28, 2^19 129 / 247, FP64 216 / 272, and four 307 / 281;
+    // five, FP32 247 / 292; 7x7, 2.3 a row, 40000 rows FP32 30 / 26, 80000 40 / 43, 2^19 FP64
+    // 298 / 293, three a row 397 / 344, FP32 304 / 270.
     const bool int_end = near_int_end(m.n_blocks);
-    const bool thread_rows = int_end || (m.n_rows >= 1024ll * sm_count() &&
-                                         m.n_blocks * bs * (int64_t)sizeof(VT) <= short_row * m.n_rows);
+    const int64_t most_vals = bs <= 16 ? std::min<int64_t>(256 / (int64_t)sizeof(VT), m.n_rows / 1500)
+                                       : std::min<int64_t>(sizeof(VT) == 4 ? 128 : 112, m.n_rows / 400);
+    const bool thread_rows = int_end || (m.n_blocks * bs <= most_vals * m.n_rows &&
+                                         (bs <= 16 || sizeof(VT) == 4 || m.n_blocks < 4 * m.n_rows));
     // a lane per in-block position, `lanes` lanes per block row
     auto go_lanes = [&](auto kern, int lanes) {
         kern<<<ceil_div_u(m.n_rows, 8 * (32 / lanes)), 256, 0, st>>>(
@@ -510,9 +515,12 @@ void bcrs_spmv(const DevBCRS &m, const VT *x, VT *y, cudaStream_t st) {
             });
         }
     } else if (bs <= 32 && !thread_rows) {
-        // fewer than three warp steps a block row: several block rows a warp
-        const int per = 32 / (int)bs;
-        go_lanes(bcrs_lane_kernel<VT, 1, 4>, m.n_blocks < 3 * per * m.n_rows ? (int)bs : 32);
+        // several block rows a warp: fewer than three warp steps a block row, or more
+        // where there are rows for all warps (2^19 rows of nine 3x3 blocks FP64: 135 us,
+        // 260 with a warp each; 27 of them on 160000 rows 88 and 131; 1000 rows 13.6 and 11.7)
+        const int64_t per = 32 / bs;
+        const bool many = bs <= 16 && m.n_rows >= 64ll * sm_count() && m.n_blocks <= 32 * m.n_rows;
+        go_lanes(bcrs_lane_kernel<VT, 1, 4>, many || m.n_blocks < 3 * per * m.n_rows ? (int)bs : 32);
     } else if (bs <= 64 && !thread_rows) {
         go_lanes(bcrs_lane_kernel<VT, 2, 2>, 32);
     } else if (bs <= kMaxBs && !thread_rows) {

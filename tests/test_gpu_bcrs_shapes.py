@@ -76,3 +76,28 @@ def test_many_short_block_rows(vt, most):
     k.run()
     smax.close()
     assert normwise(y, O.spmv_bcrs(nb, 3, 3, 3, 3, rp, col, val, False, x)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("nb,per_row,bs", [(9999, 1, 5), (10000, 1, 5), (10001, 1, 5), (40000, 4, 5), (51200, 5, 5),
+                                           (43200, 3, 6), (13499, 1, 3), (13500, 1, 3), (9471, 12, 3), (9500, 32, 3),
+                                           (9500, 33, 3), (33000, 1, 9)])
+def test_thread_or_lanes_at_their_border(vt, nb, per_row, bs):
+    """Block rows of one length, where the kernel changes with their number and size."""
+    from smaxkernels_b200 import FloatType, Interface, IntType, KernelType, PlatformType
+    rng = np.random.default_rng(nb)
+    rp = (np.arange(nb + 1) * per_row).astype(np.int32)
+    col = rng.integers(0, nb, rp[-1]).astype(np.int32)
+    val = rng.uniform(-1, 1, len(col) * bs * bs).astype(vt)
+    x, y = rng.uniform(-1, 1, nb * bs).astype(vt), np.zeros(nb * bs, vt)
+    smax = Interface()
+    smax.register_kernel("k", KernelType.SPMV, PlatformType.CUDA, IntType.INT32,
+                         FloatType.FLOAT64 if vt == np.float64 else FloatType.FLOAT32)
+    k = smax.kernel("k")
+    k.set_mat_bcrs(True)
+    k.register_A(nb, nb, len(col), bs, bs, bs, bs, col, rp, val)
+    k.register_B(nb * bs, x)
+    k.register_C(nb * bs, y)
+    k.run()
+    smax.close()
+    assert normwise(y, O.spmv_bcrs(nb, bs, bs, bs, bs, rp, col, val, False, x)) <= tol(vt)
