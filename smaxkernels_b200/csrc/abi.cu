@@ -156,7 +156,7 @@ void spmv_upload(smax_kernel_s *k) {
         if (k->spmv_variant == 2)
             k->crs_plan.build(k->dA.rp(), k->dA.n_rows, crs_default_cap(k->vbytes * 8), st);
         else
-            k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, st);
+            k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, st, k->dA.ci());
     }
 }
 
@@ -186,7 +186,8 @@ void spmm_upload(smax_kernel_s *k) {
     read_status(k);
     k->crs_stream = CrsStreamPlan();
     k->spmm_plan.build(k->dA, !k->f_row_major, k->stream);
-    if (!k->f_row_major) k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, k->stream);
+    if (!k->f_row_major)
+        k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, k->stream, k->dA.ci());
 }
 
 template <typename VT> void spmm_apply_t(smax_kernel_s *k, const VT *X, VT *Y) {
@@ -423,7 +424,7 @@ bool pipe_ready(smax_kernel_s *k) {
         for (int64_t i = 0; i <= rows; ++i) h[i] = rp[r0[b] + i] - (int)e0[b];
         P.rps[b].alloc(sizeof(int) * (rows + 1));
         SMAX_CUDA(cudaMemcpyAsync(P.rps[b].p, h.data(), sizeof(int) * (rows + 1), cudaMemcpyHostToDevice, k->stream));
-        P.plans[b].build(P.rps[b].as<int>(), rows, e0[b + 1] - e0[b], k->vbytes, k->stream);
+        P.plans[b].build(P.rps[b].as<int>(), rows, e0[b + 1] - e0[b], k->vbytes, k->stream, k->dA.ci() + e0[b]);
     }
     P.r0 = std::move(r0);
     P.e0 = std::move(e0);
@@ -582,7 +583,7 @@ void smax::build_crs_plans(smax_kernel_s *k) {
     k->crs_plan = CrsTilePlan();
     k->crs_plan.build(k->dA.rp(), k->dA.n_rows, crs_default_cap(k->vbytes * 8), k->stream);
     k->crs_stream = CrsStreamPlan();
-    k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, k->stream);
+    k->crs_stream.build(k->dA.rp(), k->dA.n_rows, k->dA.nnz, k->vbytes, k->stream, k->dA.ci());
     SMAX_CUDA(cudaStreamSynchronize(k->stream));
 }
 

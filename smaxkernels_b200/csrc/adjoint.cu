@@ -146,7 +146,7 @@ void build_transpose(const DevCRS &a, int vbytes, bool desc, bool with_plan, Dev
     SMAX_CUDA(cudaGetLastError());
     gather_values(a, vbytes, t, true, st);
     t.plan = CrsStreamPlan();
-    if (with_plan) t.plan.build(at.rp(), m, nnz, vbytes, st);
+    if (with_plan) t.plan.build(at.rp(), m, nnz, vbytes, st, at.ci());
     t.has_plan = with_plan;
     t.descending = desc;
     t.built = true;

@@ -256,6 +256,39 @@ __global__ void row_flags_kernel(const int *__restrict__ row_ptr, int64_t n, uns
     if ((threadIdx.x & 31) == 0 && len > 0) atomicMax(max_len, len);
 }
 
+// A sample of the columns, 32 neighbouring rows a warp: found[0] counts entries of
+// rows short enough for crs_rows_kernel, found[1] those whose column lies more
+// than kFar from that of the row before's entry in the same place.
+constexpr int kFar = 16384;
+constexpr int kSampleWarps = 512;
+__global__ void scatter_sample_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col, int64_t n,
+                                      int *__restrict__ found) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t r = (n > 32 ? (n - 32) * w / kSampleWarps : 0) + lane;
+    int s = 0, len = 0;
+    if (r < n) {
+        s = row_ptr[r];
+        len = min(row_ptr[r + 1] - s, 32);
+    }
+    int seen = 0, far = 0;
+    const int most = __reduce_max_sync(0xffffffffu, len);
+    for (int i = 0; i < most; ++i) {
+        const int c = i < len ? col[s + i] : -1;
+        const int before = __shfl_up_sync(0xffffffffu, c, 1);
+        if (lane > 0 && c >= 0 && before >= 0) {
+            ++seen;
+            far += abs(c - before) > kFar;
+        }
+    }
+    seen = __reduce_add_sync(0xffffffffu, seen);
+    far = __reduce_add_sync(0xffffffffu, far);
+    if (lane == 0) {
+        atomicAdd(found, seen);
+        atomicAdd(found + 1, far);
+    }
+}
+
 // rank of the row holding entry t*W: the largest r with row_ptr[r] <= t*W
 // (that row is non-empty), then its position among the non-empty rows.
 __global__ void task_rank_kernel(const int *__restrict__ row_ptr, int64_t n, const int *__restrict__ row_list,
@@ -284,7 +317,8 @@ __global__ void task_rank_kernel(const int *__restrict__ row_ptr, int64_t n, con
 
 int crs_stream_pad() { return kW; }
 
-void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vbytes, cudaStream_t st) {
+void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vbytes, cudaStream_t st,
+                          const int *d_col) {
     n_rows = n;
     nnz = nnz_;
     n_tasks = (nnz + kW - 1) / kW;
@@ -295,12 +329,15 @@ void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vby
     n_nonempty = 0;
     row_ptr = d_row_ptr;
     longest = 0;
+    scattered = false;
     if (n > 0) {
-        DevBuf fe(n), fne(n), cnt(sizeof(int) * 3);
+        DevBuf fe(n), fne(n), cnt(sizeof(int) * 5);
         SMAX_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes, st));
         row_flags_kernel<<<ceil_div_u(n, 256), 256, 0, st>>>(d_row_ptr, n, fe.as<unsigned char>(),
                                                              fne.as<unsigned char>(), endbits.as<uint32_t>(),
                                                              cnt.as<int>() + 2);
+        if (d_col)
+            scatter_sample_kernel<<<kSampleWarps / 8, 256, 0, st>>>(d_row_ptr, d_col, n, cnt.as<int>() + 3);
         SMAX_CUDA(cudaGetLastError());
         thrust::counting_iterator<int> it(0);
         empty_rows.alloc(sizeof(int) * n);
@@ -310,11 +347,12 @@ void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vby
         DevBuf tmp(tb);
         SMAX_CUDA(cub::DeviceSelect::Flagged(tmp.p, tb, it, fe.as<unsigned char>(), empty_rows.as<int>(),
                                              cnt.as<int>(), (int)n, st));
-        int h[3] = {0, 0, 0};
+        int h[5] = {0, 0, 0, 0, 0};
         SMAX_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, st));
         SMAX_CUDA(cudaStreamSynchronize(st));
         n_empty = h[0];
         longest = h[2];
+        scattered = 2 * h[4] > h[3];
         n_nonempty = n - n_empty;
         if (n_empty > 0) {
             row_list.alloc(sizeof(int) * (n_nonempty > 0 ? n_nonempty : 1));
@@ -344,8 +382,11 @@ void crs_spmv_stream(const CrsStreamPlan &p, const int *col, const VT *val, cons
     // thirds full on average.  B200, us, stream -> rows: 128^3 7-point FP64
     // (98% full) 54.8 -> 48.1, 96^3 27-point 86.3 -> 70.9, 2^20 rows of 5, one in
     // 100 of 7 (72%) 32.3 -> 25.0; 2^22 rows of 0 to 32 evenly (50%) 299 -> 318,
-    // of 2, one in 100 of 32 (7%) 57 -> 229.
-    if (p.n_rows > 0 && p.longest <= 32 && 3 * p.nnz >= 2 * p.n_rows * p.longest) {
+    // of 2, one in 100 of 32 (7%) 57 -> 229.  Columns all over a large x push a row's
+    // own lines out of L1 before its lanes have used them: 2^20 rows of 17 FP64 88 ->
+    // 107, of 32 150 -> 172 (of 8 45 -> 47, and 2^17 rows of 32 30 -> 30).
+    const bool crowded = p.scattered && p.longest > 8 && p.n_rows >= (1 << 18);
+    if (p.n_rows > 0 && p.longest <= 32 && !crowded && 3 * p.nnz >= 2 * p.n_rows * p.longest) {
         // rows without entries get their zero here as well
         auto rows = [&](auto kern, int g) {
             kern<<<ceil_div_u((uint64_t)p.n_rows * g, 256), 256, 0, st>>>(col, val, p.row_ptr, p.n_rows, x, y);

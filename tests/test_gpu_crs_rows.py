@@ -62,3 +62,21 @@ def test_row_blocks_of_a_host_product(longest):
         k.run()
     smax.close()
     assert normwise(y, O.spmv_crs(rp, col, val, x)) <= 1e-12
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("longest", [8, 9, 32])
+@pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18])
+@pytest.mark.parametrize("far", [False, True])
+def test_columns_near_and_all_over(vt, longest, n, far):
+    """Neighbouring rows' columns decide between the kernels from 2^18 rows on."""
+    from helpers import gpu_spmv
+    rng = np.random.default_rng(longest)
+    lens = np.full(n, longest)
+    lens[:5] = [0, 1, longest, 2, 0]
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    rows = np.repeat(np.arange(n), lens)
+    col = (rng.integers(0, n, rp[-1]) if far else np.minimum(rows + rng.integers(0, 99, rp[-1]), n - 1)).astype(np.int32)
+    val = rng.uniform(-1, 1, len(col)).astype(vt)
+    x = rng.uniform(-1, 1, n).astype(vt)
+    assert normwise(gpu_spmv(rp, col, val, x), O.spmv_crs(rp, col, val, x)) <= tol(vt)
