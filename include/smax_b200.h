@@ -92,7 +92,8 @@ typedef int smax_status;
 #define SMAX_FLAG_SPMV_VARIANT 10      /* CRS SpMV kernel: 0 auto, 1 warp-stream, 2 row-tile; row-major SpMM:
                                           0 auto, 1 a grid of all rows, 2 one CTA per SM walking a row range */
 #define SMAX_FLAG_SOLVE_MODE 11        /* SpTRSV/SpTRSM launch scheme, one of SMAX_SOLVE_* */
-#define SMAX_FLAG_LEVEL_MERGE 12       /* levels with <= this many rows*rhs run merged in one CTA (0: never) */
+#define SMAX_FLAG_LEVEL_MERGE 12       /* levels with <= this many rows*rhs run merged in one CTA (0: never); default
+                                          4096, for sweeps 4096 entries if rows have more than 2.5 off the diagonal */
 #define SMAX_FLAG_SPIN_LIMIT 13        /* polls (x 1000) before a wait of a solve times out; the level sweeps, whose
                                           waits sleep, count 128 ns a poll (default 20000: 2.56 s) */
 #define SMAX_FLAG_TEST_FORCE_TIMEOUT 14 /* test only: a wait of the solve (barrier, level, solution) is never ended */

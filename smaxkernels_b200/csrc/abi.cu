@@ -67,6 +67,8 @@ SweepWait sweep_wait(const smax_kernel_s *k) { return {k->spin_limit * SweepWait
 void tri_plan(smax_kernel_s *k) {
     k->tri.status = dstatus(k);
     k->tri.wait = sweep_wait(k);
+    k->tri.off_diag = k->dA.nnz - k->dA.n_rows;
+    k->tri.run_rows = tri_run_rows(k);
     if (k->f_perm) {
         require(k->ctx != nullptr && k->ctx->n_levels > 0, SMAX_ERR_STATE,
                 "level-scheduled solve needs the levels of generate_perm in the context");

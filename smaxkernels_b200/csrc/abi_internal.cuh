@@ -28,6 +28,14 @@ inline int tri_merge_rows(const smax_kernel_s *k) {
     return k->solve_mode == SMAX_SOLVE_PER_LEVEL ? 0 : (k->level_merge >= 0 ? k->level_merge : kDefaultLevelMerge);
 }
 
+// rows up to which a level of the sweeps is swept in a run, if the default (no
+// threshold is set); -1: the threshold in effect
+inline int tri_run_rows(const smax_kernel_s *k) {
+    return k->solve_mode == SMAX_SOLVE_PER_LEVEL || k->level_merge >= 0
+               ? -1
+               : default_run_rows(k->dA.n_rows, k->dA.nnz - k->dA.n_rows);
+}
+
 // the launches of one apply of an initialized kernel (SpMV, SpMM, SpTRSV,
 // SpTRSM), without the stopwatch events
 void apply_core(smax_kernel_s *k, uint64_t b_off, uint64_t c_off);

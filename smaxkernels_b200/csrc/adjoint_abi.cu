@@ -47,6 +47,8 @@ void ensure_adjoint(smax_kernel_s *k) {
     }
     k->adj_plan.status = dstatus(k);
     k->adj_plan.wait = sweep_wait(k);
+    k->adj_plan.off_diag = k->tri.off_diag;
+    k->adj_plan.run_rows = k->tri.run_rows;
 }
 
 template <typename VT> void adjoint_t(smax_kernel_s *k, const VT *x, const VT *g, VT *din, VT *dval) {

@@ -212,6 +212,7 @@ void TriPlan::finish(cudaStream_t) {
 
 bool TriPlan::ensure_pack(const int *rp, const int *ci, const void *val, const void *D, int vbytes, int merge_rows,
                           uint64_t tag, cudaStream_t st, int64_t k) {
+    merge_rows = run_threshold(merge_rows);
     if (pack_unfit(merge_rows, k)) return false;
     if (!pack_is(val, D, vbytes, merge_rows, pack_tag, k)) {
         if (scheduled_k != 1 || scheduled_merge != merge_rows) schedule(1, merge_rows);
@@ -406,7 +407,7 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
     if (p.n_rows == 0) return;
     // the pack is built outside the capture (it synchronises); a rebuild drops the graph
     bool packed = false;
-    if (k == 1 || sweep_suits(p, merge_rows)) {
+    if (k == 1 || sweep_suits(p, k, merge_rows)) {
         try {
             packed = p.ensure_pack(a.rp(), a.ci(), a.val.p, D, sizeof(VT), merge_rows, tag, caller, k);
         } catch (const Error &e) {
@@ -415,7 +416,7 @@ void tri_solve_graph(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *
             if (k == 1 || e.code != SMAX_ERR_OOM) throw;
             p.pack = SweepPack();
             p.pack_ok = false;
-            p.pack_refused.push_back({merge_rows, true});
+            p.pack_refused.push_back({p.run_threshold(merge_rows), true});
             p.release_graph();
         }
     }
@@ -485,14 +486,31 @@ void TriPlan::release_graph() {
 
 TriPlan::~TriPlan() { release_graph(); }
 
-bool sweep_suits(const TriPlan &p, int merge_rows) {
+// One SM goes through a level of 4096 entries in about the time of a launch: 0.3 ns
+// an entry whose solution is in the ring, 0.8 to 1.3 from global memory, against
+// 2.3 us and a whole chip.  FP64, random sources, run / grid: 1500 rows of 3 entries 3.1 /
+// 2.2 us a level, of 8 8.9 / 4.0, of 40 69 / 5.5; 600 of 8 3.9 / 3.7; 200 of 40 10 / 5.2; 30 of
+// 40 3.6 / 4.8.  Rows of two entries (5-point triangles) stay in runs up to 4096.
+int default_run_rows(int64_t n_rows, int64_t off_diag) {
+    constexpr int kRows = 4096;
+    if (2 * off_diag <= 5 * n_rows) return kRows;
+    return (int)std::max<int64_t>(1, (int64_t)kRows * n_rows / off_diag);
+}
+
+// k > 1 vectors: the wide levels of the sweeps read a solution from k separate
+// vectors, where the level launches and the sync-free rows read k neighbours.
+// FP64, random sources, sweeps / those: 1500 x 40 levels of 3 entries k = 32 124 / 123 us, of 8 200
+// / 136, k = 4 173 / 136, of 40 k = 32 422 / 272, k = 4 235 / 284; 600 x 60 of 8 k = 32 237 / 197, k = 4 236 / 456;
+// 200 x 100 of 40 k = 32 530 / 635.
+bool sweep_suits(const TriPlan &p, int64_t k, int merge_rows) {
     const int64_t L = p.n_levels();
-    return L > 0 && !p.pack_unfit(merge_rows, 2) && p.n_rows <= L * 2048;
+    return L > 0 && !p.pack_unfit(merge_rows, 2) && p.n_rows <= L * 2048 &&
+           (p.off_diag <= L * 4096 || p.n_rows * k <= L * 8192);
 }
 
 bool syncfree_suits(const TriPlan &p, int64_t k, int merge_rows) {
     const int64_t L = p.n_levels();
-    if (L <= 0 || (k > 1 && sweep_suits(p, merge_rows))) return false;
+    if (L <= 0 || (k > 1 && sweep_suits(p, k, merge_rows))) return false;
     if (k == 1) return p.n_rows >= (1 << 17) && p.n_rows >= L * 32768;
     return p.n_rows >= (1 << 16) && L >= 64 && p.n_rows <= L * 16384;
 }

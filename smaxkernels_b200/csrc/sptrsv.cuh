@@ -56,11 +56,16 @@ struct TriPlan {
     // tag, the merge threshold and one or several right-hand sides below
     SweepPack pack;
     bool pack_ok = false;
+    // Rows of a level up to which it is swept in a run, -1: the merge threshold
+    // that a call gives; and the matrix's off-diagonal entries.  Set by the owner.
+    int run_rows = -1;
+    int64_t off_diag = 0;
+    int run_threshold(int merge_rows) const { return run_rows >= 0 ? run_rows : merge_rows; }
     // merge thresholds (and one or several right-hand sides) whose pack was
     // refused: the levels swept in runs, and so the limits on a run, are theirs
     std::vector<std::pair<int, bool>> pack_refused;
     bool pack_unfit(int merge_rows, int64_t k) const {
-        return std::find(pack_refused.begin(), pack_refused.end(), std::make_pair(merge_rows, k > 1)) !=
+        return std::find(pack_refused.begin(), pack_refused.end(), std::make_pair(run_threshold(merge_rows), k > 1)) !=
                pack_refused.end();
     }
     const void *pack_key[2] = {nullptr, nullptr};
@@ -77,8 +82,8 @@ struct TriPlan {
                      uint64_t tag, cudaStream_t st, int64_t k = 1);
     // whether the pack is the one a solve with these arguments uses
     bool pack_is(const void *val, const void *D, int vbytes, int merge_rows, uint64_t tag, int64_t k) const {
-        return pack_ok && pack_key[0] == val && pack_key[1] == D && pack_tag == tag && pack_merge == merge_rows &&
-               pack_vbytes == vbytes && pack.div == (k > 1);
+        return pack_ok && pack_key[0] == val && pack_key[1] == D && pack_tag == tag &&
+               pack_merge == run_threshold(merge_rows) && pack_vbytes == vbytes && pack.div == (k > 1);
     }
 
     // sync-free form of the pack (SMAX_SOLVE_SYNCFREE): every level its own
@@ -124,9 +129,13 @@ void tri_solve(TriPlan &p, const DevCRS &a, const VT *D, const VT *B, VT *X, int
 template <typename VT>
 void tri_solve_raw(TriPlan &p, const int *rp, const int *ci, const VT *val, const VT *D, const VT *B, VT *X,
                    int64_t k, bool row_major, int64_t ld, int merge_rows, uint64_t tag, cudaStream_t st);
+// Rows of a level of a matrix with off_diag off-diagonal entries up to which it
+// is swept in a run by default.
+int default_run_rows(int64_t n_rows, int64_t off_diag);
 // Whether blocks of k > 1 right-hand sides run as sweeps of the pack, one CTA
-// each: levels of at most 2048 rows on average, and a pack not yet refused.
-bool sweep_suits(const TriPlan &p, int merge_rows);
+// each: levels of at most 2048 rows on average, whose entries one SM or whose
+// k solutions the grid takes in a launch's time, and a pack not yet refused.
+bool sweep_suits(const TriPlan &p, int64_t k, int merge_rows);
 // The sync-free solve of one right-hand side (pack_solve_syncfree).  Returns
 // false, launching nothing, when it does not apply: the matrix does not pack,
 // an entry reads a row not solved before it, or B and X overlap.

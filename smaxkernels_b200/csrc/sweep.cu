@@ -365,6 +365,51 @@ __global__ void __launch_bounds__(256, 8) sw_wide_kernel(SweepPack::Wide L, cons
     xp[p] = finish_row<VT, DIV>(b, sum, d);
 }
 
+// The same of longer rows: kLongEnts entries and their solutions at a time, the
+// next entries on their way while these are added.  64 threads a CTA, so that a
+// level of a few hundred rows still spreads over the SMs.
+constexpr int kLongEnts = 16;
+template <typename VT, bool DIV>
+__global__ void __launch_bounds__(64) sw_wide_long_kernel(SweepPack::Wide L, const unsigned char *__restrict__ blob,
+                                                          int64_t npos, const VT *__restrict__ bp, VT *xp) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= L.m) return;
+    const unsigned char *data = blob + (int64_t)L.off * 16 + kHeader;
+    const VT *pv = reinterpret_cast<const VT *>(data) + t;
+    const int *ps = reinterpret_cast<const int *>(data + (int64_t)(L.w + 1) * L.mp * (int)sizeof(VT)) + t;
+    const int64_t p = blockIdx.y * npos + L.pos + t;
+    VT *x = xp + blockIdx.y * npos;
+    const VT b = bp[p], d = pv[(int64_t)L.w * L.mp];
+    int src[kLongEnts];
+    VT v[kLongEnts], sum = VT(0);
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int i = 0; i < kLongEnts; ++i) {
+            src[i] = 0;  // padding
+            v[i] = VT(0);
+            if (i0 + i < L.w) {
+                src[i] = ps[(int64_t)(i0 + i) * L.mp];
+                v[i] = pv[(int64_t)(i0 + i) * L.mp];
+            }
+        }
+    };
+    fetch(0);
+    for (int i0 = 0; i0 < L.w; i0 += kLongEnts) {
+        VT xs[kLongEnts], w[kLongEnts];
+#pragma unroll
+        for (int i = 0; i < kLongEnts; ++i) {
+            xs[i] = src[i] < 0 ? x[~src[i]] : VT(0);
+            w[i] = v[i];
+        }
+        const bool last = src[kLongEnts - 1] >= 0;  // the row ends here
+        if (!last) fetch(i0 + kLongEnts);
+#pragma unroll
+        for (int i = 0; i < kLongEnts; ++i) sum += w[i] * xs[i];
+        if (last) break;
+    }
+    xp[p] = finish_row<VT, DIV>(b, sum, d);
+}
+
 // ----------------------------------------------------------------- runs ----
 // Shared state of a sweeping CTA, at the start of its dynamic shared memory.
 struct SweepShared {
@@ -629,17 +674,18 @@ __device__ VT sw_sum_any(const unsigned char *stage, int at, const ChunkView &c,
     const VT *pv = reinterpret_cast<const VT *>(stage + at + kHeader);
     const int *ps = reinterpret_cast<const int *>(pv + (w + 1) * c.mp());
     // four entries at a time: their solutions are read before any is used
+    constexpr int U = 4;
 #pragma unroll 1
-    for (int i = 0; i < w; i += 4) {
-        VT v[4], x[4];
+    for (int i = 0; i < w; i += U) {
+        VT v[U], x[U];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < U; ++q)
             if (i + q < w) {
                 v[q] = pv[(i + q) * c.mp() + t];
                 x[q] = sw_solution<VT>(ps[(i + q) * c.mp() + t], ring, xp);
             }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < U; ++q)
             if (i + q < w) sum += v[q] * x[q];
     }
     return sum;
@@ -1236,8 +1282,10 @@ void sweep_solve(const SweepPack &pk, const VT *B, VT *X, int64_t k, int64_t rs,
         for (const SweepPack::Item &it : pk.items) {
             if (it.wide) {
                 const SweepPack::Wide &L = pk.wides[it.index];
-                const dim3 g(ceil_div_u(L.m, 256), (unsigned)kv);
-                if (pk.div) sw_wide_kernel<VT, true><<<g, 256, 0, st>>>(L, blob, pk.npos, bp, xp);
+                const dim3 g(ceil_div_u(L.m, L.w > 2 * kWideEnts ? 64 : 256), (unsigned)kv);
+                if (L.w > 2 * kWideEnts && pk.div) sw_wide_long_kernel<VT, true><<<g, 64, 0, st>>>(L, blob, pk.npos, bp, xp);
+                else if (L.w > 2 * kWideEnts) sw_wide_long_kernel<VT, false><<<g, 64, 0, st>>>(L, blob, pk.npos, bp, xp);
+                else if (pk.div) sw_wide_kernel<VT, true><<<g, 256, 0, st>>>(L, blob, pk.npos, bp, xp);
                 else sw_wide_kernel<VT, false><<<g, 256, 0, st>>>(L, blob, pk.npos, bp, xp);
             } else if (pk.div) {
                 launch_run<VT, true>(pk, pk.runs[it.index], it.threads, kv, bp, xp, status, wait, st);

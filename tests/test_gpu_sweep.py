@@ -65,6 +65,7 @@ def _solve(*args, **kw):
     return x
 
 
+MERGED = 2
 EDGES = [1, 2, 3, 4, 5, 31, 33, 127, 128, 129, 1, 255, 256, 257, 479, 480, 481, 607, 608, 609, 1215, 1217, 2000, 7]
 
 
@@ -77,6 +78,32 @@ def test_sweep_vs_oracle(vt, width, sizes):
     b = np.random.default_rng(1).uniform(-1, 1, len(rp) - 1).astype(vt)
     x = _solve("SPTRSV", rp, col, val, b)
     assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("width", [4, 5, 9, 40, 200])
+@pytest.mark.parametrize("merge", [0, 4096])
+def test_longer_rows_on_a_grid_and_in_runs(vt, width, merge):
+    """Levels at the edges of a run's chunks, of a grid's CTAs and of the entries it takes at a time."""
+    rp, col, val = level_matrix([3, 63, 64, 65, 1, 255, 257, 700, 31, 33, 128, 129] * 2, width, width, vt)
+    n = len(rp) - 1
+    b = np.random.default_rng(1).uniform(-1, 1, n).astype(vt)
+    smax, kern, x = _kernel("SPTRSV", rp, col, val, b)
+    kern.set_level_merge(merge)
+    kern.run()
+    smax.close()
+    assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("width,sizes,k", [(12, [300] * 30, 3), (12, [300] * 30, 40), (40, [200] * 40, 3), (17, [64, 65, 2] * 20, 5)])
+def test_blocks_of_longer_rows_equal_the_level_launches(vt, width, sizes, k):
+    """Sweeps, with wide levels of several vectors, and what takes their place."""
+    rp, col, val = level_matrix(sizes, width, 5, vt)
+    b = np.random.default_rng(k).uniform(-1, 1, (len(rp) - 1) * k).astype(vt)
+    for row_major in (True, False):
+        x = _solve("SPTRSM", rp, col, val, b, k=k, row_major=row_major)
+        np.testing.assert_array_equal(x, _solve("SPTRSM", rp, col, val, b, k=k, row_major=row_major, mode=MERGED))
 
 
 @pytest.mark.parametrize("vt", [np.float64, np.float32])
@@ -144,9 +171,6 @@ def test_sweep_waits_for_a_very_long_row():
     b = rng.uniform(-1, 1, n)
     x = _solve("SPTRSV", rp, col, val, b)
     assert normwise(x, O.sptrsv(rp, col, val, b)) <= tol(np.float64)
-
-
-MERGED = 2
 
 
 @pytest.mark.parametrize("vt", [np.float64, np.float32])
