@@ -9,7 +9,9 @@
 //    (sweep.cu: operands copied ahead into shared memory, a ring of recent
 //    solutions, an mbarrier per level; every wait is bounded and one that gives up
 //    is reported).  Matrices that would pack too sparsely use the plain kernel
-//    below, whose level barrier is the CTA barrier.  The launch (queue reset + kernel) is
+//    below, whose level barrier is the CTA barrier.  Few matrices with levels that
+//    are too much for one SM are solved a level of all of them at a time, each a launch of
+//    the whole chip (levels_on_grid).  The launches (queue reset + kernel) are
 //    captured once into a CUDA graph and replayed.
 // 2. Grid-wide persistent (one matrix, wide levels): a cooperative launch of
 //    co-resident CTAs sweeps all levels, with a software grid barrier between
@@ -142,6 +144,35 @@ __global__ void grid_persistent(const int *__restrict__ rp, const int *__restric
 
 }  // namespace
 
+namespace {
+
+// Whether launches that take the same level of every matrix are the faster way,
+// from what a level costs one SM (0.25 us at least; 0.3 ns an entry of rows of up to 2.5
+// entries in levels that the ring holds, 0.8 of others) and a launch the chip (2.5 us, 0.006
+// ns an entry).  level_entries: of each matrix's levels, off the diagonal.
+// FP64, random sources, one SM a matrix / launches: 20 matrices of 6 levels of 9000
+// rows of 3 entries 165 / 33 us; 4 of 20 x 2000 x 3 76 / 44; 8 of 20 x 1500 x 40 1900 / 158; 16 of
+// 40 x 50 x 100 340 either way.
+bool levels_on_grid(const std::vector<int64_t> &level_entries, const std::vector<int> &mat_levels, int64_t n_rows) {
+    int64_t entries = 0;
+    for (int64_t e : level_entries) entries += e;
+    const bool near = 2 * entries <= 5 * n_rows && n_rows <= 4096 * (int64_t)level_entries.size();
+    const double each = near ? 0.3e-3 : 0.8e-3;  // us
+    double longest = 0, total = 0;
+    int levels = 0;
+    size_t at = 0;
+    for (int L : mat_levels) {
+        double t = 0;
+        for (int l = 0; l < L; ++l) t += std::max(0.25, each * (double)level_entries[at++]);
+        longest = std::max(longest, t);
+        total += t;
+        levels = std::max(levels, L);
+    }
+    return 1.2 * (2.5 * levels + 0.006e-3 * (double)entries) < std::max(longest, total / sm_count());
+}
+
+}  // namespace
+
 // ------------------------------------------------------------- the batch ---
 void TriBatch::build(int vbytes_, const std::vector<RegCRS> &mats, cudaStream_t st) {
     vbytes = vbytes_;
@@ -209,7 +240,6 @@ void TriBatch::build(int vbytes_, const std::vector<RegCRS> &mats, cudaStream_t 
         mat_levels[m] = L;
     }
     lrows.push_back((int)n_rows);
-    (void)nl;
     // longest critical path first
     std::vector<int> qo(n_mats);
     std::iota(qo.begin(), qo.end(), 0);
@@ -231,10 +261,31 @@ void TriBatch::build(int vbytes_, const std::vector<RegCRS> &mats, cudaStream_t 
     h_mat_lvl_off = moff;
     row_off = roff;
     SMAX_CUDA(cudaStreamSynchronize(st));
-    // sweep steps = every matrix's levels in order; each matrix is one run
     const int L = total_levels;
-    std::vector<int> src_begin(L), count(L);
+    std::vector<int> src_begin, count;
     std::vector<SweepStep> steps;
+    std::vector<int64_t> entries(L, 0);
+    for (int l = 0; l < L; ++l)
+        for (int i = lrows[l]; i < lrows[l + 1]; ++i) entries[l] += rp[ord[i] + 1] - rp[ord[i]] - 1;
+    if (levels_on_grid(entries, mat_levels, n_rows)) {
+        // sweep steps = the levels of the block-diagonal matrix, each wide
+        src_begin.assign(nl, 0);
+        count.assign(nl, 0);
+        for (int64_t r = 0; r < n_rows; ++r) count[hl[r]]++;
+        for (int l = 1; l < nl; ++l) src_begin[l] = src_begin[l - 1] + count[l - 1];
+        std::vector<int> at(src_begin), by_level(n_rows);
+        for (int64_t r = 0; r < n_rows; ++r) by_level[at[hl[r]]++] = (int)r;
+        for (int l = 0; l < nl; ++l) steps.push_back(SweepStep{l, 1, 0});
+        DevBuf d_order;
+        up(d_order, by_level);
+        on_grid = pack_ok = build_sweep_pack(pack, A.rp(), A.ci(), A.val.p, D.p, vbytes, n_rows, d_order.as<int>(),
+                                             src_begin, count, steps, false, false, st);
+        if (on_grid) return;
+        steps.clear();
+    }
+    // sweep steps = every matrix's levels in order; each matrix is one run
+    src_begin.assign(L, 0);
+    count.assign(L, 0);
     for (int m = 0; m < n_mats; ++m) {
         for (int l = moff[m]; l < moff[m + 1]; ++l) {
             src_begin[l] = lrows[l];
@@ -252,6 +303,10 @@ template <typename VT>
 void TriBatch::solve_persistent(const VT *B, VT *X, cudaStream_t st) {
     if (n_mats == 0) return;
     check_status();
+    if (on_grid) {
+        sweep_solve<VT>(pack, B, X, 1, 1, 1, nullptr, wait, st);
+        return;
+    }
     if (pack_ok) {
         sweep_solve_batch<VT>(pack, queue_order.as<int>(), n_mats, queue.as<int>(), B, X, error.p, wait, st);
         return;

@@ -32,6 +32,7 @@ struct TriBatch {
     DevBuf D, order, mat_lvl_off, lvl_rows, queue_order, queue;
     SweepPack pack;          // level-ordered pack, one single-CTA run per matrix
     bool pack_ok = false;    // false: the plain batch kernel (the pack would be too sparse)
+    bool on_grid = false;    // the pack's levels are all the matrices', each a launch of the whole chip
     SweepWait wait, graph_wait;
     cudaGraphExec_t graph = nullptr;
     const void *graph_b = nullptr, *graph_x = nullptr;

@@ -322,6 +322,28 @@ def test_a_wait_that_runs_out_is_an_error_and_recoverable(kind, k, mode, most):
     assert normwise(x.reshape(n, k), ref) <= tol(np.float64)
 
 
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+def test_batches_with_levels_for_the_whole_chip(vt):
+    """Few matrices of wide levels, of different depth, one without levels to wait for."""
+    import torch
+    from smaxkernels_b200.interface import FloatType, TriangularBatch
+    mats = [wide_levels([9000] * 6, 3, 1, vt), wide_levels([20000, 1], 5, 2, vt), wide_levels([5], 1, 3, vt),
+            wide_levels([3000] * 9, 8, 4, vt)]
+    tb = TriangularBatch(mats, FloatType.FLOAT64 if vt == np.float64 else FloatType.FLOAT32)
+    b = np.random.default_rng(3).uniform(-1, 1, sum(len(m[0]) - 1 for m in mats)).astype(vt)
+    bd = torch.from_numpy(b).cuda()
+    xd = torch.zeros_like(bd)
+    for mode in (0, MERGED):
+        xd.zero_()
+        tb.solve(bd, xd, mode)
+        tb.sync()
+        x = xd.cpu().numpy()
+        for m, (rp, col, val) in enumerate(mats):
+            a, e = tb.row_offset(m), tb.row_offset(m + 1)
+            assert normwise(x[a:e], O.sptrsv(rp, col, val, b[a:e])) <= tol(vt), m
+    tb.close()
+
+
 def test_batch_of_a_level_with_more_chunks_than_a_barrier_counts():
     """One diagonal matrix of 2^18 chunks of 256 rows and a little more, and a small one."""
     import torch
