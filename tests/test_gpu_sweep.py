@@ -323,6 +323,38 @@ def test_a_wait_that_runs_out_is_an_error_and_recoverable(kind, k, mode, most):
 
 
 @pytest.mark.parametrize("vt", [np.float64, np.float32])
+def test_batch_of_more_matrices_than_sms_with_narrow_levels(vt):
+    """Levels of at most 30 rows: two CTAs share an SM and half the stage each, and
+    take several matrices one after the other; some of one row, one with a row
+    of 300 entries, which that stage does not hold."""
+    import torch
+    from smaxkernels_b200.interface import FloatType, TriangularBatch
+    rng = np.random.default_rng(4)
+    count = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 104
+    mats = [level_matrix([1] if m % 50 == 7 else rng.integers(1, 31, 12).tolist(), 1 + m % 5, m, vt) for m in range(count)]
+    n = 400
+    rows = [[r - 1, r] if r else [0] for r in range(n)]
+    rows[350] = list(range(50, 350)) + [350]
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    val = rng.uniform(-1, 1, rp[-1]) / 20
+    val[rp[1:] - 1] = rng.uniform(1, 2, n)
+    mats[100] = (rp, np.concatenate(rows).astype(np.int32), val.astype(vt))
+    tb = TriangularBatch(mats, FloatType.FLOAT64 if vt == np.float64 else FloatType.FLOAT32)
+    b = rng.uniform(-1, 1, sum(len(m[0]) - 1 for m in mats)).astype(vt)
+    bd = torch.from_numpy(b).cuda()
+    xd, again = torch.zeros_like(bd), torch.zeros_like(bd)
+    tb.solve(bd, xd)
+    tb.solve(bd, again)
+    tb.sync()
+    assert torch.equal(xd, again)
+    x = xd.cpu().numpy()
+    for m, (rp, col, val) in enumerate(mats):
+        a, e = tb.row_offset(m), tb.row_offset(m + 1)
+        assert normwise(x[a:e], O.sptrsv(rp, col, val, b[a:e])) <= tol(vt), m
+    tb.close()
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
 def test_batches_with_levels_for_the_whole_chip(vt):
     """Few matrices of wide levels, of different depth, one without levels to wait for."""
     import torch
