@@ -17,6 +17,7 @@ struct SpgemmWork {
     DevBuf wts, wsz, woff, wkeys, wfirst, wvals, wpos;
     DevBuf masks;              // merge path: each row's first-touch mask
     bool direct_hint = false;  // the last apply took the direct merge path
+    AuxStream side;            // of the rows with global tables
 };
 
 // C's columns per row are in first-touch order and its values are summed in

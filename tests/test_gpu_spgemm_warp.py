@@ -70,3 +70,33 @@ def test_large_product_is_downloaded_whole(vt, nnz):
     np.testing.assert_array_equal(cval, val)
     cval[-1] = 2
     assert cval[-1] == 2
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+def test_rows_of_every_size_at_once(vt):
+    """Rows for every table of the warps and for tables in global memory, which run
+    beside each other; repeated, and with the sizes in another order."""
+    from smaxkernels_b200 import FloatType, Interface, IntType, KernelType, PlatformType
+    rng = np.random.default_rng(15)
+    n = 1200
+    lens = rng.choice([1, 8, 20, 40, 70, 120, 260], n)
+    for order in (np.argsort(lens), rng.permutation(n)):
+        ls = lens[order]
+        rp = np.concatenate([[0], np.cumsum(ls)]).astype(np.int32)
+        col = np.concatenate([np.sort(rng.choice(n, l, replace=False)) for l in ls]).astype(np.int32)
+        val = rng.uniform(-1, 1, len(col)).astype(vt)
+        orp, ocol, oval = O.spgemm(rp, col, val, rp, col, val, n)
+        smax = Interface()
+        smax.register_kernel("k", KernelType.SPGEMM, PlatformType.CUDA, IntType.INT32,
+                             FloatType.FLOAT64 if vt == np.float64 else FloatType.FLOAT32)
+        k = smax.kernel("k")
+        k.register_A(n, n, len(col), col, rp, val)
+        k.register_B(n, n, len(col), col, rp, val)
+        k.register_C()
+        for _ in range(3):
+            k.run()
+            _, _, _, crp, ccol, cval = k.result()
+            np.testing.assert_array_equal(crp, orp)
+            np.testing.assert_array_equal(ccol, ocol)
+            assert normwise(cval, oval) <= tol(vt)
+        smax.close()
