@@ -29,10 +29,10 @@
 //
 // Measured before and after (before: the grid kernel, a warp per row for
 // widths that are no power of two, k SpMVs for column-major blocks):
-//   27-point 128^3, k = 16, FP64              635 -> 489 us
+//   27-point 128^3, k = 16, FP64              652 -> 495 us
 //   27-point 96^3, k = 5, FP64                560 -> 136 us
-//   27-point 96^3, k = 8, column-major, FP64  664 -> 191 us
-//   lognormal 600000 rows, k = 20, FP32       366 -> 208 us
+//   27-point 96^3, k = 8, column-major, FP64  688 -> 196 us
+//   lognormal 600000 rows, k = 20, FP32       341 -> 177 us
 //   lognormal 500000 rows, k = 16, FP64       569 -> 256 us
 #include "spmv_formats.cuh"
 
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
 // a lane per vector and 32 / G entries side by side, four of them in flight a
 // lane; then the lanes of one vector are added up.  part: kq sums a piece.
 // Bound by the gathers of X, as the group kernel is.  10^6 rows of 5 entries, one
-// of 10^6, k = 8 column-major FP64: 112 ms by one group, see spmm_by_columns.
+// of 10^6, k = 8 column-major FP64: 112 ms with that row left to a group, 0.19 ms now.
 template <typename VT>
 __global__ void __launch_bounds__(256) spmm_piece_kernel(const int2 *__restrict__ pieces, int64_t n_pieces,
                                                          const int *__restrict__ col, const VT *__restrict__ val,

@@ -186,8 +186,8 @@ class Kernel:
         return self._register_dense(2, args)
 
     def result(self):
-        """SpGEMM: C as (n_rows, n_cols, nnz, row_ptr, col, val) numpy copies of
-        the arrays finalize() allocated (which are then released)."""
+        """SpGEMM: C as (n_rows, n_cols, nnz, row_ptr, col, val) numpy arrays
+        that own the memory finalize() allocated."""
         r = self._cref
         n_rows, n_cols, nnz = r[0].value, r[1].value, r[2].value
         vt = np.float64 if self.float_type == FloatType.FLOAT64 else np.float32
