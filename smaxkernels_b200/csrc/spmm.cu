@@ -22,10 +22,12 @@
 // and not once per vector.  The products per vector that it replaces spread a long
 // row over the chip and add it up in slices.  So a row far longer than the
 // others is not left to one group, which takes 0.1 us an entry, but cut into
-// pieces, a warp each (spmm_piece_kernel, spmm_combine_kernel), and four products
-// at a time are added to a sum that loses less: 64 bits wide for FP32,
-// compensated for FP64.  (A row-major block is added up in stored order, by
-// whichever kernel.)
+// pieces, a warp each (spmm_piece_kernel, spmm_combine_kernel), and eight
+// products at a time (four where a lane has four vectors) are added to a sum that
+// loses less: 64 bits wide for FP32, compensated for FP64.  (Four at a time: rows of
+// 900, k = 33 FP32 100 us, 87 with eight; sixteen in two plain sums lose more than
+// the products do.)  (A row-major block is added up in stored order, by whichever
+// kernel.)
 //
 // Measured before and after (before: the grid kernel, a warp per row for
 // widths that are no power of two, k SpMVs for column-major blocks):
@@ -206,8 +208,13 @@ template <typename VT> __device__ __forceinline__ void read4(const VT *p, VT (&v
     }
 }
 
-// The sums of a column-major block: 64 bits for FP32; for FP64, the rounding errors
-// of the additions beside the sum.
+// The sums of a column-major block: eight products at a time are summed plainly, and
+// those sums in 64 bits for FP32; for FP64, with the rounding errors of the additions
+// beside the sum.
+template <typename VT> struct Plain {
+    VT sum;
+    __device__ __forceinline__ void add(VT x) { sum += x; }
+};
 struct Wide {
     double sum;
     __device__ __forceinline__ void add(float x) { sum += x; }
@@ -353,6 +360,16 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
 #pragma unroll
         for (int i = 0; i < VEC; ++i) acc[m][i] = AT{};
 
+    // a plain sum of some entries to the row's
+    using Part = Plain<VT>;
+    auto fold = [&](const Part(&part)[NV][VEC]) {
+        if constexpr (COL) {
+#pragma unroll
+            for (int m = 0; m < NV; ++m)
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) acc[m][i].add(part[m][i].sum);
+        }
+    };
     // the entries of a staged chunk, n of them, into acc
     auto chunk = [&](int b, int n) {
         const VT *sv = reinterpret_cast<const VT *>(reinterpret_cast<unsigned char *>(sv0) + b * stage);
@@ -361,13 +378,38 @@ __global__ void __launch_bounds__(group_warps(NV) * 32, 1)
         // lane, fewer entries at a time, for the same bytes in flight
         constexpr int U = group_unroll(NV);
         int j = 0;
-        for (; j + U <= n; j += U) take<VT, AT, VB, NV, U>(sc + j, sv + j, xl, ldx, acc);
-        if constexpr (U > 2)
-            if (j + 2 <= n) {
-                take<VT, AT, VB, NV, 2>(sc + j, sv + j, xl, ldx, acc);
-                j += 2;
+        if constexpr (COL) {
+            for (; j + 2 * U <= n; j += 2 * U) {
+                Part part[NV][VEC] = {};
+                take<VT, Part, VB, NV, U>(sc + j, sv + j, xl, ldx, part);
+                take<VT, Part, VB, NV, U>(sc + j + U, sv + j + U, xl, ldx, part);
+                fold(part);
             }
-        if (j < n) take<VT, AT, VB, NV, 1>(sc + j, sv + j, xl, ldx, acc);
+            if (j < n) {
+                Part part[NV][VEC] = {};
+                if (j + U <= n) {
+                    take<VT, Part, VB, NV, U>(sc + j, sv + j, xl, ldx, part);
+                    j += U;
+                }
+                if constexpr (U > 2) {
+                    if (j + 2 <= n) {
+                        take<VT, Part, VB, NV, 2>(sc + j, sv + j, xl, ldx, part);
+                        j += 2;
+                    }
+                }
+                if (j < n) take<VT, Part, VB, NV, 1>(sc + j, sv + j, xl, ldx, part);
+                fold(part);
+            }
+        } else {
+            for (; j + U <= n; j += U) take<VT, AT, VB, NV, U>(sc + j, sv + j, xl, ldx, acc);
+            if constexpr (U > 2) {
+                if (j + 2 <= n) {
+                    take<VT, AT, VB, NV, 2>(sc + j, sv + j, xl, ldx, acc);
+                    j += 2;
+                }
+            }
+            if (j < n) take<VT, AT, VB, NV, 1>(sc + j, sv + j, xl, ldx, acc);
+        }
     };
     // the finished row to Y (store: it was not left out), and acc back to zero
     auto finish = [&](int row, bool store) {

@@ -71,9 +71,10 @@ def test_values_that_are_not_finite(vt, bad):
 
 @pytest.mark.parametrize("vt", [np.float64, np.float32])
 @pytest.mark.parametrize("lens", ["mixed", "27", "400", "2000"])
-def test_sums_no_worse_than_the_products_per_column(vt, lens):
+@pytest.mark.parametrize("k", [8, 40, 200])
+def test_sums_no_worse_than_the_products_per_column(vt, lens, k):
     rng = np.random.default_rng(7)
-    n, k = 6000, 8
+    n = 6000 if k == 8 else 1500
     lens = {"mixed": np.exp(rng.normal(2.3, 1.2, n)).astype(int) + 1, "27": np.full(n, 27), "400": np.full(n, 400),
             "2000": np.where(np.arange(n) % 10 == 0, 2000, 1200)}[lens]
     rp, col, val = _matrix(lens, 8, vt)
