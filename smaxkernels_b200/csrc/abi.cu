@@ -200,7 +200,7 @@ template <typename VT> void spmm_apply_t(smax_kernel_s *k, const VT *X, VT *Y) {
         // column-major: the reference uses A's n_rows as the leading dimension
         // of both X and Y (src/kernels/spmm/spmm_cpu/spmm_cpu_crs_impl.hpp:29,44)
         const int64_t ld = k->dA.n_rows;
-        if (kk > 1 && !spmm_by_columns(k->dA, kk, k->crs_stream.longest) &&
+        if (kk > 1 && !spmm_by_columns(k->dA, kk, k->vbytes, k->crs_stream.longest) &&
             (int64_t)k->spmm_plan.work.bytes >= spmm_col_major_work(k->dA.n_cols, kk, k->vbytes) &&
             (int64_t)k->spmm_plan.part.bytes >= k->spmm_plan.part_bytes(kk)) {
             crs_spmm_col_major<VT>(k->dA, kk, X, Y, ld, k->spmm_plan.work.as<VT>(), k->stream, k->spmm_plan);
@@ -482,7 +482,7 @@ void do_initialize(smax_kernel_s *k, bool wait = true) {
     // pieces, allocated here so that applies allocate nothing; without room for
     // them they run one product per column
     if (k->ktype == SMAX_KERNEL_SPMM && !k->f_row_major && k->B.n_cols > 1 &&
-        !spmm_by_columns(k->dA, (int64_t)k->B.n_cols, k->crs_stream.longest)) {
+        !spmm_by_columns(k->dA, (int64_t)k->B.n_cols, k->vbytes, k->crs_stream.longest)) {
         const int64_t kk = (int64_t)k->B.n_cols;
         try {
             k->spmm_plan.part.ensure((size_t)k->spmm_plan.part_bytes(kk));

@@ -904,11 +904,27 @@ void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStre
 // where their lengths differ (products and block, lognormal 30000 rows FP64 28 and 47 us, 300000
 // 66 and 141; 2^19 rows of 8, one in 100 of 64: 60 and 89; 20000 of these 27 and
 // 23) and three where some are far longer (lognormal 30000 FP32 37 and 47, 300000 92 and 105).
-bool spmm_by_columns(const DevCRS &a, int64_t k, int64_t longest) {
+// Two vectors of even rows too, once A is large: a lane then has a row to itself and
+// waits for a vector of X per entry.  27-point 24^3 FP64 19 and 20, 40^3 26 and 38, 96^3
+// 166 and 532; FP32 40^3 22 and 23, 64^3 43 and 61, 96^3 106 and 159; 40000 rows of 100
+// FP32 66 and 50, 200000 179 and 257.  Rows of hundreds keep their lanes waiting for
+// the longest already where it has a quarter more than the average (3000 rows of 50 to
+// 150 FP64 30 and 38, 1500 of 100 to 300 35 and 50; three vectors, 1111 of 450 to 1350
+// 83 and 108; 1500 of 200 each 35 and 34).  And, of many short rows, where the copies of X
+// and the columns of Y outweigh A: three vectors (7-point 200^3 FP64 522 and 637, FP32
+// 351 and 476; 3.3 million rows of 6 FP64 301 and 346), in FP32 of rows below 8 entries
+// also four to six (7-point 200^3 447 and 487, 557 and 682, 658 and 688; 13 million
+// rows of 6, k = 6 1952 and 2439).
+bool spmm_by_columns(const DevCRS &a, int64_t k, int vbytes, int64_t longest) {
     if (near_int_end(a.n_rows) || k >= (1 << 30)) return true;
     const bool skewed = longest * a.n_rows > 64 * a.nnz;
     const bool uneven = longest * a.n_rows > 2 * a.nnz + 8 * a.n_rows;
     if (a.nnz < 4 * a.n_rows) return (k < 8 && a.n_rows >= (1 << 17)) || (k <= 8 && skewed);
+    if (k == 2 && a.nnz >= (vbytes == 8 ? 1 << 19 : a.nnz < 64 * a.n_rows ? 1 << 21 : 1 << 23)) return true;
+    if (k == 3 && a.n_rows >= (1 << 21) && a.nnz < 16 * a.n_rows) return true;
+    if (k <= 6 && vbytes == 4 && a.n_rows >= (1 << 22) && a.nnz < 8 * a.n_rows) return true;
+    const bool long_uneven = a.nnz >= (k == 2 ? 64 : 512) * a.n_rows && 4 * longest * a.n_rows > 5 * a.nnz;
+    if (k <= 3 && a.nnz >= (1 << 18) && long_uneven) return true;
     return a.nnz >= (1 << 18) && ((k == 2 && uneven) || (k == 3 && longest * a.n_rows > 32 * a.nnz));
 }
 

@@ -83,7 +83,7 @@ template <typename VT>
 void crs_spmm_row_major(const DevCRS &a, int64_t k, const VT *X, VT *Y, cudaStream_t st, const SpmmPlan &plan,
                         int variant = 0);
 // whether a column-major block of k vectors runs as k products instead
-bool spmm_by_columns(const DevCRS &a, int64_t k, int64_t longest);
+bool spmm_by_columns(const DevCRS &a, int64_t k, int vbytes, int64_t longest);
 // bytes of workspace crs_spmm_col_major needs for k vectors
 int64_t spmm_col_major_work(int64_t n_cols, int64_t k, int vbytes);
 template <typename VT>

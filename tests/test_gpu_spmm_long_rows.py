@@ -99,3 +99,34 @@ def test_few_vectors_where_the_products_begin(vt, k, n, most):
     X = np.random.default_rng(9).uniform(-1, 1, n * k).astype(vt)
     Y = gpu_spmm(rp, col, val, X, k, False)
     assert normwise(Y, O.spmm(rp, col, val, X, k, row_major=False)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("n,length", [(65535, 8), (65536, 8), (32767, 64), (32768, 63), (32768, 64),
+                                       (5000, 64), (600, 512)])
+def test_even_rows_where_the_products_begin(vt, k, n, length):
+    """2^19 and 2^21 entries, less and more, in rows on both sides of 64; a few
+    longer ones by a quarter, or just more."""
+    lens = np.full(n, length)
+    lens[:20] += length // 4 + (k == 3)
+    lens[20:40] -= length // 4 + (k == 3)
+    rp, col, val = _matrix(lens, k, vt)
+    X = np.random.default_rng(10).uniform(-1, 1, n * k).astype(vt)
+    Y = gpu_spmm(rp, col, val, X, k, False)
+    assert normwise(Y, O.spmm(rp, col, val, X, k, row_major=False)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("n,k", [((1 << 21) - 1, 3), (1 << 21, 3), ((1 << 22) - 1, 5), (1 << 22, 5), (1 << 22, 7)])
+def test_many_short_rows_where_the_products_begin(vt, n, k):
+    """2^21 and 2^22 rows of four entries, and one less."""
+    rng = np.random.default_rng(k)
+    rp = np.arange(0, 4 * n + 1, 4, dtype=np.int32)
+    col = rng.integers(0, n, 4 * n).astype(np.int32)
+    val = rng.uniform(-1, 1, 4 * n).astype(vt)
+    X = rng.uniform(-1, 1, n * k).astype(vt)
+    Y = gpu_spmm(rp, col, val, X, k, False).reshape(k, n)
+    for v in range(k):
+        ref = (val.astype(np.float64) * X[v * n:(v + 1) * n][col]).reshape(n, 4).sum(1)
+        assert normwise(Y[v], ref) <= tol(vt)
