@@ -23,6 +23,7 @@ struct CrsStreamPlan {
     const int *row_ptr = nullptr;  // the matrix's device row pointer given to build (not owned)
     int longest = 0;               // entries of the longest row; up to 32: slices need no carries
     bool scattered = false;        // neighbouring rows' columns lie far apart (if build was given them)
+    bool narrow = false;           // most rows' columns lie close together (likewise)
     DevBuf endbits, task_rank, carry_val, carry_rank, row_list, empty_rows;
     void build(const int *d_row_ptr, int64_t n_rows, int64_t nnz, int vbytes, cudaStream_t st,
                const int *d_col = nullptr);

@@ -258,8 +258,20 @@ __global__ void row_flags_kernel(const int *__restrict__ row_ptr, int64_t n, uns
 
 // A sample of the columns, 32 neighbouring rows a warp: found[0] counts entries of
 // rows short enough for crs_rows_kernel, found[1] those whose column lies more
-// than kFar from that of the row before's entry in the same place.
+// than kFar from that of the row before's entry in the same place, found[2] rows,
+// found[3] those whose columns span at most narrow_width an entry.
 constexpr int kFar = 16384;
+// The columns an entry up to which a matrix of rows of len entries is better streamed
+// (crs_spmv_stream).  Of a multiple of four entries, a stream's lanes, of four each,
+// gather neighbouring rows' neighbouring columns together; rows that leave a third of
+// crs_rows_kernel's slots unused cost it more.  Others gather worse than it does, unless
+// their columns follow on each other (12 million entries FP64, stream and rows: of 27,
+// 37 apart, 59 and 43, neighbours 38 and 41).
+__device__ __forceinline__ int narrow_width(int len) {
+    if (len == 8 || len == 16) return 80;
+    const int slots = len <= 4 ? 4 : (len <= 8 ? 8 : (len <= 16 ? 16 : 32));
+    return len % 4 == 0 || 3 * len < 2 * slots ? 40 : 4;
+}
 constexpr int kSampleWarps = 512;
 __global__ void scatter_sample_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col, int64_t n,
                                       int *__restrict__ found) {
@@ -271,10 +283,14 @@ __global__ void scatter_sample_kernel(const int *__restrict__ row_ptr, const int
         s = row_ptr[r];
         len = min(row_ptr[r + 1] - s, 32);
     }
-    int seen = 0, far = 0;
+    int seen = 0, far = 0, lo = INT_MAX, hi = -1;
     const int most = __reduce_max_sync(0xffffffffu, len);
     for (int i = 0; i < most; ++i) {
         const int c = i < len ? col[s + i] : -1;
+        if (c >= 0) {
+            lo = min(lo, c);
+            hi = max(hi, c);
+        }
         const int before = __shfl_up_sync(0xffffffffu, c, 1);
         if (lane > 0 && c >= 0 && before >= 0) {
             ++seen;
@@ -283,9 +299,13 @@ __global__ void scatter_sample_kernel(const int *__restrict__ row_ptr, const int
     }
     seen = __reduce_add_sync(0xffffffffu, seen);
     far = __reduce_add_sync(0xffffffffu, far);
+    const int rows = __popc(__ballot_sync(0xffffffffu, hi >= 0));
+    const int close = __popc(__ballot_sync(0xffffffffu, hi >= 0 && hi - lo <= narrow_width(len) * len));
     if (lane == 0) {
         atomicAdd(found, seen);
         atomicAdd(found + 1, far);
+        atomicAdd(found + 2, rows);
+        atomicAdd(found + 3, close);
     }
 }
 
@@ -329,9 +349,9 @@ void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vby
     n_nonempty = 0;
     row_ptr = d_row_ptr;
     longest = 0;
-    scattered = false;
+    scattered = narrow = false;
     if (n > 0) {
-        DevBuf fe(n), fne(n), cnt(sizeof(int) * 5);
+        DevBuf fe(n), fne(n), cnt(sizeof(int) * 7);
         SMAX_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes, st));
         row_flags_kernel<<<ceil_div_u(n, 256), 256, 0, st>>>(d_row_ptr, n, fe.as<unsigned char>(),
                                                              fne.as<unsigned char>(), endbits.as<uint32_t>(),
@@ -347,12 +367,13 @@ void CrsStreamPlan::build(const int *d_row_ptr, int64_t n, int64_t nnz_, int vby
         DevBuf tmp(tb);
         SMAX_CUDA(cub::DeviceSelect::Flagged(tmp.p, tb, it, fe.as<unsigned char>(), empty_rows.as<int>(),
                                              cnt.as<int>(), (int)n, st));
-        int h[5] = {0, 0, 0, 0, 0};
+        int h[7] = {0, 0, 0, 0, 0, 0, 0};
         SMAX_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, st));
         SMAX_CUDA(cudaStreamSynchronize(st));
         n_empty = h[0];
         longest = h[2];
         scattered = 2 * h[4] > h[3];
+        narrow = 2 * h[6] > h[5];
         n_nonempty = n - n_empty;
         if (n_empty > 0) {
             row_list.alloc(sizeof(int) * (n_nonempty > 0 ? n_nonempty : 1));
@@ -386,7 +407,16 @@ void crs_spmv_stream(const CrsStreamPlan &p, const int *col, const VT *val, cons
     // own lines out of L1 before its lanes have used them: 2^20 rows of 17 FP64 88 ->
     // 107, of 32 150 -> 172 (of 8 45 -> 47, and 2^17 rows of 32 30 -> 30).
     const bool crowded = p.scattered && p.longest > 8 && p.n_rows >= (1 << 18);
-    if (p.n_rows > 0 && p.longest <= 32 && !crowded && 3 * p.nnz >= 2 * p.n_rows * p.longest) {
+    // Columns close together are in L1 either way, and the stream loads col and val
+    // better.  Rows of 8, 16 and, in FP32, 32 entries put a warp's loads on few of L1's
+    // banks (columns 37 apart, 4 million entries FP64: of 8 21 and 24, of 16 21 and 24;
+    // below a million 12 and 12); beyond L2 other lengths lose as well (12 million FP64: of
+    // 9 42 and 51, of 12 41 and 45; FP32: of 2 31 and 48, of 12 28 and 30; 4 million
+    // FP64: of 12 22 and 18).
+    const bool banks = p.longest == 8 || p.longest == 16 || (p.longest == 32 && sizeof(VT) == 4);
+    const bool beyond = p.nnz * (int64_t)(sizeof(VT) + sizeof(int)) >= (int64_t)80 << 20;
+    const bool streams = p.narrow && (beyond || (banks && p.nnz >= (1 << 20)));
+    if (p.n_rows > 0 && p.longest <= 32 && !crowded && !streams && 3 * p.nnz >= 2 * p.n_rows * p.longest) {
         // rows without entries get their zero here as well
         auto rows = [&](auto kern, int g) {
             kern<<<ceil_div_u((uint64_t)p.n_rows * g, 256), 256, 0, st>>>(col, val, p.row_ptr, p.n_rows, x, y);

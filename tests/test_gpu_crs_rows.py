@@ -80,3 +80,43 @@ def test_columns_near_and_all_over(vt, longest, n, far):
     val = rng.uniform(-1, 1, len(col)).astype(vt)
     x = rng.uniform(-1, 1, n).astype(vt)
     assert normwise(gpu_spmv(rp, col, val, x), O.spmv_crs(rp, col, val, x)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt,n9", [(np.float64, 776722), (np.float64, 776724), (np.float32, 1165084)])
+def test_narrow_rows_beyond_the_cache(vt, n9):
+    """Rows of 9 on both sides of 80 MiB of entries, and as many of 27 a little wide."""
+    from helpers import gpu_spmv
+    rng = np.random.default_rng(n9)
+    for longest, apart in ((9, 40), (27, 37)):
+        n = n9 * 9 // longest
+        rp = np.arange(n + 1, dtype=np.int32) * longest
+        col = ((np.arange(n)[:, None] + apart * np.arange(longest)) % n).astype(np.int32).reshape(-1)
+        val = rng.uniform(-1, 1, len(col)).astype(vt)
+        x = rng.uniform(-1, 1, n).astype(vt)
+        assert normwise(gpu_spmv(rp, col, val, x), O.spmv_crs(rp, col, val, x)) <= tol(vt)
+
+
+@pytest.mark.parametrize("vt", [np.float64, np.float32])
+@pytest.mark.parametrize("longest,nnz", [(8, 1 << 20), (16, 1 << 20), (16, (1 << 20) - 16), (32, 1 << 20)])
+@pytest.mark.parametrize("more", [0, 1])
+def test_rows_that_share_banks(vt, longest, nnz, more):
+    """2^20 entries and less, columns as wide apart as counts as narrow and one more,
+    some rows shorter or empty."""
+    from helpers import gpu_spmv
+    n = nnz // longest + 110
+    width = (80 if longest < 32 else 40) * longest + more
+    rng = np.random.default_rng(longest)
+    lens = np.full(n, longest)
+    lens[100:200] = 0
+    lens[300:320] = longest // 2
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    first = np.repeat(np.arange(n), lens)
+    last = np.zeros(len(first), bool)
+    last[rp[1:][lens > 0] - 1] = True
+    step = np.where(last, width, rng.integers(0, width, len(first)))
+    head = np.zeros(len(first), bool)
+    head[rp[:-1][lens > 0]] = True
+    col = (np.minimum(first, n - width - 1) + np.where(head, 0, step)).astype(np.int32)
+    val = rng.uniform(-1, 1, len(col)).astype(vt)
+    x = rng.uniform(-1, 1, n).astype(vt)
+    assert normwise(gpu_spmv(rp, col, val, x), O.spmv_crs(rp, col, val, x)) <= tol(vt)
