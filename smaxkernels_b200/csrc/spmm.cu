@@ -33,8 +33,8 @@
 // widths that are no power of two, k SpMVs for column-major blocks):
 //   27-point 128^3, k = 16, FP64              652 -> 495 us
 //   27-point 96^3, k = 5, FP64                560 -> 136 us
-//   27-point 96^3, k = 8, column-major, FP64  688 -> 196 us
-//   lognormal 600000 rows, k = 20, FP32       341 -> 177 us
+//   27-point 96^3, k = 8, column-major, FP64  688 -> 185 us
+//   lognormal 600000 rows, k = 20, FP32       341 -> 183 us
 //   lognormal 500000 rows, k = 16, FP64       569 -> 256 us
 #include "spmv_formats.cuh"
 
